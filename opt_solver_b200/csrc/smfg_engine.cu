@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "smfg_kernels.cuh"
+#include "smfg_small.cuh"
 #include "smfg_tc.cuh"
 
 namespace smfg {
@@ -79,7 +80,7 @@ int sm_count(int dev) {
 // rows, positions and tags.
 size_t front_smem_bytes(int fmax, int nb, int blocked_min_front = 0) {
   const size_t w = (fmax >= blocked_min_front) ? (size_t)fmax * nb * 8 : 0;
-  return (size_t)fmax * fmax * 8 + w + (size_t)fmax * 12 + (size_t)fmax + 64;
+  return (size_t)fmax * (fmax | 1) * 8 + w + (size_t)fmax * 12 + (size_t)fmax + 64;
 }
 
 }  // namespace
@@ -177,6 +178,11 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
     const int s = a.postorder[i];
     lvl_sn[fill[level[s]]++] = s;
   }
+  // each level's fronts by symbolic rows, largest first: the size classes are
+  // ranges of the list
+  for (int l = 0; l < nl; ++l)
+    std::stable_sort(lvl_sn.begin() + pl.lvl_ptr[l], lvl_sn.begin() + pl.lvl_ptr[l + 1],
+                     [&](int x, int y) { return fsym[x] > fsym[y]; });
   // large fronts (multi-block path): by symbolic rows; fronts that delays
   // take to the APTP size join later (large_lists)
   pl.h_large.assign(ns, 0);
@@ -697,6 +703,111 @@ static void ensure_tri_inv(Plan &pl) {
   pl.x.tri_inv = dalloc<double>(pl, (size_t)tot);
 }
 
+// Threads of the fused front kernel's blocks (fronts of 33..64 rows, of
+// 65..95; a warp below). Half as many: 9% slower on one small trajectory KKT;
+// twice as many: 12% slower on a batch of 256 (fewer fronts resident).
+constexpr int kSmallNT = 128, kUpperNT = 256;
+
+// Rows of the largest front that is assembled, factored and stored by one
+// block (k_small_front): those below the blocked size.
+static int fuse_rows(const smfg_control_t &c) { return std::min(kFuseMax, c.blocked_min_front - 1); }
+
+// The fronts of level l outside the large-front path, by size class. The
+// classes work on different fronts, so they run side by side: each nonempty
+// class but the last on a side stream after the level's set-up (or after its
+// assembly, for fronts too large to be assembled by their own block), the
+// last on the plan's stream unless the large fronts come there. Returns the
+// side streams used, whose events the caller waits for.
+// A class is a range of the level's list (largest symbolic front first).
+// SPD: exact. Indefinite: delays may have grown any smaller front into it, so
+// the range runs to the end of the list (level 0 has no children: exact);
+// the kernels test the realized rows.
+static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, int fuse, const PivotParams &prm,
+                                    bool has_large, LaunchCount &lc) {
+  DevPlan &d = pl.d;
+  DevFactor &x = pl.x;
+  cudaStream_t st = pl.stream;
+  const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
+  const bool exact = c.posdef || l == 0;
+  // first list position of at most v symbolic rows
+  auto at_most = [&](int v) {
+    return (int)(std::partition_point(pl.h_lvl_sn.begin() + lo, pl.h_lvl_sn.begin() + hi,
+                                      [&](int s) { return pl.h_fsym[s] > v; }) - pl.h_lvl_sn.begin());
+  };
+  enum Kind { kGlobal, kMedium, kUpper, kSmall, kWarp };
+  struct Class { Kind kind; int fmin, fmax, i0, n; };
+  Class cls[6];
+  int nc = 0;
+  auto add = [&](Kind k, int fmin, int fmax) {
+    if (fmin > fmax) return;
+    int i0 = at_most(fmax);
+    if (k == kGlobal) {  // past the large fronts, which head the list
+      while (i0 < hi && pl.h_large[pl.h_lvl_sn[i0]] && pl.h_fsym[pl.h_lvl_sn[i0]] >= kLargeMin) ++i0;
+    }
+    const int i1 = exact ? at_most(fmin - 1) : hi;
+    if (i1 > i0) cls[nc++] = {k, fmin, fmax, i0, i1 - i0};
+  };
+  // the longest first: they start first
+  add(kGlobal, kMediumMax + 1, 1 << 30);
+  if (fuse == kFuseMax) {
+    add(kMedium, fuse + 1, kMediumMax);
+  } else {  // a smaller blocked_min_front: the fronts past it in two sizes
+    add(kMedium, std::max(fuse, 96) + 1, kMediumMax);
+    add(kMedium, fuse + 1, 96);
+  }
+  add(kUpper, 65, fuse);
+  add(kSmall, 33, std::min(fuse, 64));
+  add(kWarp, 1, std::min(fuse, 32));
+  auto fused = [](const Class &k) { return k.kind >= kUpper; };  // assembled by their own block
+  auto launch = [&](const Class &k, cudaStream_t q) {
+    const size_t sm = fused(k) ? small_smem_bytes(k.fmax) : front_smem_bytes(k.fmax, c.nb, c.blocked_min_front);
+    switch (k.kind) {
+      case kWarp: k_small_front<32, 32><<<k.n, 32, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
+      case kSmall: k_small_front<kSmallNT, 64><<<k.n, kSmallNT, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
+      case kUpper: k_small_front<kUpperNT, 96><<<k.n, kUpperNT, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
+      case kMedium:
+        // SPD fronts take their updates with four times the threads (per
+        // entry the same operations in the same order)
+        if (c.posdef) k_factor<512, true><<<k.n, 512, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax);
+        else k_factor<128, true><<<k.n, 128, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax);
+        break;
+      case kGlobal: k_factor<512, false><<<k.n, 512, 0, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
+    }
+    lc.n += 1;
+  };
+  unsigned used = 0;
+  int next = 0;
+  auto launch_side = [&](const Class &k, cudaEvent_t after) {
+    const int i = std::min(next++, kSideStreams - 1);
+    SMFG_CUDA(cudaStreamWaitEvent(pl.side[i], after, 0));
+    used |= 1u << i;
+    launch(k, pl.side[i]);
+  };
+  const int first = has_large ? 0 : 1;  // cls[0] stays on the plan's stream without large fronts
+  if (nc > first && fused(cls[nc - 1])) {
+    SMFG_CUDA(cudaEventRecord(pl.ev_setup, st));
+    for (int i = first; i < nc; ++i)
+      if (fused(cls[i])) launch_side(cls[i], pl.ev_setup);
+  }
+  // rows and assembly of the fronts past fuse rows
+  const int na = exact ? at_most(fuse) - lo : hi - lo;
+  if (na > 0) {
+    k_level_rows<<<na, 128, 0, st>>>(d, x, lo, fuse);
+    // 32-column work items: a level of a few large fronts has hundreds
+    k_level_assemble<<<4 * sm_count(pl.device), 256, 0, st>>>(d, x, lo, hi, l);
+    lc.n += 2;
+  }
+  if (nc > first && !fused(cls[first])) {
+    SMFG_CUDA(cudaEventRecord(pl.ev_asm, st));
+    for (int i = first; i < nc; ++i)
+      if (!fused(cls[i])) launch_side(cls[i], pl.ev_asm);
+  }
+  if (nc > 0 && first == 1) launch(cls[0], st);
+  for (int i = 0; i < kSideStreams; ++i)
+    if (used >> i & 1) SMFG_CUDA(cudaEventRecord(pl.ev_side[i], pl.side[i]));
+  return used;
+}
+
 static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_t &c, LaunchCount &lc,
                            GemmProfile &gp, bool fixed = false) {
   DevPlan &d = pl.d;
@@ -734,35 +845,13 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
                   aptp_on ? c.aptp_min_rows : 0};
   const MixedCfg mc = mixed_cfg(c);
   const int wcols = w_rows(pl, c, gp.on);
-  // the shared-memory front kernels by size bucket: each launch's shared
-  // memory sized to its bucket (more blocks per SM for the many small fronts)
-  const int bmf = c.blocked_min_front;
-  const size_t smem_s32 = front_smem_bytes(32, c.nb, bmf), smem_s48 = front_smem_bytes(48, c.nb, bmf);
-  const size_t smem_s56 = front_smem_bytes(56, c.nb, bmf), smem_s64 = front_smem_bytes(kSmallMax, c.nb, bmf);
-  const size_t smem_m96 = front_smem_bytes(96, c.nb, bmf), smem_m128 = front_smem_bytes(kMediumMax, c.nb, bmf);
+  const int fuse = fuse_rows(c);
   for (int l = 0; l < pl.nlevels; ++l) {
     const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1], m = hi - lo;
-    k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols);
-    k_level_rows<<<m, 128, 0, st>>>(d, x, lo, hi);
-    // 32-column work items: a level of a few large fronts has hundreds
-    const int asm_grid = 4 * sms;
-    k_level_assemble<<<asm_grid, 256, 0, st>>>(d, x, lo, hi, l);
-    k_factor<32, 1, 32, true><<<m, 32, smem_s32, st>>>(d, x, lo, hi, prm);
-    k_factor<32, 33, 48, true><<<m, 32, smem_s48, st>>>(d, x, lo, hi, prm);
-    k_factor<32, 49, 56, true><<<m, 32, smem_s56, st>>>(d, x, lo, hi, prm);
-    k_factor<32, 57, kSmallMax, true><<<m, 32, smem_s64, st>>>(d, x, lo, hi, prm);
-    // SPD fronts of 65..128 rows take their updates with four times the
-    // threads (per entry the same operations in the same order)
-    if (c.posdef) {
-      k_factor<512, kSmallMax + 1, 96, true><<<m, 512, smem_m96, st>>>(d, x, lo, hi, prm);
-      k_factor<512, 97, kMediumMax, true><<<m, 512, smem_m128, st>>>(d, x, lo, hi, prm);
-    } else {
-      k_factor<128, kSmallMax + 1, 96, true><<<m, 128, smem_m96, st>>>(d, x, lo, hi, prm);
-      k_factor<128, 97, kMediumMax, true><<<m, 128, smem_m128, st>>>(d, x, lo, hi, prm);
-    }
-    k_factor<512, kMediumMax + 1, 1 << 30, false><<<m, 512, 0, st>>>(d, x, lo, hi, prm);
-    lc.n += 10;
+    k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse);
+    lc.n += 1;
     const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
+    const unsigned side = launch_level_fronts(pl, c, l, fuse, prm, nL > 0, lc);
     if (nL > 0) {
       const int *lg = d.lvl_large + pl.lvl_large_ptr[l];
       // the fronts of at least aptp_min_rows realized rows take the APTP
@@ -889,6 +978,8 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
       k_large_store<<<ggrid, 256, 0, st>>>(d, x, lg, nL, c.posdef);
       lc.n += 4;
     }
+    for (int i = 0; i < kSideStreams; ++i)
+      if (side >> i & 1) SMFG_CUDA(cudaStreamWaitEvent(st, pl.ev_side[i], 0));
     if (limits) {
       k_level_limits<<<1, 256, 0, st>>>(d, x, lo, hi, neg_limit, work_cap);
       lc.n += 1;
@@ -906,23 +997,16 @@ static void set_kernel_attrs(int nb) {
   static int done_nb = -1;
   if (done_nb == nb) return;
   SMFG_CUDA(cudaFuncSetAttribute(k_tri_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem));
-  // (the with-W sizes: launches ask for at most these)
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<32, 1, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)front_smem_bytes(32, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<32, 33, 48, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)front_smem_bytes(48, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<32, 49, 56, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)front_smem_bytes(56, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<32, 57, kSmallMax, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)front_smem_bytes(kSmallMax, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<128, kSmallMax + 1, 96, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_smem_bytes(96, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<128, 97, kMediumMax, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)front_smem_bytes(kMediumMax, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<512, 97, kMediumMax, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)front_smem_bytes(kMediumMax, nb)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_factor<512, kSmallMax + 1, 96, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_smem_bytes(96, nb)));
+  // (the with-W size: launches ask for at most this)
+  for (auto kern : {k_factor<128, true>, k_factor<512, true>})
+    SMFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)front_smem_bytes(kMediumMax, nb)));
+  SMFG_CUDA(cudaFuncSetAttribute(k_small_front<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 small_smem_bytes(32)));
+  SMFG_CUDA(cudaFuncSetAttribute(k_small_front<kSmallNT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 small_smem_bytes(64)));
+  SMFG_CUDA(cudaFuncSetAttribute(k_small_front<kUpperNT, 96>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 small_smem_bytes(96)));
   SMFG_CUDA(cudaFuncSetAttribute(k_large_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
   SMFG_CUDA(cudaFuncSetAttribute(tc::k_tc_syrk<tc::kTF32x3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(tc::Smem)));
@@ -1372,6 +1456,12 @@ SMFG_API int smfg_plan_create(const smfg_analysis_t *a, int device, smfg_plan_t 
     SMFG_CUDA(cudaStreamCreateWithFlags(&h->pl.stream2, cudaStreamNonBlocking));
     SMFG_CUDA(cudaEventCreateWithFlags(&h->pl.ev_panel, cudaEventDisableTiming));
     SMFG_CUDA(cudaEventCreateWithFlags(&h->pl.ev_rest, cudaEventDisableTiming));
+    SMFG_CUDA(cudaEventCreateWithFlags(&h->pl.ev_setup, cudaEventDisableTiming));
+    SMFG_CUDA(cudaEventCreateWithFlags(&h->pl.ev_asm, cudaEventDisableTiming));
+    for (int i = 0; i < kSideStreams; ++i) {
+      SMFG_CUDA(cudaStreamCreateWithFlags(&h->pl.side[i], cudaStreamNonBlocking));
+      SMFG_CUDA(cudaEventCreateWithFlags(&h->pl.ev_side[i], cudaEventDisableTiming));
+    }
     {
       cudaMemPoolProps props = {};
       props.allocType = cudaMemAllocationTypePinned;
@@ -1410,6 +1500,8 @@ SMFG_API void smfg_plan_destroy(smfg_plan_t *plan) {
   Plan &pl = (*plan)->pl;
   cudaSetDevice(pl.device);
   if (pl.stream) cudaStreamSynchronize(pl.stream);
+  for (cudaStream_t q : pl.side)
+    if (q) cudaStreamSynchronize(q);
   for (void *p : pl.allocs) cudaFree(p);
   if (pl.ev0) cudaEventDestroy(pl.ev0);
   if (pl.ev1) cudaEventDestroy(pl.ev1);
@@ -1418,6 +1510,12 @@ SMFG_API void smfg_plan_destroy(smfg_plan_t *plan) {
   if (pl.stream2) cudaStreamSynchronize(pl.stream2);
   if (pl.ev_panel) cudaEventDestroy(pl.ev_panel);
   if (pl.ev_rest) cudaEventDestroy(pl.ev_rest);
+  if (pl.ev_setup) cudaEventDestroy(pl.ev_setup);
+  if (pl.ev_asm) cudaEventDestroy(pl.ev_asm);
+  for (int i = 0; i < kSideStreams; ++i) {
+    if (pl.ev_side[i]) cudaEventDestroy(pl.ev_side[i]);
+    if (pl.side[i]) cudaStreamDestroy(pl.side[i]);
+  }
   if (pl.stream2) cudaStreamDestroy(pl.stream2);
   if (pl.stream) cudaStreamDestroy(pl.stream);
   if (pl.pool) cudaMemPoolDestroy(pl.pool);

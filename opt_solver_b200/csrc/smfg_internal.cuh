@@ -13,7 +13,8 @@
 namespace smfg {
 
 // Size classes of the front kernels (rows f after delays).
-constexpr int kSmallMax = 64;    // one warp, front in shared memory
+constexpr int kFuseMax = 95;     // assembled, factored and stored by one block (smfg_small.cuh), below
+                                 // the blocked size (blocked_min_front, 96)
 constexpr int kMediumMax = 128;  // one block, front in shared memory
 constexpr int kAsmCols = 32;     // columns per assembly work item
 
@@ -81,6 +82,8 @@ struct DevFactor {
   int inv_nitems = 0;
 };
 
+constexpr int kSideStreams = 3;
+
 struct Plan {
   int device = 0;
   int n = 0, nsn = 0, nlevels = 0;
@@ -112,6 +115,10 @@ struct Plan {
   // while the next panel factors (events: a panel done, a rest update done)
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_panel = nullptr, ev_rest = nullptr;
+  // the size classes of a tree level run side by side (events: the level set
+  // up, assembled, each side stream done)
+  cudaStream_t side[kSideStreams] = {};
+  cudaEvent_t ev_setup = nullptr, ev_asm = nullptr, ev_side[kSideStreams] = {};
   // last factorization
   bool factored = false;
   int posdef = 0;

@@ -76,7 +76,7 @@ __global__ void k_eff_small(unsigned long long *cnt, double small_pivot) {
 // offsets by exclusive scan, delay offsets of the children in the parent's
 // row list (multifrontal_serial.cpp:510-545), assembly work items.
 template <int NT>
-__global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, int nb) {
+__global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, int nb, int fuse) {
   static_assert(NT % 32 == 0 && NT <= 1024, "block size");
   constexpr int NW = NT / 32;
   __shared__ long long wa[NW], wr[NW], wb[NW];
@@ -106,7 +106,8 @@ __global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, i
       X.sn_ne[s] = nd + P.sn_width[s];
       fa = (long long)f * f + (long long)f * nb;
       fr = f;
-      fb = (f + kAsmCols - 1) / kAsmCols;
+      // (fronts of at most fuse rows are assembled by their front kernel)
+      fb = (f <= fuse && !P.sn_large[s]) ? 0 : (f + kAsmCols - 1) / kAsmCols;
     }
     // inclusive block scan of (fa, fr, fb): warp shuffles, then the warps'
     // totals scanned by warp 0
@@ -176,13 +177,15 @@ __global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, i
   }
 }
 
-// Rows of each front (children's delayed rows in child order, then its
-// symbolic rows) and each child's contribution-block row map into it.
-__global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int hi) {
+// Rows of each front of more than fuse rows (children's delayed rows in child
+// order, then its symbolic rows) and each child's contribution-block row map
+// into it. Fronts P.lvl_sn[lo + block].
+__global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int fuse) {
   if (X.counters[kCFlags] & kFAbort) return;
   const int s = P.lvl_sn[lo + blockIdx.x];
   const int64_t roff = X.sn_roff[s];
   const int nd = X.sn_nd[s], f = X.sn_f[s], fsym = P.sn_fsym[s];
+  if (f <= fuse && !P.sn_large[s]) return;
   int *rows = X.rows + roff;
   for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
     const int c = P.child_idx[t];
@@ -405,7 +408,7 @@ __device__ int spd_front_panels(FrontRef &v, const PivotParams &prm, FrontShared
       for (int k = 0; k < NB; ++k) {
         if (k < np && i > ps + k) {
           const double w = a[k];
-          W[(size_t)k * sf + i] = w;
+          W[(size_t)k * f + i] = w;
 #pragma unroll
           for (int j = k + 1; j < NB; ++j) {
             if (j < nbp && ps + j <= i) {
@@ -456,7 +459,7 @@ __device__ void factor_one_front(DevPlan &P, DevFactor &X, int s, const PivotPar
   PivotParams prm = prm0;
   prm.eff_small = __longlong_as_double((long long)X.counters[kCEffSmall]);
   FrontRef v;
-  v.ld = f;
+  v.ld = SMEM ? f | 1 : f;  // (odd: rows of the front without bank conflicts)
   v.f = f;
   v.ne = ne;
   int *inv;
@@ -465,12 +468,23 @@ __device__ void factor_one_front(DevPlan &P, DevFactor &X, int s, const PivotPar
     // memory holds W only for buckets that can reach it), then the ints
     const bool blocked = f >= prm0.blocked_min_front && nb > 1;
     double *F = smem;
-    double *W = F + sf * sf;
+    double *W = F + sf * v.ld;
     int *rows = (int *)(W + (blocked ? sf * nb : 0));
     int *loc = rows + f;
     inv = loc + f;
     int8_t *tags = (int8_t *)(inv + f);
-    for (size_t t = threadIdx.x; t < sf * sf; t += NT) F[t] = Fg[t];
+    // the lower part, a warp per column, four columns in flight
+    constexpr int NWF = NT / 32;
+    const int lane = threadIdx.x & 31;
+    for (int j0 = threadIdx.x >> 5; j0 < f; j0 += 4 * NWF)
+      for (int i = j0 + lane; i < f; i += 32) {
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = (j0 + u * NWF <= i) ? Fg[(size_t)(j0 + u * NWF) * f + i] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (j0 + u * NWF <= i) F[(size_t)(j0 + u * NWF) * v.ld + i] = x[u];
+      }
     for (int t = threadIdx.x; t < f; t += NT) {
       rows[t] = rows_g[t];
       loc[t] = t;
@@ -504,7 +518,7 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
                             const PivotParams &prm, FrontShared &sh, int *inv, double *Fg,
                             int *rows_g, int8_t *tags_g) {
   const int f = v.f, ne = v.ne;
-  const size_t sf = (size_t)f;
+  const size_t sf = (size_t)v.ld;
   const bool is_root = P.sn_parent[s] < 0;
   int pstore = p;
   if (is_root && p < ne) {
@@ -516,16 +530,12 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
   if (prm.posdef) {
     if (p < ne && threadIdx.x == 0) set_flag(X.counters, kFNotPosdef);
     // L = L_unit sqrt(D), upper part zero
-    for (long long t = threadIdx.x; t < (long long)pstore * f; t += NT) {
-      const int c = (int)(t / f), i = (int)(t % f);
+    // (a warp per column: its square root taken once)
+    for (int c = threadIdx.x >> 5; c < pstore; c += NT / 32) {
       double *Lc = v.F + (size_t)c * sf;
-      if (i < c) Lc[i] = 0.0;
-      else if (i > c) Lc[i] = __dmul_rn(Lc[i], sqrt(Lc[c]));
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < pstore; c += NT) {
-      double *Lc = v.F + (size_t)c * sf;
-      Lc[c] = sqrt(Lc[c]);
+      const double sq = sqrt(Lc[c]);
+      __syncwarp();
+      for (int i = threadIdx.x & 31; i < f; i += 32) Lc[i] = i < c ? 0.0 : i == c ? sq : __dmul_rn(Lc[i], sq);
     }
   } else {
     // D inline: d on the diagonal, a 2x2 block's off-diagonal in the upper
@@ -545,23 +555,19 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
       }
     }
     __syncthreads();
-    for (long long t = threadIdx.x; t < (long long)pstore * f; t += NT) {
-      const int c = (int)(t / f), i = (int)(t % f);
+    for (int c = threadIdx.x >> 5; c < pstore; c += NT / 32) {
       double *Lc = v.F + (size_t)c * sf;
       const int8_t tag = v.tags[c];
-      if (tag == 0) {
-        if (i >= c) Lc[i] = 0.0;
-        else Lc[i] = 0.0;
-      } else if (i < c) {
-        if (!(tag == -1 && i == c - 1)) Lc[i] = 0.0;
-      } else if (tag == 2 && i == c + 1) {
-        Lc[i] = 0.0;
-      }
+      const int end = tag == 0 ? f : tag == 2 ? c + 2 : c;  // rows past it keep their values
+      for (int i = threadIdx.x & 31; i < end; i += 32)
+        if (tag == 0 || (i != c && !(tag == -1 && i == c - 1))) Lc[i] = 0.0;
     }
   }
   __syncthreads();
   if (SMEM) {
-    for (size_t t = threadIdx.x; t < sf * sf; t += NT) Fg[t] = v.F[t];
+    // the pivot columns whole, the contribution block's lower part
+    for (int c = threadIdx.x >> 5; c < f; c += NT / 32)
+      for (int i = (c < pstore ? 0 : c) + (int)(threadIdx.x & 31); i < f; i += 32) Fg[(size_t)c * f + i] = v.F[c * sf + i];
     for (int t = threadIdx.x; t < f; t += NT) {
       rows_g[t] = v.rows[t];
       tags_g[t] = v.tags[t];
@@ -590,13 +596,14 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
   }
 }
 
-template <int NT, int FMIN, int FMAX, bool SMEM>
-__global__ void __launch_bounds__(NT) k_factor(DevPlan P, DevFactor X, int lo, int hi, PivotParams prm) {
+// Fronts of fmin..fmax rows among P.lvl_sn[i0 + block].
+template <int NT, bool SMEM>
+__global__ void __launch_bounds__(NT) k_factor(DevPlan P, DevFactor X, int i0, PivotParams prm, int fmin, int fmax) {
   extern __shared__ __align__(16) double smem[];
   if (X.counters[kCFlags] & kFAbort) return;
-  const int s = P.lvl_sn[lo + blockIdx.x];
+  const int s = P.lvl_sn[i0 + blockIdx.x];
   const int f = X.sn_f[s];
-  if (f < FMIN || f > FMAX || P.sn_large[s]) return;
+  if (f < fmin || f > fmax || P.sn_large[s]) return;
   if (!SMEM && prm.aptp_min > 0 && !prm.posdef && f >= prm.aptp_min && prm.u >= kWeakPivotRatio) {
     // delays took the front to the APTP size: it must take the large-front
     // path; recorded, and the factorization is redone

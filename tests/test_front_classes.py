@@ -1,0 +1,139 @@
+"""The front kernels by size class on a B200, bit for bit against the oracle:
+single dense fronts at the edges of the classes, SPD and indefinite (zero
+diagonal blocks force 2x2 pivots and failing candidates), a front with more
+children than the fused kernel describes at a time, chains of fronts that
+delay columns, a matrix that is not positive definite, and a blocked size
+below the fused kernel's.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from opt_solver_b200 import smfg
+from opt_solver_b200 import workloads as W
+from oracle import oracle as O
+from tests.cases import dense_lower
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _built(oracle_lib):
+    return oracle_lib
+
+
+def _spd(n, rng):
+    G = rng.standard_normal((n, n))
+    return G @ G.T + n * np.eye(n)
+
+
+def _indefinite(n, rng):
+    """Mixed signs, a third of the diagonal zero, some zero entries."""
+    A = rng.standard_normal((n, n))
+    A = A + A.T
+    A[rng.random((n, n)) < 0.2] = 0.0
+    A = np.tril(A) + np.tril(A, -1).T
+    z = rng.permutation(n)[: n // 3]
+    A[z, z] = 0.0
+    return A
+
+
+def _compare(a, sv, info, v, posdef, scale=None, **oracle_kw):
+    ox = O.restated_factorize(a, O.permuted_values(a, v, scale), posdef, **oracle_kw)
+    gx = sv.export()
+    assert info.delayed_pivots == ox.delayed and info.two_by_two_pivots == ox.two_by_two
+    assert info.flops == ox.flops
+    if not posdef:
+        assert info.inertia == ox.inertia
+    for s in range(a.nsn):
+        assert gx.f[s] == ox.f[s] and gx.p[s] == ox.p[s], s
+        assert np.array_equal(gx.front_rows(s), ox.front_rows(s)), s
+        assert np.array_equal(gx.block(s), ox.block(s)), s
+    if not posdef:
+        nt = int(np.sum(gx.p))
+        assert np.array_equal(gx.tags[:nt], ox.tags[:nt])
+
+
+def _run(n, cp, ri, v, posdef, nemin=8, ordering=smfg.ORDER_ND):
+    a = smfg.analyse(n, cp, ri, ordering=ordering, nemin=nemin)
+    sv = smfg.Solver(a, device=0)
+    info = sv.factor(v, posdef=posdef)
+    _compare(a, sv, info, v, posdef)
+    sv.close()
+    return a, info
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129])
+@pytest.mark.parametrize("posdef", [True, False])
+def test_dense_front(n, posdef):
+    rng = np.random.default_rng(1000 + n)
+    A = _spd(n, rng) if posdef else _indefinite(n, rng)
+    a, _ = _run(*dense_lower(A), posdef, ordering=smfg.ORDER_NATURAL)
+    assert int(np.diff(a.front_row_ptr).max()) == n
+
+
+@pytest.mark.parametrize("posdef", [True, False])
+def test_many_children(posdef):
+    """40 leaves of one column under one root: three batches of children."""
+    rng = np.random.default_rng(5)
+    k, m = 40, 12
+    n = k + m
+    A = np.zeros((n, n))
+    A[k:, k:] = _spd(m, rng) if posdef else _indefinite(m, rng)
+    A[k:, :k] = rng.standard_normal((m, k))
+    A[:k, k:] = A[k:, :k].T
+    A[np.arange(k), np.arange(k)] = 4.0 * n if posdef else rng.standard_normal(k)
+    A[np.arange(k, n), np.arange(k, n)] += 4.0 * n if posdef else 0.0
+    rows, cols = np.nonzero(np.tril(A))
+    keep = (rows >= k) | (rows == cols)
+    rows, cols = rows[keep], cols[keep]
+    order = np.lexsort((rows, cols))
+    cp = np.zeros(n + 1, np.int32)
+    np.add.at(cp, cols + 1, 1)
+    a, _ = _run(n, np.cumsum(cp).astype(np.int32), rows[order].astype(np.int32), A[rows, cols][order], posdef,
+                nemin=1, ordering=smfg.ORDER_NATURAL)
+    assert int(np.diff(a.child_ptr).max()) > 32
+
+
+@pytest.mark.parametrize("T", [3, 30, 90])
+def test_delaying_chain(T):
+    n, cp, ri, v = W.trajectory_kkt(T, np.random.default_rng(T))
+    _, info = _run(n, cp, ri, v, False)
+    assert info.delayed_pivots > 0 and info.two_by_two_pivots > 0
+
+
+def test_grid_levels():
+    _run(*W.laplacian_2d(61, 47), True)
+
+
+def test_not_positive_definite():
+    A = _spd(50, np.random.default_rng(2))
+    A[37, 37] = -1.0
+    n, cp, ri, v = dense_lower(A)
+    a = smfg.analyse(n, cp, ri)
+    sv = smfg.Solver(a, device=0)
+    info = sv.factor(v, posdef=True)
+    assert info.factor_status == smfg.SMFG_FACTOR_NOT_POSDEF
+    sv.close()
+
+
+@pytest.mark.parametrize("blocked", [20, 40, 96, 200])
+@pytest.mark.parametrize("posdef", [True, False])
+def test_blocked_min_front(blocked, posdef):
+    """A blocked size below or above the default moves the classes' edges."""
+    rng = np.random.default_rng(8)
+    for n in (19, 20, 39, 40, 70, 96, 100):
+        A = _spd(n, rng) if posdef else _indefinite(n, rng)
+        n, cp, ri, v = dense_lower(A)
+        a = smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL)
+        sv = smfg.Solver(a, device=0)
+        c = smfg.default_control(posdef)
+        c.blocked_min_front = blocked
+        info = smfg.Info()
+        val = np.ascontiguousarray(v)
+        rc = smfg.lib().smfg_factor(sv._h, val.ctypes.data, C.byref(c), C.byref(info))
+        assert rc in (smfg.SMFG_OK, smfg.SMFG_ERR_SINGULAR)
+        sv.posdef, sv.info = posdef, info
+        _compare(a, sv, info, v, posdef, blocked_min_front=blocked)
+        sv.close()
