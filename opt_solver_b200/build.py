@@ -20,7 +20,8 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libsmfg.so")
 SOURCES = ["smfg_engine.cu", "smfg_aptp.cu", "smfg_analyse.cpp", "smfg_scaling.cpp", "smfg_mlp.cu"]
-DEPS = ["smfg_front.cuh", "smfg_kernels.cuh", "smfg_small.cuh", "smfg_internal.cuh", "smfg_tc.cuh", "smfg_aptp.cuh",
+DEPS = ["smfg_front.cuh", "smfg_kernels.cuh", "smfg_small.cuh", "smfg_solve.cuh",
+        "smfg_internal.cuh", "smfg_tc.cuh", "smfg_aptp.cuh",
         "smfg_aptp_host.h"]
 
 

@@ -12,6 +12,7 @@
 
 #include "smfg_kernels.cuh"
 #include "smfg_small.cuh"
+#include "smfg_solve.cuh"
 #include "smfg_tc.cuh"
 
 namespace smfg {
@@ -703,6 +704,14 @@ static void ensure_tri_inv(Plan &pl) {
   pl.x.tri_inv = dalloc<double>(pl, (size_t)tot);
 }
 
+// First position in level l's list (largest symbolic front first) of a front
+// of at most v symbolic rows.
+static int level_at_most(const Plan &pl, int l, int v) {
+  const auto b = pl.h_lvl_sn.begin();
+  return (int)(std::partition_point(b + pl.lvl_ptr[l], b + pl.lvl_ptr[l + 1],
+                                    [&](int s) { return pl.h_fsym[s] > v; }) - b);
+}
+
 // Threads of the fused front kernel's blocks (fronts of 33..64 rows, of
 // 65..95; a warp below). Half as many: 9% slower on one small trajectory KKT;
 // twice as many: 12% slower on a batch of 256 (fewer fronts resident).
@@ -729,11 +738,7 @@ static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, in
   cudaStream_t st = pl.stream;
   const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
   const bool exact = c.posdef || l == 0;
-  // first list position of at most v symbolic rows
-  auto at_most = [&](int v) {
-    return (int)(std::partition_point(pl.h_lvl_sn.begin() + lo, pl.h_lvl_sn.begin() + hi,
-                                      [&](int s) { return pl.h_fsym[s] > v; }) - pl.h_lvl_sn.begin());
-  };
+  auto at_most = [&](int v) { return level_at_most(pl, l, v); };
   enum Kind { kGlobal, kMedium, kUpper, kSmall, kWarp };
   struct Class { Kind kind; int fmin, fmax, i0, n; };
   Class cls[6];
@@ -1280,13 +1285,13 @@ static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int jo
 
 // Up to kSolveRhs right-hand sides per sweep (the large fronts' block
 // kernels keep that many columns of the block's values in shared memory).
-constexpr int kSolveRhs = 8;
-
 static void enqueue_solve(Plan &pl, double *d_b, int nrhs, int ldb, int job, bool scaled, LaunchCount &lc) {
   static bool attrs = false;
   if (!attrs) {
     SMFG_CUDA(cudaFuncSetAttribute(k_fwd_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TriSmem)));
     SMFG_CUDA(cudaFuncSetAttribute(k_bwd_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TriSmem)));
+    SMFG_CUDA(cudaFuncSetAttribute(k_fwd_level, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvlSmem));
+    SMFG_CUDA(cudaFuncSetAttribute(k_bwd_level, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvlSmem));
     attrs = true;
   }
   for (int r0 = 0; r0 < nrhs; r0 += kSolveRhs)
@@ -1310,6 +1315,15 @@ static void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem,
   cfg.numAttrs = 1;
   SMFG_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
 }
+
+// The level kernels' blocks: tiny fronts eight to a block where the realized
+// rows are the symbolic ones (SPD, and the leaves), every other front its own.
+static LevelGrid level_grid(const Plan &pl, int l) {
+  const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
+  const int ic = (pl.posdef || l == 0) ? level_at_most(pl, l, kTinyRows) : hi;
+  return {lo, ic - lo, ic, hi - ic};
+}
+static int level_blocks(const LevelGrid &g) { return g.n + (g.nc + kLvlWarps - 1) / kLvlWarps; }
 
 static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int job, bool scaled, LaunchCount &lc) {
   DevPlan &d = pl.d;
@@ -1335,10 +1349,9 @@ static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int jo
   const int lgrid = 2 * sms;
   if (fwd) {
     for (int l = 0; l < pl.nlevels; ++l) {
-      const int lo = pl.lvl_ptr[l], m = pl.lvl_ptr[l + 1] - lo;
-      launch_pdl(k_fwd_small, (m + 7) / 8, 256, 0, st, d, x, lo, m, pl.posdef, xv, wk, rows_total, nrhs);
-      launch_pdl(k_fwd_front, m, kSolveNT, 0, st, d, x, lo, pl.posdef, xv, wk, rows_total, nrhs);
-      lc.n += 2;
+      const LevelGrid lv = level_grid(pl, l);
+      launch_pdl(k_fwd_level, level_blocks(lv), kLvlNT, kLvlSmem, st, d, x, lv, pl.posdef, xv, wk, rows_total, nrhs);
+      lc.n += 1;
       const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
       if (nL > 0) {
         const int *lg = d.lvl_large + pl.lvl_large_ptr[l];
@@ -1353,16 +1366,15 @@ static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int jo
   }
   if (use_lt || (use_d && !pl.posdef)) {
     for (int l = pl.nlevels - 1; l >= 0; --l) {
-      const int lo = pl.lvl_ptr[l], m = pl.lvl_ptr[l + 1] - lo;
       const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
       if (nL > 0 && use_lt) {
         launch_pdl(k_bwd_l21, lgrid, 256, 0, st, d, x, d.lvl_large + pl.lvl_large_ptr[l], nL, xv, wk, rows_total, nrhs);
         lc.n++;
       }
-      launch_pdl(k_bwd_small, (m + 7) / 8, 256, 0, st, d, x, lo, m, pl.posdef, xv, nrhs, use_d ? 1 : 0, use_lt ? 1 : 0);
-      launch_pdl(k_bwd_front, m, kSolveNT, 0, st, d, x, lo, pl.posdef, xv, wk, rows_total, nrhs, use_d ? 1 : 0,
-                 use_lt ? 1 : 0);
-      lc.n += 2;
+      const LevelGrid lv = level_grid(pl, l);
+      launch_pdl(k_bwd_level, level_blocks(lv), kLvlNT, kLvlSmem, st, d, x, lv, pl.posdef, xv, wk, rows_total, nrhs,
+                 use_d ? 1 : 0, use_lt ? 1 : 0);
+      lc.n += 1;
       if (nL > 0 && use_lt) {
         const int *lg = d.lvl_large + pl.lvl_large_ptr[l];
         const int nb = (large_pmax(pl, l) + kSB - 1) / kSB;

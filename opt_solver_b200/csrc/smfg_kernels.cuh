@@ -1848,25 +1848,11 @@ __global__ void k_solve_scatter(double *__restrict__ b, int ldb, int nrhs, int n
 // Solves by level. Each front's work vector w (length f, at the front's row
 // offset) holds its pivot rows' values and, in the forward sweep, its update
 // vector for the parent (rows p..f); x (new numbering) holds the pivot
-// results. Large fronts (symbolic rows >= kLargeMin) leave their L21 part
-// to the multi-block kernels k_fwd_l21 / k_bwd_l21. Sums run in a fixed
-// order (deterministic); solve_forward.cpp:116-293 and
-// solve_backward.cpp:135-350 compute the same quantities.
-constexpr int kSolveNT = 128;
+// results. Large fronts (symbolic rows >= kLargeMin) take the multi-block
+// kernels below; the others' sweeps are in smfg_solve.cuh.
 
-// The 32 x 32 lower block L[jb:jb+nb, jb:jb+nb) staged in shared memory
-// (coalesced column reads) for the warp triangle solves below.
-template <int NT>
-__device__ __forceinline__ void load_tri32(const double *L, size_t sf, int jb, int nb, double (*Ls)[33]) {
-  __syncthreads();
-  for (int t = threadIdx.x; t < 1024; t += NT) {
-    const int r = t & 31, c = t >> 5;
-    Ls[r][c] = (r < nb && c < nb && c <= r) ? L[(size_t)(jb + c) * sf + jb + r] : 0.0;
-  }
-  __syncthreads();
-}
-
-// The same triangle copied asynchronously (8-byte cp.async, zero fill
+// The 32 x 32 lower block L[jb:jb+nb, jb:jb+nb) copied to shared memory
+// asynchronously (8-byte cp.async, zero fill
 // outside the lower triangle); the caller waits with cp_async_wait_all()
 // and a barrier before reading Ls.
 template <int NT>
@@ -1929,9 +1915,6 @@ __device__ __forceinline__ void tri_bwd_warp(double *v, int jb, int nb, int posd
   if (lane < nb) v[jb + lane] = vi;
 }
 
-// Fronts of at most this many rows take the warp-per-front solve kernels.
-constexpr int kSolveSmall = 64;
-
 // D^-1 of the 2x2 pivot [d00 d10; d10 d11] applied to (r0, r1) by the scaled
 // Cramer rule (solve_diag.cpp:49-123); zero for a singular block.
 __device__ __forceinline__ void dinv2_apply(double d00, double d10, double d11, double r0, double r1, double &z0,
@@ -1958,308 +1941,6 @@ __device__ __forceinline__ void dinv2_apply(double d00, double d10, double d11, 
         }
       }
     }
-  }
-}
-
-// Forward sweep of the level's fronts of at most kSolveSmall rows, a warp
-// per front (no block barriers; eight fronts a block): gather, the
-// children's update vectors in child order, then column by column over the
-// whole front (the unit, or SPD non-unit, L11 solve and w[p:f) -= L21
-// w[0:p) in one pass), the front's L columns loaded eight at a time ahead
-// of their use.
-__global__ void __launch_bounds__(256, 4) k_fwd_small(DevPlan P, DevFactor X, int lo, int m, int posdef, double *x,
-                                                   double *wk, int64_t rows_total, int nrhs) {
-  __shared__ double sw_all[8][kSolveSmall];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int item = blockIdx.x * 8 + wid;
-  if (item >= m) return;
-  const int s = P.lvl_sn[lo + item];
-  const int f = X.sn_f[s];
-  if (f > kSolveSmall || P.sn_large[s]) return;
-  pdl_wait();
-  pdl_trigger();
-  const int p = X.sn_pstore[s];
-  const int64_t roff = X.sn_roff[s];
-  const int *rows = X.rows + roff;
-  const double *L = X.arena + X.sn_off[s];
-  double *sw = sw_all[wid];
-  for (int r = 0; r < nrhs; ++r) {
-    double *w = wk + (int64_t)r * rows_total + roff;
-    double *xr = x + (int64_t)r * P.n;
-    for (int i = lane; i < f; i += 32) sw[i] = (i < p) ? xr[rows[i]] : 0.0;
-    __syncwarp();
-    for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
-      const int c = P.child_idx[t];
-      const int pc = X.sn_pstore[c], q = X.sn_f[c] - pc;
-      const int *cmap = X.cbmap + X.sn_roff[c] + pc;
-      const double *wc = wk + (int64_t)r * rows_total + X.sn_roff[c] + pc;
-      for (int i = lane; i < q; i += 32) sw[cmap[i]] += wc[i];
-      __syncwarp();
-    }
-    // rows lane and lane + 32
-    double w0 = (lane < f) ? sw[lane] : 0.0, w1 = (lane + 32 < f) ? sw[lane + 32] : 0.0;
-    for (int j0 = 0; j0 < p; j0 += 8) {
-      double l0[8], l1[8], dj[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u;
-        const bool in = j < p;
-        l0[u] = (in && lane > j && lane < f) ? __ldg(L + (size_t)j * f + lane) : 0.0;
-        l1[u] = (in && lane + 32 < f) ? __ldg(L + (size_t)j * f + lane + 32) : 0.0;
-        dj[u] = (in && posdef) ? __ldg(L + (size_t)j * f + j) : 1.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int j = j0 + u;
-        if (j >= p) break;
-        // w_j of the row's owner lane
-        double wj = __shfl_sync(0xffffffffu, j < 32 ? w0 : w1, j & 31);
-        if (posdef) wj = wj / dj[u];
-        if (lane == j) w0 = wj;
-        if (lane + 32 == j) w1 = wj;
-        if (l0[u] != 0.0) w0 = fma(-l0[u], wj, w0);
-        if (l1[u] != 0.0 && lane + 32 > j) w1 = fma(-l1[u], wj, w1);
-      }
-    }
-    if (lane < f) w[lane] = w0;
-    if (lane + 32 < f) w[lane + 32] = w1;
-    if (lane < p) xr[rows[lane]] = w0;
-    if (lane + 32 < p) xr[rows[lane + 32]] = w1;
-    __syncwarp();
-  }
-}
-
-// Backward sweep of the level's fronts of at most kSolveSmall rows, a warp
-// per front: D^-1 of every pivot block (2x2 blocks where the upper slot (c,
-// c+1) is nonzero), v -= L21^T x_ext, then L11^-T from the last column on
-// (each column's dot with the solved part a warp reduction).
-__global__ void __launch_bounds__(256, 4) k_bwd_small(DevPlan P, DevFactor X, int lo, int m, int posdef, double *x,
-                                                   int nrhs, int apply_d, int apply_lt) {
-  __shared__ double sv_all[8][kSolveSmall];
-  __shared__ double sx_all[8][kSolveSmall];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int item = blockIdx.x * 8 + wid;
-  if (item >= m) return;
-  const int s = P.lvl_sn[lo + item];
-  const int f = X.sn_f[s];
-  if (f > kSolveSmall || P.sn_large[s]) return;
-  pdl_wait();
-  pdl_trigger();
-  const int p = X.sn_pstore[s];
-  const int *rows = X.rows + X.sn_roff[s];
-  const double *L = X.arena + X.sn_off[s];
-  const size_t sf = (size_t)f;
-  double *sv = sv_all[wid], *sx = sx_all[wid];
-  for (int r = 0; r < nrhs; ++r) {
-    double *xr = x + (int64_t)r * P.n;
-    for (int i = lane; i < f; i += 32) sx[i] = (i >= p) ? xr[rows[i]] : 0.0;
-    for (int c = lane; c < p; c += 32) {
-      const bool second = apply_d && !posdef && c > 0 && L[(size_t)c * sf + c - 1] != 0.0;
-      if (second) continue;
-      double y0 = xr[rows[c]];
-      if (!posdef && apply_d) {
-        const double d00 = L[(size_t)c * sf + c];
-        const double d10 = (c + 1 < p) ? L[(size_t)(c + 1) * sf + c] : 0.0;
-        if (d10 != 0.0) {
-          double z0, z1;
-          dinv2_apply(d00, d10, L[(size_t)(c + 1) * sf + c + 1], y0, xr[rows[c + 1]], z0, z1);
-          sv[c] = z0;
-          sv[c + 1] = z1;
-          continue;
-        }
-        y0 = (d00 == 0.0 || !isfinite(d00)) ? 0.0 : y0 / d00;
-      }
-      sv[c] = y0;
-    }
-    __syncwarp();
-    if (apply_lt) {
-      // v[c] -= L(p:f, c)^T x_ext: a lane per column
-      for (int c = lane; c < p; c += 32) {
-        const double *Lc = L + (size_t)c * sf;
-        double acc = 0.0;
-        for (int i = p; i < f; ++i) acc = fma(Lc[i], sx[i], acc);
-        sv[c] -= acc;
-      }
-      __syncwarp();
-      // L11^-T, last column first: x_j = (v_j - L(j+1:p, j)^T x) / L_jj
-      for (int j = p - 1; j >= 0; --j) {
-        const double *Lj = L + (size_t)j * sf;
-        double acc = 0.0;
-        for (int i = j + 1 + lane; i < p; i += 32) acc = fma(Lj[i], sx[i], acc);
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
-          double xj = sv[j] - acc;
-          if (posdef) xj = xj / Lj[j];
-          sx[j] = xj;
-        }
-        __syncwarp();
-      }
-    } else {
-      for (int c = lane; c < p; c += 32) sx[c] = sv[c];
-      __syncwarp();
-    }
-    for (int c = lane; c < p; c += 32) xr[rows[c]] = sx[c];
-    __syncwarp();
-  }
-}
-
-// Forward sweep of one level: gather, children's update vectors in child
-// order, blocked unit (indefinite) or non-unit (SPD) L11 solve, then
-// w[p:f) -= L21 w[0:p) unless the front is large. Fronts of at most
-// kSolveSmall rows are k_fwd_small's.
-__global__ void __launch_bounds__(kSolveNT, 4) k_fwd_front(DevPlan P, DevFactor X, int lo, int posdef,
-                                                        double *x, double *wk, int64_t rows_total,
-                                                        int nrhs) {
-  const int s = P.lvl_sn[lo + blockIdx.x];
-  const int f = X.sn_f[s], p = X.sn_pstore[s];
-  const int64_t roff = X.sn_roff[s];
-  const int *rows = X.rows + roff;
-  const double *L = X.arena + X.sn_off[s];
-  const size_t sf = (size_t)f;
-  const bool large = P.sn_large[s] != 0;
-  if (!large && f <= kSolveSmall) return;  // k_fwd_small's
-  pdl_wait();
-  pdl_trigger();
-  __shared__ double Ls[32][33];
-  const int warp = threadIdx.x >> 5;
-  // every right-hand side at once: gather, children's update vectors in
-  // child order, then per 32-column strip the triangle (a warp per
-  // right-hand side) and the rows below (each L entry loaded once for all)
-  // (four rows a thread in flight: a large front's gather and children's
-  // vectors are thousands of rows for one block)
-  for (int r = 0; r < nrhs; ++r) {
-    double *w = wk + (int64_t)r * rows_total + roff;
-    const double *xr = x + (int64_t)r * P.n;
-    for (int i0 = threadIdx.x; i0 < f; i0 += 4 * kSolveNT) {
-      double v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * kSolveNT;
-        v[u] = (i < p) ? xr[rows[i]] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (i0 + u * kSolveNT < f) w[i0 + u * kSolveNT] = v[u];
-    }
-  }
-  __syncthreads();
-  for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
-    const int c = P.child_idx[t];
-    const int pc = X.sn_pstore[c], q = X.sn_f[c] - pc;
-    const int *cmap = X.cbmap + X.sn_roff[c] + pc;
-    for (int r = 0; r < nrhs; ++r) {
-      double *w = wk + (int64_t)r * rows_total + roff;
-      const double *wc = wk + (int64_t)r * rows_total + X.sn_roff[c] + pc;
-      for (int i0 = threadIdx.x; i0 < q; i0 += 4 * kSolveNT) {
-        double v[4], o[4];
-        int m[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + u * kSolveNT;
-          m[u] = (i < q) ? cmap[i] : 0;
-          v[u] = (i < q) ? wc[i] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) o[u] = (i0 + u * kSolveNT < q) ? w[m[u]] : 0.0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (i0 + u * kSolveNT < q) w[m[u]] = o[u] + v[u];
-      }
-    }
-    __syncthreads();
-  }
-  if (large) return;  // the block kernels (k_fwd_tri / k_fwd_gemv) go on
-  for (int jb = 0; jb < p; jb += 32) {
-    const int nb = min(32, p - jb);
-    // the strip's triangle and this thread's first row below it loaded
-    // before the barriers and the triangle solves (in flight meanwhile)
-    double tv[1024 / kSolveNT];
-#pragma unroll
-    for (int u = 0; u < 1024 / kSolveNT; ++u) {
-      const int t = (int)threadIdx.x + kSolveNT * u, r = t & 31, c = t >> 5;
-      tv[u] = (r < nb && c < nb && c <= r) ? __ldg(L + (size_t)(jb + c) * sf + jb + r) : 0.0;
-    }
-    const int i1 = jb + nb + (int)threadIdx.x;
-    double l[32];
-#pragma unroll
-    for (int u = 0; u < 32; ++u) l[u] = (i1 < f && u < nb) ? __ldg(L + (size_t)(jb + u) * sf + i1) : 0.0;
-    __syncthreads();  // the previous strip's readers of Ls and the vectors are done
-#pragma unroll
-    for (int u = 0; u < 1024 / kSolveNT; ++u) {
-      const int t = (int)threadIdx.x + kSolveNT * u;
-      Ls[t & 31][t >> 5] = tv[u];
-    }
-    __syncthreads();
-    for (int r = warp; r < nrhs; r += kSolveNT / 32) tri_fwd_warp(wk + (int64_t)r * rows_total + roff, jb, nb, posdef, Ls);
-    __syncthreads();
-    for (int i = i1; i < f; i += kSolveNT) {
-      if (i != i1) {
-        const double *li = L + (size_t)jb * sf + i;
-#pragma unroll
-        for (int u = 0; u < 32; ++u) l[u] = (u < nb) ? __ldg(li + (size_t)u * sf) : 0.0;
-      }
-      for (int r = 0; r < nrhs; ++r) {
-        double *w = wk + (int64_t)r * rows_total + roff;
-        double acc = 0.0;
-#pragma unroll
-        for (int u = 0; u < 32; ++u)
-          if (u < nb) acc = fma(l[u], w[jb + u], acc);
-        w[i] -= acc;
-      }
-    }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < p * nrhs; t += kSolveNT) {
-    const int r = nrhs == 1 ? 0 : t / p, i = nrhs == 1 ? t : t - r * p;
-    x[(int64_t)r * P.n + rows[i]] = wk[(int64_t)r * rows_total + roff + i];
-  }
-}
-
-// w[p:f) -= L21 w[0:p) of the level's large fronts, rows split over blocks.
-__global__ void __launch_bounds__(256) k_fwd_l21(DevPlan P, DevFactor X, const int *__restrict__ large,
-                                                 int nlarge, double *wk, int64_t rows_total, int nrhs) {
-  __shared__ double ws[256];
-  __shared__ int pref[65];
-  for (int chunk = 0; chunk < nlarge; chunk += 64) {
-    const int cnt = min(64, nlarge - chunk);
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) {
-        const int s = large[chunk + q];
-        pref[q + 1] = pref[q] + (X.sn_f[s] - X.sn_pstore[s] + 255) / 256 * nrhs;
-      }
-    }
-    __syncthreads();
-    const int total = pref[cnt];
-    for (int wi = blockIdx.x; wi < total; wi += gridDim.x) {
-      int a = 0, b = cnt;
-      while (b - a > 1) {
-        const int mid = (a + b) >> 1;
-        if (pref[mid] <= wi) a = mid;
-        else b = mid;
-      }
-      const int s = large[chunk + a];
-      const int f = X.sn_f[s], p = X.sn_pstore[s];
-      const int nchunks = (f - p + 255) / 256;
-      const int item = wi - pref[a];
-      const int r = item / nchunks, rc = item % nchunks;
-      double *w = wk + (int64_t)r * rows_total + X.sn_roff[s];
-      const double *L = X.arena + X.sn_off[s];
-      const size_t sf = (size_t)f;
-      const int i = p + rc * 256 + threadIdx.x;
-      double acc = (i < f) ? w[i] : 0.0;
-      for (int j0 = 0; j0 < p; j0 += 256) {
-        const int nj = min(256, p - j0);
-        __syncthreads();
-        if (threadIdx.x < nj) ws[threadIdx.x] = w[j0 + threadIdx.x];
-        __syncthreads();
-        if (i < f)
-          for (int j = 0; j < nj; ++j) acc = fma(-L[(size_t)(j0 + j) * sf + i], ws[j], acc);
-      }
-      if (i < f) w[i] = acc;
-      __syncthreads();
-    }
-    __syncthreads();
   }
 }
 
@@ -2330,150 +2011,6 @@ __global__ void __launch_bounds__(256) k_bwd_l21(DevPlan P, DevFactor X, const i
         if (lane == 0 && jw + c < p) wk[(int64_t)r * rows_total + X.sn_roff[s] + jw + c] = v;
       }
     }
-  }
-}
-
-// Backward sweep of one level: v = D^-1 w_piv (indefinite, apply_inline_d
-// with solve_2x2_scaled's scaled Cramer rule, solve_backward.cpp:135-171,
-// pivoting.cpp:30-62), v -= L21^T x_ext (here for small fronts, from
-// k_bwd_l21 for large ones), then the blocked L11^-T solve.
-__global__ void __launch_bounds__(kSolveNT) k_bwd_front(DevPlan P, DevFactor X, int lo, int posdef,
-                                                        double *x, double *wk, int64_t rows_total,
-                                                        int nrhs, int apply_d, int apply_lt) {
-  const int s = P.lvl_sn[lo + blockIdx.x];
-  const int f = X.sn_f[s], p = X.sn_pstore[s];
-  const int64_t roff = X.sn_roff[s];
-  const int *rows = X.rows + roff;
-  const double *L = X.arena + X.sn_off[s];
-  const size_t sf = (size_t)f;
-  const bool large = P.sn_large[s] != 0;
-  if (!large && f <= kSolveSmall) return;  // k_bwd_small's
-  pdl_wait();
-  pdl_trigger();
-  __shared__ double Ls[32][33];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // every right-hand side at once. D^-1 of each pivot block; 2x2 blocks
-  // start where the upper slot (c, c+1) is nonzero. (large: v[0:p) holds
-  // L21^T x_ext)
-  for (int t = threadIdx.x; t < p * nrhs; t += kSolveNT) {
-    const int r = nrhs == 1 ? 0 : t / p, c = nrhs == 1 ? t : t - r * p;
-    double *v = wk + (int64_t)r * rows_total + roff;
-    const double *xr = x + (int64_t)r * P.n;
-    const bool second = apply_d && !posdef && (c > 0) && L[(size_t)c * sf + c - 1] != 0.0;
-    if (second) continue;
-    double y0 = xr[rows[c]];
-    if (!posdef && apply_d) {
-      const double d00 = L[(size_t)c * sf + c];
-      const double d10 = (c + 1 < p) ? L[(size_t)(c + 1) * sf + c] : 0.0;
-      if (d10 != 0.0) {
-        const double d11 = L[(size_t)(c + 1) * sf + c + 1];
-        const double r0 = y0, r1 = xr[rows[c + 1]];
-        const double s2 = max3_ref(fabs(d00), fabs(d10), fabs(d11));
-        double z0 = 0.0, z1 = 0.0;
-        if (isfinite(s2) && s2 != 0.0) {
-          const double a = d00 / s2, bb = d10 / s2, cc = d11 / s2;
-          const double det = __dsub_rn(__dmul_rn(a, cc), __dmul_rn(bb, bb));
-          if (isfinite(det) && det != 0.0) {
-            if (!isfinite(r0) || !isfinite(r1)) {
-              z0 = r0;
-              z1 = r1;
-            } else {
-              const double rs = fmax(fabs(r0), fabs(r1));
-              if (rs != 0.0) {
-                const double q0 = r0 / rs, q1 = r1 / rs;
-                const double u0 = __dsub_rn(__dmul_rn(cc, q0), __dmul_rn(bb, q1)) / det;
-                const double u1 = __dadd_rn(__dmul_rn(-bb, q0), __dmul_rn(a, q1)) / det;
-                const double ratio = rs / s2;
-                z0 = __dmul_rn(u0, ratio);
-                z1 = __dmul_rn(u1, ratio);
-              }
-            }
-          }
-        }
-        if (apply_lt && large) {
-          z0 -= v[c];
-          z1 -= v[c + 1];
-        }
-        v[c] = z0;
-        v[c + 1] = z1;
-        continue;
-      }
-      y0 = (d00 == 0.0 || !isfinite(d00)) ? 0.0 : y0 / d00;
-    }
-    if (apply_lt && large) y0 -= v[c];
-    v[c] = y0;
-  }
-  __syncthreads();
-  if (!apply_lt) {
-    for (int t = threadIdx.x; t < p * nrhs; t += kSolveNT) {
-      const int r = nrhs == 1 ? 0 : t / p, i = nrhs == 1 ? t : t - r * p;
-      x[(int64_t)r * P.n + rows[i]] = wk[(int64_t)r * rows_total + roff + i];
-    }
-    return;
-  }
-  if (large) return;  // the block kernels (k_bwd_dots / k_bwd_tri) go on
-  // v -= L21^T x_ext: a warp per column, its lanes' rows loaded once for
-  // every right-hand side
-  for (int j = warp; j < p; j += kSolveNT / 32) {
-    const double *Lj = L + (size_t)j * sf;
-    for (int i0 = p; i0 < f; i0 += 32 * 4) {
-      double l[4];
-      int ri[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + lane + 32 * u;
-        l[u] = (i < f) ? __ldg(Lj + i) : 0.0;
-        ri[u] = (i < f) ? rows[i] : -1;
-      }
-      for (int r = 0; r < nrhs; ++r) {
-        const double *xr = x + (int64_t)r * P.n;
-        double acc = 0.0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (ri[u] >= 0) acc = fma(l[u], xr[ri[u]], acc);
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) wk[(int64_t)r * rows_total + roff + j] -= acc;
-      }
-    }
-  }
-  __syncthreads();
-  // blocked L11^-T: blocks from the end; dots with the solved part, then
-  // the 32 x 32 triangle (a warp per right-hand side)
-  for (int je = p; je > 0; je -= 32) {
-    const int jb = max(0, je - 32), nb = je - jb;
-    // the strip's triangle copied to Ls first, in flight during the dots
-    // (the previous strip's solves, the last readers of Ls, ended at a barrier)
-    load_tri32_async<kSolveNT>(L, sf, jb, nb, Ls);
-    for (int j = jb + warp; j < je; j += kSolveNT / 32) {
-      const double *Lj = L + (size_t)j * sf;
-      for (int i0 = je; i0 < p; i0 += 32 * 4) {
-        double l[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + lane + 32 * u;
-          l[u] = (i < p) ? __ldg(Lj + i) : 0.0;
-        }
-        for (int r = 0; r < nrhs; ++r) {
-          double *v = wk + (int64_t)r * rows_total + roff;
-          double acc = 0.0;
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int i = i0 + lane + 32 * u;
-            if (i < p) acc = fma(l[u], v[i], acc);
-          }
-          for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-          if (lane == 0) v[j] -= acc;
-        }
-      }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    for (int r = warp; r < nrhs; r += kSolveNT / 32) tri_bwd_warp(wk + (int64_t)r * rows_total + roff, jb, nb, posdef, Ls);
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < p * nrhs; t += kSolveNT) {
-    const int r = nrhs == 1 ? 0 : t / p, i = nrhs == 1 ? t : t - r * p;
-    x[(int64_t)r * P.n + rows[i]] = wk[(int64_t)r * rows_total + roff + i];
   }
 }
 
@@ -2968,6 +2505,7 @@ __global__ void __launch_bounds__(256) k_fwd_gemv(DevPlan P, DevFactor X, const 
       }
     }
   }
+  if (!waited) pdl_wait();  // (every grid waits: the next one's wait covers all before)
 }
 
 // v[j] -= sum_{i in [j1, p)} L(i, j) v[i] for the columns j of block b of

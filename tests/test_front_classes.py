@@ -137,3 +137,46 @@ def test_blocked_min_front(blocked, posdef):
         sv.posdef, sv.info = posdef, info
         _compare(a, sv, info, v, posdef, blocked_min_front=blocked)
         sv.close()
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 5, 8, 9])
+@pytest.mark.parametrize("posdef", [True, False])
+def test_solve_by_class(nrhs, posdef):
+    """Solves of single dense fronts at the edges of the solve kernels' sizes
+    against dense solutions, and the sweeps one by one against the full solve.
+    Both are backward stable: |x - y| <= 2 (3 n eps g) cond(A) |x|, with g = 1
+    for Cholesky and at most 1 / u growth per pivot bound u = 0.01."""
+    rng = np.random.default_rng(40 + nrhs)
+    eps = np.finfo(float).eps
+    for n in (1, 2, 31, 32, 33, 64, 65, 96, 97, 160, 383, 384, 700):
+        A = _spd(n, rng) if posdef else _indefinite(n, rng) + np.diag(np.full(n, 0.5))
+        n, cp, ri, v = dense_lower(A)
+        sv = smfg.Solver(smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL), device=0)
+        sv.factor(v, posdef=posdef, aptp_min_rows=0)
+        b = rng.standard_normal((nrhs, n)) if nrhs > 1 else rng.standard_normal(n)
+        want = np.linalg.solve(A, b.T).T
+        x = sv.solve(b)
+        tol = 6 * n * eps * np.linalg.cond(A) * (1.0 if posdef else 100.0)
+        assert np.max(np.abs(x - want)) <= tol * np.max(np.abs(want)), n
+        y = sv.solve(sv.solve(sv.solve(b, smfg.SOLVE_FORWARD), smfg.SOLVE_DIAGONAL), smfg.SOLVE_BACKWARD)
+        assert np.max(np.abs(y - want)) <= tol * np.max(np.abs(want)), n
+        sv.close()
+
+
+@pytest.mark.parametrize("nrhs", [1, 4, 7])
+@pytest.mark.parametrize("kind", ["grid", "chain"])
+def test_solve_trees(kind, nrhs):
+    """Trees with leaves, tiny and medium fronts, with and without delays: the
+    backward error the refinement gate reads (componentwise, 1e-12 after one
+    step of refinement at most), and the single columns' solutions."""
+    n, cp, ri, v = W.laplacian_2d(83, 71) if kind == "grid" else W.trajectory_kkt(60, np.random.default_rng(1))
+    sv = smfg.Solver(smfg.analyse(n, cp, ri), device=0)
+    sv.factor(v, posdef=kind == "grid")
+    b = np.random.default_rng(2).standard_normal((nrhs, n))
+    x = sv.solve(b if nrhs > 1 else b[0]).reshape(nrhs, n)
+    for r in range(nrhs):
+        one = sv.solve(b[r])
+        assert np.max(np.abs(one - x[r])) <= 1e-10 * np.max(np.abs(one))
+        _, _, om, steps = sv.refine(b[r], one, omega_target=1e-12)
+        assert om <= 1e-12 and steps <= 1
+    sv.close()
