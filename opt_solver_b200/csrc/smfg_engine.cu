@@ -852,7 +852,7 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
   const int wcols = w_rows(pl, c, gp.on);
   const int fuse = fuse_rows(c);
   for (int l = 0; l < pl.nlevels; ++l) {
-    const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1], m = hi - lo;
+    const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
     k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse);
     lc.n += 1;
     const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
@@ -1321,9 +1321,26 @@ static void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem,
 static LevelGrid level_grid(const Plan &pl, int l) {
   const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
   const int ic = (pl.posdef || l == 0) ? level_at_most(pl, l, kTinyRows) : hi;
-  return {lo, ic - lo, ic, hi - ic};
+  const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
+  // (the large fronts by symbolic rows head the list: their blocks there go)
+  int i0 = lo;
+  while (i0 < ic && pl.h_large[pl.h_lvl_sn[i0]]) ++i0;
+  return {pl.d.lvl_large + pl.lvl_large_ptr[l], nL, i0, ic - i0, ic, hi - ic};
 }
-static int level_blocks(const LevelGrid &g) { return g.n + (g.nc + kLvlWarps - 1) / kLvlWarps; }
+static int level_blocks(const LevelGrid &g, int nrhs) {
+  return g.nl * nrhs + g.n + (g.nc + kLvlWarps - 1) / kLvlWarps;
+}
+
+// Right-hand sides per block of the large fronts' triangle kernels: the
+// fewest for which a block of threads per front and group still has an SM of
+// its own (a block's chain warps and strips fill one). 40^3, 16 right-hand
+// sides: 8 in one block 7.8 ms a solve, groups by this rule (with the products
+// over all right-hand sides at once) 4.6.
+static int tri_group(int nL, int nrhs, int sms) {
+  int g = 1;
+  while (g < kPipeRhs && (int64_t)nL * ((nrhs + g - 1) / g) > sms) g *= 2;
+  return g;
+}
 
 static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int job, bool scaled, LaunchCount &lc) {
   DevPlan &d = pl.d;
@@ -1347,18 +1364,23 @@ static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int jo
   k_solve_gather<<<g, 256, 0, st>>>(d_b, ldb, nrhs, pl.n, d.perm, sc_in, xv);
   lc.n++;
   const int lgrid = 2 * sms;
+  auto gemv = nrhs == 1 ? k_fwd_gemv<1> : nrhs <= 4 ? k_fwd_gemv<4> : k_fwd_gemv<8>;
+  auto dots = nrhs == 1 ? k_bwd_dots<1> : nrhs <= 4 ? k_bwd_dots<4> : k_bwd_dots<8>;
+  auto l21 = nrhs == 1 ? k_bwd_l21<1> : nrhs <= 4 ? k_bwd_l21<4> : k_bwd_l21<8>;
   if (fwd) {
     for (int l = 0; l < pl.nlevels; ++l) {
       const LevelGrid lv = level_grid(pl, l);
-      launch_pdl(k_fwd_level, level_blocks(lv), kLvlNT, kLvlSmem, st, d, x, lv, pl.posdef, xv, wk, rows_total, nrhs);
+      launch_pdl(k_fwd_level, level_blocks(lv, nrhs), kLvlNT, kLvlSmem, st, d, x, lv, pl.posdef, xv, wk, rows_total, nrhs);
       lc.n += 1;
       const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
       if (nL > 0) {
         const int *lg = d.lvl_large + pl.lvl_large_ptr[l];
         const int nb = (large_pmax(pl, l) + kSB - 1) / kSB;
+        const int grp = tri_group(nL, nrhs, sms), ng = (nrhs + grp - 1) / grp;
         for (int b = 0; b < nb; ++b) {
-          launch_pdl(k_fwd_tri, nL, kTriNT, sizeof(TriSmem), st, d, x, lg, b, pl.posdef, xv, wk, rows_total, nrhs);
-          launch_pdl(k_fwd_gemv, lgrid, 256, 0, st, d, x, lg, nL, b, wk, rows_total, nrhs);
+          launch_pdl(k_fwd_tri, nL * ng, kTriNT, sizeof(TriSmem), st, d, x, lg, b, pl.posdef, xv, wk, rows_total,
+                     nrhs, grp);
+          launch_pdl(gemv, lgrid, 256, 0, st, d, x, lg, nL, b, wk, rows_total, nrhs);
         }
         lc.n += 2 * nb;
       }
@@ -1368,21 +1390,24 @@ static void enqueue_solve_chunk(Plan &pl, double *d_b, int nrhs, int ldb, int jo
     for (int l = pl.nlevels - 1; l >= 0; --l) {
       const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
       if (nL > 0 && use_lt) {
-        launch_pdl(k_bwd_l21, lgrid, 256, 0, st, d, x, d.lvl_large + pl.lvl_large_ptr[l], nL, xv, wk, rows_total, nrhs);
+        launch_pdl(l21, lgrid, 256, 0, st, d, x, d.lvl_large + pl.lvl_large_ptr[l], nL, xv, wk, rows_total, nrhs);
         lc.n++;
       }
       const LevelGrid lv = level_grid(pl, l);
-      launch_pdl(k_bwd_level, level_blocks(lv), kLvlNT, kLvlSmem, st, d, x, lv, pl.posdef, xv, wk, rows_total, nrhs,
+      launch_pdl(k_bwd_level, level_blocks(lv, nrhs), kLvlNT, kLvlSmem, st, d, x, lv, pl.posdef, xv, wk, rows_total, nrhs,
                  use_d ? 1 : 0, use_lt ? 1 : 0);
       lc.n += 1;
       if (nL > 0 && use_lt) {
         const int *lg = d.lvl_large + pl.lvl_large_ptr[l];
         const int nb = (large_pmax(pl, l) + kSB - 1) / kSB;
+        const int grp = tri_group(nL, nrhs, sms), ng = (nrhs + grp - 1) / grp;
         for (int b = nb - 1; b >= 0; --b) {
-          launch_pdl(k_bwd_dots, lgrid, 256, 0, st, d, x, lg, nL, b, wk, rows_total, nrhs);
-          launch_pdl(k_bwd_tri, nL, kTriNT, sizeof(TriSmem), st, d, x, lg, b, pl.posdef, xv, wk, rows_total, nrhs);
+          // (no rows of a front lie past its last block)
+          if (b < nb - 1) launch_pdl(dots, lgrid, 256, 0, st, d, x, lg, nL, b, wk, rows_total, nrhs);
+          launch_pdl(k_bwd_tri, nL * ng, kTriNT, sizeof(TriSmem), st, d, x, lg, b, pl.posdef, xv, wk, rows_total,
+                     nrhs, grp);
         }
-        lc.n += 2 * nb;
+        lc.n += 2 * nb - 1;
       }
     }
   }

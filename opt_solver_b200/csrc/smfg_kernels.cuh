@@ -1945,19 +1945,21 @@ __device__ __forceinline__ void dinv2_apply(double d00, double d10, double d11, 
 }
 
 // t[0:p) = L21^T x_ext of the level's large fronts, stored at the front's
-// work vector positions [0, p): a work item is kL21Cols columns of one
-// front for one right-hand side. x_ext is gathered into shared memory a
-// tile of rows at a time, once for all the item's columns; a warp takes
-// kL21Cols / 8 columns, lane = row. Each column's sum runs over its rows as
-// a warp per column would take them (lane l: rows p + l + 32m in turn),
-// then a shuffle tree.
-constexpr int kL21Cols = 16, kL21Tile = 1024;
+// work vector positions [0, p): a work item is kL21Cols columns of one front
+// for every right-hand side (up to R), L read once for all of them. x_ext is
+// gathered into shared memory a tile of rows at a time, once for all the
+// item's columns; a warp takes kL21Cols / 8 columns, lane = row. Each
+// column's sum runs over its rows as a warp per column would take them (lane
+// l: rows p + l + 32m in turn), then a shuffle tree.
+constexpr int kL21Cols = 16;
+template <int R>
 __global__ void __launch_bounds__(256) k_bwd_l21(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                  int nlarge, const double *x, double *wk,
                                                  int64_t rows_total, int nrhs) {
   constexpr int CW = kL21Cols / 8;  // columns a warp
+  constexpr int TILE = R == 1 ? 1024 : 512;
   __shared__ int pref[65];
-  __shared__ double xs[kL21Tile];
+  __shared__ double xs[R][TILE];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_wait();
   pdl_trigger();
@@ -1966,10 +1968,7 @@ __global__ void __launch_bounds__(256) k_bwd_l21(DevPlan P, DevFactor X, const i
     __syncthreads();
     if (threadIdx.x == 0) {
       pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) {
-        const int s = large[chunk + q];
-        pref[q + 1] = pref[q] + (X.sn_pstore[s] + kL21Cols - 1) / kL21Cols * nrhs;
-      }
+      for (int q = 0; q < cnt; ++q) pref[q + 1] = pref[q] + (X.sn_pstore[large[chunk + q]] + kL21Cols - 1) / kL21Cols;
     }
     __syncthreads();
     const int total = pref[cnt];
@@ -1982,34 +1981,45 @@ __global__ void __launch_bounds__(256) k_bwd_l21(DevPlan P, DevFactor X, const i
       }
       const int s = large[chunk + a];
       const int f = X.sn_f[s], p = X.sn_pstore[s];
-      const int ncc = (p + kL21Cols - 1) / kL21Cols;
-      const int item = wi - pref[a];
-      const int r = item / ncc, cc = item % ncc;
-      const int jw = cc * kL21Cols + warp * CW;
+      const int jw = (wi - pref[a]) * kL21Cols + warp * CW;
       const int *rows = X.rows + X.sn_roff[s] + p;
       const double *L = X.arena + X.sn_off[s] + p;
-      const double *xr = x + (int64_t)r * P.n;
-      double acc[CW];
+      double acc[CW][R];
 #pragma unroll
-      for (int c = 0; c < CW; ++c) acc[c] = 0.0;
-      for (int t0 = 0; t0 < f - p; t0 += kL21Tile) {
-        const int tn = min(kL21Tile, f - p - t0);
+      for (int c = 0; c < CW; ++c)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[c][r] = 0.0;
+      for (int t0 = 0; t0 < f - p; t0 += TILE) {
+        const int tn = min(TILE, f - p - t0);
         __syncthreads();  // the tile before read
-        for (int i = threadIdx.x; i < tn; i += 256) xs[i] = xr[rows[t0 + i]];
-        __syncthreads();
-        for (int i = lane; i < tn; i += 32) {
-          const double xv = xs[i];
+        for (int i = threadIdx.x; i < tn; i += 256) {
+          const int ri = rows[t0 + i];
 #pragma unroll
-          for (int c = 0; c < CW; ++c)
-            if (jw + c < p) acc[c] = fma(L[(size_t)(jw + c) * f + t0 + i], xv, acc[c]);
+          for (int r = 0; r < R; ++r) xs[r][i] = r < nrhs ? x[(int64_t)r * P.n + ri] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll(R == 1 ? 8 : 2)
+        for (int i = lane; i < tn; i += 32) {
+          double l[CW];
+#pragma unroll
+          for (int c = 0; c < CW; ++c) l[c] = (jw + c < p) ? L[(size_t)(jw + c) * f + t0 + i] : 0.0;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const double xv = xs[r][i];
+#pragma unroll
+            for (int c = 0; c < CW; ++c) acc[c][r] = fma(l[c], xv, acc[c][r]);
+          }
         }
       }
 #pragma unroll
-      for (int c = 0; c < CW; ++c) {
-        double v = acc[c];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && jw + c < p) wk[(int64_t)r * rows_total + X.sn_roff[s] + jw + c] = v;
-      }
+      for (int c = 0; c < CW; ++c)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          double v = acc[c][r];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0 && r < nrhs && jw + c < p) wk[(int64_t)r * rows_total + X.sn_roff[s] + jw + c] = v;
+        }
     }
   }
 }
@@ -2032,9 +2042,13 @@ constexpr int kTriNT = 256;  // threads of the triangle kernels
 // strip's 32 columns hit distinct banks.
 constexpr int kSBP = kSB + 1;
 constexpr int kRing = 3;
+// Right-hand sides of one block of threads in the block solves: their warps run
+// the triangle chains, the others the rest of the block a strip behind. More
+// right-hand sides take more blocks.
+constexpr int kPipeRhs = 4;
 struct TriSmem {
   double buf[kRing][32][kSBP];
-  double w[8][kSB];  // the block's values, per right-hand side (at most 8)
+  double w[kPipeRhs][kSB];  // the block's values, per right-hand side
 };
 
 // Inverses of the SPD large fronts' 32 x 32 diagonal blocks of L (after
@@ -2322,12 +2336,6 @@ __device__ __forceinline__ void bwd_cols_update(const double (*L2)[kSBP], int j0
   }
 }
 
-// At most this many right-hand sides take the pipelined block solves (the
-// first nrhs warps run the triangle chains, the others the rest of the
-// block a strip behind); more take the step-by-step form, which computes
-// the same sums.
-constexpr int kPipeRhs = 4;
-
 // sm.w[r][0, j1 - j0) <- L_bb^-1 sm.w[r] for each right-hand side, the
 // block's first kRing strips issued by fwd_block_issue. Row i of the block
 // takes each strip's product in strip order: the strips up to two before
@@ -2337,28 +2345,6 @@ __device__ void fwd_block_solve(const double *L, size_t sf, int j0, int j1, int 
                                 const double *inv) {
   const int warp = threadIdx.x >> 5;
   const int nstrip = (j1 - j0 + 31) / 32;
-  if (nrhs > kPipeRhs) {
-    cp_async_wait_pending(0);
-    __syncthreads();
-    for (int k = 0; k < nstrip; ++k) {
-      int jb, nb;
-      fwd_strip(j0, j1, k, jb, nb);
-      const double(*Lb)[kSBP] = sm.buf[k % kRing];
-      if (k >= kRing) cp_async_wait_pending(min(kRing - 1, nstrip - 1 - k));
-      __syncthreads();
-      if (warp < nrhs) fwd_chain32(Lb, j0, jb, nb, posdef, sm.w[warp], 0.0, inv != nullptr);
-      __syncthreads();
-      fwd_rows_update(Lb, j0, j1, jb, nb, jb + nb, nrhs, sm, (int)threadIdx.x, kTriNT);
-      __syncthreads();  // this strip's buffer is free
-      if (k + kRing < nstrip) {
-        int jb3, nb3;
-        fwd_strip(j0, j1, k + kRing, jb3, nb3);
-        tri_strip_async(L, sf, j0, j1, jb3, nb3, sm.buf[k % kRing], 0, kTriNT, inv);
-      }
-    }
-    __syncthreads();
-    return;
-  }
   // Step k: the chain warps solve strip k and form its look-ahead product
   // with strip k + 1's rows; the other warps apply strip k - 1 to the rows
   // past strip k and then stream strip k + 2 into strip k - 1's buffer.
@@ -2399,14 +2385,19 @@ __device__ void fwd_block_solve(const double *L, size_t sf, int j0, int j1, int 
   }
 }
 
-// Forward block b of each large front (a block of threads per front):
-// w[j0:j1) <- L_bb^-1 w[j0:j1).
+// Forward block b of each large front (a block of threads per front and group
+// of right-hand sides): w[j0:j1) <- L_bb^-1 w[j0:j1).
 __global__ void __launch_bounds__(kTriNT) k_fwd_tri(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                     int b, int posdef, double *x, double *wk,
-                                                    int64_t rows_total, int nrhs) {
+                                                    int64_t rows_total, int nrhs_all, int group) {
   extern __shared__ __align__(16) unsigned char tri_smem[];
   TriSmem &sm = *reinterpret_cast<TriSmem *>(tri_smem);
-  const int s = large[blockIdx.x];
+  // (front, group of right-hand sides)
+  const int ng = (nrhs_all + group - 1) / group, rg = (int)blockIdx.x % ng * group;
+  const int nrhs = min(group, nrhs_all - rg);
+  x += (int64_t)rg * P.n;
+  wk += (int64_t)rg * rows_total;
+  const int s = large[blockIdx.x / ng];
   const int f = X.sn_f[s], p = X.sn_pstore[s];
   const int j0 = b * kSB;
   if (j0 >= p) return;
@@ -2435,13 +2426,15 @@ __global__ void __launch_bounds__(kTriNT) k_fwd_tri(DevPlan P, DevFactor X, cons
 }
 
 // w[j1:f) -= L[j1:f, j0:j1) w[j0:j1) of each large front: a work item is 32
-// rows; its 8 warps take 32-column strips of the block, lane = row, and the
-// strips' partial sums are added in strip order.
+// rows for every right-hand side (up to R), L read once for all of them; its
+// 8 warps take 32-column strips of the block, lane = row, and the strips'
+// partial sums are added in strip order.
+template <int R>
 __global__ void __launch_bounds__(256) k_fwd_gemv(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                   int nlarge, int b, double *wk, int64_t rows_total,
                                                   int nrhs) {
-  __shared__ double ws[kSB];
-  __shared__ double part[8][33];
+  __shared__ __align__(16) double ws[R][kSB];
+  __shared__ double part[8][R][33];
   __shared__ int pref[65];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bool waited = false;
@@ -2453,7 +2446,7 @@ __global__ void __launch_bounds__(256) k_fwd_gemv(DevPlan P, DevFactor X, const 
       for (int q = 0; q < cnt; ++q) {
         const int s = large[chunk + q];
         const int f = X.sn_f[s], p = X.sn_pstore[s], j1 = min(p, (b + 1) * kSB);
-        pref[q + 1] = pref[q] + ((b * kSB < p && f > j1) ? (f - j1 + 31) / 32 * nrhs : 0);
+        pref[q + 1] = pref[q] + ((b * kSB < p && f > j1) ? (f - j1 + 31) / 32 : 0);
       }
     }
     __syncthreads();
@@ -2468,13 +2461,10 @@ __global__ void __launch_bounds__(256) k_fwd_gemv(DevPlan P, DevFactor X, const 
       const int s = large[chunk + a];
       const int f = X.sn_f[s], p = X.sn_pstore[s];
       const int j0 = b * kSB, j1 = min(p, j0 + kSB);
-      const int nchunks = (f - j1 + 31) / 32;
-      const int item = wi - pref[a];
-      const int r = item / nchunks, rc = item % nchunks;
-      double *w = wk + (int64_t)r * rows_total + X.sn_roff[s];
+      double *w = wk + X.sn_roff[s];
       const double *L = X.arena + X.sn_off[s];
       const size_t sf = (size_t)f;
-      const int i = j1 + rc * 32 + lane;
+      const int i = j1 + (wi - pref[a]) * 32 + lane;
       const int jb = j0 + warp * 32;
       const int nbw = (i < f && jb < j1) ? min(32, j1 - jb) : 0;
       // this lane's 32 entries of L in flight before the wait (the first
@@ -2489,34 +2479,44 @@ __global__ void __launch_bounds__(256) k_fwd_gemv(DevPlan P, DevFactor X, const 
         waited = true;
       }
       __syncthreads();
-      for (int t = threadIdx.x; t < j1 - j0; t += 256) ws[t] = w[j0 + t];
+      for (int r = 0; r < R && r < nrhs; ++r)
+        ws[r][threadIdx.x] = j0 + (int)threadIdx.x < j1 ? w[(int64_t)r * rows_total + j0 + threadIdx.x] : 0.0;
       __syncthreads();
-      double acc = 0.0;
+      for (int r = 0; r < R && r < nrhs; ++r) {
+        // (two chains: even and odd columns)
+        double a0 = 0.0, a1 = 0.0;
 #pragma unroll
-      for (int u = 0; u < 32; ++u)
-        if (u < nbw) acc = fma(l[u], ws[jb + u - j0], acc);
-      part[warp][lane] = acc;
-      __syncthreads();
-      if (warp == 0 && i < f) {
-        double sum = 0.0;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) sum += part[g][lane];
-        w[i] -= sum;
+        for (int u = 0; u < 32; u += 2) {
+          const double2 y = *reinterpret_cast<const double2 *>(&ws[r][warp * 32 + u]);
+          a0 = fma(l[u], y.x, a0);
+          a1 = fma(l[u + 1], y.y, a1);
+        }
+        part[warp][r][lane] = a0 + a1;
       }
+      __syncthreads();
+      for (int r = warp; r < R && r < nrhs; r += 8)
+        if (i < f) {
+          double sum = 0.0;
+#pragma unroll
+          for (int g = 0; g < 8; ++g) sum += part[g][r][lane];
+          w[(int64_t)r * rows_total + i] -= sum;
+        }
     }
   }
   if (!waited) pdl_wait();  // (every grid waits: the next one's wait covers all before)
 }
 
 // v[j] -= sum_{i in [j1, p)} L(i, j) v[i] for the columns j of block b of
-// each large front: a work item is one column, its rows split over the
-// block's threads (all loads of a thread in flight), partial sums added in
-// thread order.
+// each large front: a work item is CW columns for every right-hand side (up
+// to R), their rows split over the block's threads (a thread's loads in
+// flight), partial sums added in thread order.
+template <int R>
 __global__ void __launch_bounds__(256) k_bwd_dots(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                   int nlarge, int b, double *wk, int64_t rows_total,
                                                   int nrhs) {
+  constexpr int CW = R == 1 ? 1 : 2, AHEAD = R == 1 ? 8 : 2;
   __shared__ int pref[65];
-  __shared__ double red[8];
+  __shared__ double red[8][CW * R];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_wait();
   pdl_trigger();
@@ -2528,7 +2528,7 @@ __global__ void __launch_bounds__(256) k_bwd_dots(DevPlan P, DevFactor X, const 
       for (int q = 0; q < cnt; ++q) {
         const int s = large[chunk + q];
         const int p = X.sn_pstore[s], j0 = b * kSB, j1 = min(p, j0 + kSB);
-        pref[q + 1] = pref[q] + ((j0 < p && j1 < p) ? (j1 - j0) * nrhs : 0);
+        pref[q + 1] = pref[q] + ((j0 < p && j1 < p) ? (j1 - j0 + CW - 1) / CW : 0);
       }
     }
     __syncthreads();
@@ -2543,31 +2543,46 @@ __global__ void __launch_bounds__(256) k_bwd_dots(DevPlan P, DevFactor X, const 
       const int s = large[chunk + a];
       const int f = X.sn_f[s], p = X.sn_pstore[s];
       const int j0 = b * kSB, j1 = min(p, j0 + kSB);
-      const int item = wi - pref[a];
-      const int r = item / (j1 - j0), j = j0 + item % (j1 - j0);
-      double *v = wk + (int64_t)r * rows_total + X.sn_roff[s];
+      const int j = j0 + (wi - pref[a]) * CW, nj = min(CW, j1 - j);
+      double *v = wk + X.sn_roff[s];
       const double *Lj = X.arena + X.sn_off[s] + (size_t)j * f;
-      double acc = 0.0;
-      int i = j1 + (int)threadIdx.x;
-      for (; i + 7 * 256 < p; i += 8 * 256) {
-        double l[8], y[8];
+      double acc[CW][R];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          l[u] = __ldg(Lj + i + u * 256);
-          y[u] = v[i + u * 256];
+      for (int c = 0; c < CW; ++c)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[c][r] = 0.0;
+      for (int i0 = j1 + (int)threadIdx.x; i0 < p; i0 += AHEAD * 256) {
+        double l[CW][AHEAD], y[R][AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+          const int i = i0 + u * 256;
+#pragma unroll
+          for (int c = 0; c < CW; ++c) l[c][u] = (i < p && c < nj) ? __ldg(Lj + (size_t)c * f + i) : 0.0;
+#pragma unroll
+          for (int r = 0; r < R; ++r) y[r][u] = (i < p && r < nrhs) ? v[(int64_t)r * rows_total + i] : 0.0;
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc = fma(l[u], y[u], acc);
+        for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int c = 0; c < CW; ++c) acc[c][r] = fma(l[c][u], y[r][u], acc[c][r]);
       }
-      for (; i < p; i += 256) acc = fma(Lj[i], v[i], acc);
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       __syncthreads();
-      if (lane == 0) red[warp] = acc;
+#pragma unroll
+      for (int c = 0; c < CW; ++c)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) acc[c][r] += __shfl_xor_sync(0xffffffffu, acc[c][r], o);
+          if (lane == 0) red[warp][c * R + r] = acc[c][r];
+        }
       __syncthreads();
-      if (threadIdx.x == 0) {
+      const int c = (int)threadIdx.x / R, r = (int)threadIdx.x % R;
+      if (c < nj && r < nrhs) {
         double sum = 0.0;
-        for (int g = 0; g < 8; ++g) sum += red[g];
-        v[j] -= sum;
+        for (int g = 0; g < 8; ++g) sum += red[g][c * R + r];
+        v[(int64_t)r * rows_total + j + c] -= sum;
       }
     }
   }
@@ -2583,43 +2598,6 @@ __device__ void bwd_block_solve(const double *L, size_t sf, int j0, int j1, int 
                                 const double *inv) {
   const int warp = threadIdx.x >> 5;
   const int nstrip = (j1 - j0 + 31) / 32;
-  if (nrhs > kPipeRhs) {
-    cp_async_wait_pending(0);
-    __syncthreads();
-    for (int k = 0; k < nstrip; ++k) {
-      int jb, nb;
-      bwd_strip(j0, j1, k, jb, nb);
-      const double(*Lb)[kSBP] = sm.buf[k % kRing];
-      if (k >= kRing) cp_async_wait_pending(min(kRing - 1, nstrip - 1 - k));
-      __syncthreads();
-      if (k >= 2) {
-        int jm, nm;
-        bwd_strip(j0, j1, k - 2, jm, nm);
-        bwd_cols_update(Lb, j0, j1, jb, nb, jm, nrhs, sm, warp, kTriNT / 32);
-      }
-      __syncthreads();
-      if (warp < nrhs) {
-        double la = 0.0;
-        if (k >= 1) {
-          // strip k - 1's solved values in the lanes, as the chain left them
-          int jp, np;
-          bwd_strip(j0, j1, k - 1, jp, np);
-          const int lane = threadIdx.x & 31;
-          const double xp = (lane < np) ? sm.w[warp][jp - j0 + lane] : 0.0;
-          la = bwd_ahead32(Lb, j0, jp, np, xp);
-        }
-        bwd_chain32(Lb, j0, jb, nb, posdef, sm.w[warp], la, inv != nullptr);
-      }
-      __syncthreads();  // this strip's buffer is free
-      if (k + kRing < nstrip) {
-        int jb3, nb3;
-        bwd_strip(j0, j1, k + kRing, jb3, nb3);
-        tri_strip_async(L, sf, j0, j1, jb3, nb3, sm.buf[k % kRing], 0, kTriNT, inv);
-      }
-    }
-    __syncthreads();
-    return;
-  }
   // Step k: the chain warps solve strip k and form its look-ahead product
   // with strip k + 1's columns; the other warps stream strip k + 2 into
   // strip k - 1's buffer and apply the rows solved up to strip k - 1 to
@@ -2657,14 +2635,19 @@ __device__ void bwd_block_solve(const double *L, size_t sf, int j0, int j1, int 
   }
 }
 
-// Backward block b of each large front (a block of threads per front; its
-// rows past the block already taken by k_bwd_dots).
+// Backward block b of each large front (a block of threads per front and group
+// of right-hand sides; its rows past the block already taken by k_bwd_dots).
 __global__ void __launch_bounds__(kTriNT) k_bwd_tri(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                     int b, int posdef, double *x, double *wk,
-                                                    int64_t rows_total, int nrhs) {
+                                                    int64_t rows_total, int nrhs_all, int group) {
   extern __shared__ __align__(16) unsigned char tri_smem[];
   TriSmem &sm = *reinterpret_cast<TriSmem *>(tri_smem);
-  const int s = large[blockIdx.x];
+  // (front, group of right-hand sides)
+  const int ng = (nrhs_all + group - 1) / group, rg = (int)blockIdx.x % ng * group;
+  const int nrhs = min(group, nrhs_all - rg);
+  x += (int64_t)rg * P.n;
+  wk += (int64_t)rg * rows_total;
+  const int s = large[blockIdx.x / ng];
   const int f = X.sn_f[s], p = X.sn_pstore[s];
   const int j0 = b * kSB;
   if (j0 >= p) return;

@@ -7,10 +7,12 @@
 // (programmatic dependent launch), every right-hand side's chain runs beside
 // the others, and the reciprocals of an SPD diagonal are taken off the chain.
 // One grid: a block per front -- of up to 64 rows with L in shared memory and
-// a warp per right-hand side, of more in 32-column strips (large fronts only
-// gather here: the block kernels go on) -- then blocks of eight tiny fronts
+// a warp per right-hand side, of more in 32-column strips -- then blocks of
+// eight tiny fronts
 // (up to 32 rows), a warp each, where the sizes are known beforehand (SPD
-// fronts, leaves): delays may grow the others.
+// fronts, leaves): delays may grow the others. Before them a block per large
+// front and right-hand side: it only gathers (forward) or applies D^-1
+// (backward), the block kernels go on.
 // Sums run in a fixed order (deterministic); solve_forward.cpp:116-293 and
 // solve_backward.cpp:135-350 compute the same quantities.
 // Measured on one B200 against the two kernels a level and direction before
@@ -39,11 +41,13 @@ constexpr int kLvlDoubles = kLvlWarps * kTinyDoubles;
 constexpr int kLvlSmem = kLvlDoubles * 8;
 static_assert(kLvlDoubles >= kStageRows * (kStageRows + 1) + 3 * kSolveRhs * kStageRows, "staged front");
 
-// The blocks of a level's launch: n fronts P.lvl_sn[i0 + block], a block
-// each, then nc tiny ones from ic, a warp each. Every front is in one of the
-// two, so every launch has a block that waits for the kernel before it.
+// The blocks of a level's launch: nl large fronts (list lg), a block for each
+// right-hand side; n fronts P.lvl_sn[i0 + block], a block each (the large
+// ones among them leave); nc tiny ones from ic, a warp each. Every front is
+// taken, so every launch has a block that waits for the kernel before it.
 struct LevelGrid {
-  int i0, n, ic, nc;
+  const int *lg;
+  int nl, i0, n, ic, nc;
 };
 // The larger fronts' strip: its triangle and solved values, then vectors.
 constexpr int kStripDoubles = 32 * 33 + 32 * kSolveRhs;
@@ -172,28 +176,31 @@ __device__ __forceinline__ bool pivot_value(const double *Lc, int ldn, int c, in
 // A child's update vectors added into the parent's vectors in child order.
 // sw: the parent's vectors, right-hand side r at sw + r * stride; threads t
 // of nt; sync() between children.
-template <typename Sync>
+template <int RB, typename Sync>
 __device__ __forceinline__ void add_children(const DevPlan &P, const DevFactor &X, int s, const double *wk,
                                              int64_t rows_total, int r0, int r1, double *sw, int64_t stride, int t,
                                              int nt, Sync sync) {
   for (int ti = P.child_ptr[s]; ti < P.child_ptr[s + 1]; ++ti) {
     const int c = P.child_idx[ti];
-    const int pc = X.sn_pstore[c], q = X.sn_f[c] - pc;
+    const int pc = X.sn_pstore[c], n = X.sn_f[c] - pc;
     const int64_t co = X.sn_roff[c] + pc;
     const int *cmap = X.cbmap + co;
-    for (int i0 = t; i0 < q; i0 += 4 * nt) {
+    for (int i0 = t; i0 < n; i0 += 4 * nt) {
       int m[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) m[u] = i0 + u * nt < q ? cmap[i0 + u * nt] : 0;
-      for (int r = r0; r < r1; ++r) {
-        const double *wc = wk + (int64_t)r * rows_total + co;
-        double *w = sw + r * stride;
-        double v[4];
+      for (int u = 0; u < 4; ++u) m[u] = i0 + u * nt < n ? cmap[i0 + u * nt] : 0;
+      for (int r = r0; r < r1; r += RB) {  // RB right-hand sides' loads in flight
+        double v[RB][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = i0 + u * nt < q ? wc[i0 + u * nt] : 0.0;
+        for (int q = 0; q < RB; ++q)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (i0 + u * nt < q) w[m[u]] += v[u];
+          for (int u = 0; u < 4; ++u)
+            v[q][u] = (r + q < r1 && i0 + u * nt < n) ? wk[(int64_t)(r + q) * rows_total + co + i0 + u * nt] : 0.0;
+#pragma unroll
+        for (int q = 0; q < RB; ++q)
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (r + q < r1 && i0 + u * nt < n) sw[(r + q) * stride + m[u]] += v[q][u];
       }
     }
     sync();
@@ -212,7 +219,32 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
                                                       double *wk, int64_t rows_total, int nrhs) {
   extern __shared__ __align__(16) double lvl_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int blk = blockIdx.x;
+  const int blk = (int)blockIdx.x - g.nl * nrhs;
+  if (blk < 0) {
+    // --- a large front, one right-hand side: gather, children
+    const int s = g.lg[blockIdx.x / nrhs], r = (int)blockIdx.x % nrhs;
+    const int f = X.sn_f[s], p = X.sn_pstore[s];
+    const int64_t roff = X.sn_roff[s];
+    const int *rows = X.rows + roff;
+    double *w = wk + (int64_t)r * rows_total + roff;
+    const double *xr = x + (int64_t)r * P.n;
+    pdl_wait();
+    pdl_trigger();
+    for (int i0 = tid; i0 < f; i0 += 8 * kLvlNT) {
+      int ri[8];
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) ri[u] = i0 + u * kLvlNT < p ? rows[i0 + u * kLvlNT] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = i0 + u * kLvlNT < p ? xr[ri[u]] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i0 + u * kLvlNT < f) w[i0 + u * kLvlNT] = v[u];
+    }
+    __syncthreads();
+    add_children<1>(P, X, s, wk + (int64_t)r * rows_total, rows_total, 0, 1, w, 0, tid, kLvlNT, [] { __syncthreads(); });
+    return;
+  }
   if (blk >= g.n) {
     // --- tiny fronts, a warp each
     const int item = (blk - g.n) * kLvlWarps + warp;
@@ -238,7 +270,7 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
       for (int q = 0; q < rn; ++q)
         if (lane < f) sw[q * kTinyRows + lane] = lane < p ? x[(int64_t)(r0 + q) * P.n + my] : 0.0;
       __syncwarp();
-      add_children(P, X, s, wk + (int64_t)r0 * rows_total, rows_total, 0, rn, sw, kTinyRows, lane, 32,
+      add_children<R>(P, X, s, wk + (int64_t)r0 * rows_total, rows_total, 0, rn, sw, kTinyRows, lane, 32,
                    [] { __syncwarp(); });
       double w0[R];
 #pragma unroll
@@ -284,10 +316,10 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
   }
   const int s = P.lvl_sn[g.i0 + blk];
   const int f = X.sn_f[s], p = X.sn_pstore[s];
-  const bool large = P.sn_large[s] != 0;
+  if (P.sn_large[s]) return;
   const int64_t roff = X.sn_roff[s];
   const int *rows = X.rows + roff;
-  if (!large && f <= kStageRows) {
+  if (f <= kStageRows) {
     // --- up to 64 rows: L in shared memory, a warp per right-hand side
     const int ld = f | 1;
     double *Ls = lvl_smem, *rd = Ls + kStageRows * (kStageRows + 1), *sw = rd + kStageRows + warp * kStageRows;
@@ -306,7 +338,7 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
     sw[lane] = lane < p ? xr[r0] : 0.0;
     sw[lane + 32] = lane + 32 < p ? xr[r1] : 0.0;
     __syncwarp();
-    add_children(P, X, s, w, rows_total, 0, 1, sw, 0, lane, 32, [] { __syncwarp(); });
+    add_children<1>(P, X, s, w, rows_total, 0, 1, sw, 0, lane, 32, [] { __syncwarp(); });
     double w0[1] = {sw[lane]}, w1[1] = {sw[lane + 32]};
     small_fwd_chain<1, true>(Ls, ld, f, p, rd, posdef != 0, w0, w1);
     if (lane < p) xr[r0] = w0[0];
@@ -318,32 +350,39 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
   // --- more than 64 rows
   const double *L = X.arena + X.sn_off[s];
   const size_t sf = (size_t)f;
-  if (!large) prefetch_front(L, f, p);
+  prefetch_front(L, f, p);
   pdl_wait();
   pdl_trigger();
   double(*wt)[kSolveRhs] = reinterpret_cast<double(*)[kSolveRhs]>(lvl_smem);  // the strip's solved values, a row a column
   double(*Ls)[33] = reinterpret_cast<double(*)[33]>(lvl_smem + 32 * kSolveRhs);
-  // the vectors in shared memory when they fit (large fronts': global)
-  const bool in_smem = !large && (int64_t)f * nrhs <= kLvlDoubles - kStripDoubles;
+  // the vectors in shared memory when they fit
+  const bool in_smem = (int64_t)f * nrhs <= kLvlDoubles - kStripDoubles;
   double *sw = in_smem ? lvl_smem + kStripDoubles : wk + roff;
   const int64_t stride = in_smem ? f : rows_total;
-  for (int i0 = tid; i0 < f; i0 += 4 * kLvlNT) {
-    int ri[4];
+  auto gather = [&](auto tag) {
+    constexpr int R = decltype(tag)::value;  // right-hand sides' loads in flight
+    for (int i0 = tid; i0 < f; i0 += 2 * kLvlNT) {
+      const int i1 = i0 + kLvlNT, ra = i0 < p ? rows[i0] : 0, rb = i1 < p ? rows[i1] : 0;
+      for (int r0 = 0; r0 < nrhs; r0 += R) {
+        double va[R], vb[R];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) ri[u] = i0 + u * kLvlNT < p ? rows[i0 + u * kLvlNT] : 0;
-    for (int r = 0; r < nrhs; ++r) {
-      const double *xr = x + (int64_t)r * P.n;
-      double v[4];
+        for (int q = 0; q < R; ++q) {
+          va[q] = (i0 < p && r0 + q < nrhs) ? x[(int64_t)(r0 + q) * P.n + ra] : 0.0;
+          vb[q] = (i1 < p && r0 + q < nrhs) ? x[(int64_t)(r0 + q) * P.n + rb] : 0.0;
+        }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = i0 + u * kLvlNT < p ? xr[ri[u]] : 0.0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (i0 + u * kLvlNT < f) sw[r * stride + i0 + u * kLvlNT] = v[u];
+        for (int q = 0; q < R; ++q)
+          if (r0 + q < nrhs) {
+            sw[(r0 + q) * stride + i0] = va[q];
+            if (i1 < f) sw[(r0 + q) * stride + i1] = vb[q];
+          }
+      }
     }
-  }
-  __syncthreads();
-  add_children(P, X, s, wk, rows_total, 0, nrhs, sw, stride, tid, kLvlNT, [] { __syncthreads(); });
-  if (large) return;  // the block kernels (k_fwd_tri / k_fwd_gemv) go on
+    __syncthreads();
+    add_children<R>(P, X, s, wk, rows_total, 0, nrhs, sw, stride, tid, kLvlNT, [] { __syncthreads(); });
+  };
+  if (nrhs == 1) gather(std::integral_constant<int, 1>{});
+  else gather(std::integral_constant<int, 4>{});
   for (int jb = 0; jb < p; jb += 32) {
     const int nb = min(32, p - jb);
     // the strip's triangle and this thread's first row below it loaded
@@ -415,8 +454,37 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_bwd_level(DevPlan P, DevFactor X,
                                                       int apply_lt) {
   extern __shared__ __align__(16) double lvl_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int blk = blockIdx.x;
+  const int blk = (int)blockIdx.x - g.nl * nrhs;
   const bool use_d = apply_d && !posdef;
+  if (blk < 0) {
+    // --- a large front, one right-hand side: D^-1 of its pivot blocks, minus
+    // L21^T x_ext (in v[0:p))
+    const int s = g.lg[blockIdx.x / nrhs], r = (int)blockIdx.x % nrhs;
+    const int f = X.sn_f[s], p = X.sn_pstore[s];
+    const int *rows = X.rows + X.sn_roff[s];
+    const double *L = X.arena + X.sn_off[s];
+    pdl_wait();
+    pdl_trigger();
+    double *xr = x + (int64_t)r * P.n, *v = wk + (int64_t)r * rows_total + X.sn_roff[s];
+#pragma unroll 4
+    for (int c = tid; c < p; c += kLvlNT) {
+      const double *Lc = L + (size_t)c * f;
+      const double y0 = xr[rows[c]], y1 = (use_d && c + 1 < p) ? xr[rows[c + 1]] : 0.0;
+      double z0, z1;
+      bool pair;
+      if (!pivot_value(Lc, f, c, p, use_d, y0, y1, z0, z1, pair)) continue;
+      if (apply_lt) {
+        z0 -= v[c];
+        if (pair) z1 -= v[c + 1];
+      }
+      v[c] = z0;
+      if (pair) v[c + 1] = z1;
+    }
+    if (apply_lt) return;
+    __syncthreads();
+    for (int c = tid; c < p; c += kLvlNT) xr[rows[c]] = v[c];
+    return;
+  }
   if (blk >= g.n) {
     // --- tiny fronts, a warp each
     const int item = (blk - g.n) * kLvlWarps + warp;
@@ -495,10 +563,10 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_bwd_level(DevPlan P, DevFactor X,
   }
   const int s = P.lvl_sn[g.i0 + blk];
   const int f = X.sn_f[s], p = X.sn_pstore[s];
-  const bool large = P.sn_large[s] != 0;
+  if (P.sn_large[s]) return;
   const int64_t roff = X.sn_roff[s];
   const int *rows = X.rows + roff;
-  if (!large && f <= kStageRows) {
+  if (f <= kStageRows) {
     // --- up to 64 rows
     const int ld = f | 1;
     double *Ls = lvl_smem, *rd = Ls + kStageRows * (kStageRows + 1), *sx = rd + kStageRows + warp * kStageRows;
@@ -566,37 +634,42 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_bwd_level(DevPlan P, DevFactor X,
   // --- more than 64 rows
   const double *L = X.arena + X.sn_off[s];
   const size_t sf = (size_t)f;
-  if (!large && apply_lt) prefetch_front(L, f, p);
+  if (apply_lt) prefetch_front(L, f, p);
   pdl_wait();
   pdl_trigger();
   double(*Ls)[33] = reinterpret_cast<double(*)[33]>(lvl_smem);
-  const bool in_smem = !large && (int64_t)f * nrhs <= kLvlDoubles - kStripDoubles;
+  const bool in_smem = (int64_t)f * nrhs <= kLvlDoubles - kStripDoubles;
   double *sv = in_smem ? lvl_smem + kStripDoubles : wk + roff;  // the pivots' values, then the rows past them
   const int64_t stride = in_smem ? f : rows_total;
-  // D^-1 of each pivot block (large: v[0:p) holds L21^T x_ext)
-  for (int c = tid; c < p; c += kLvlNT) {
-    const double *Lc = L + (size_t)c * sf;
-    const bool second = use_d && c > 0 && Lc[c - 1] != 0.0;
-    if (second) continue;
-    const int rc = rows[c], rc1 = c + 1 < p ? rows[c + 1] : rc;
-    for (int r = 0; r < nrhs; ++r) {
-      const double *xr = x + (int64_t)r * P.n;
-      double z0, z1;
-      bool pair;
-      pivot_value(Lc, f, c, p, use_d, xr[rc], use_d ? xr[rc1] : 0.0, z0, z1, pair);
-      double *v = sv + r * stride;
-      if (apply_lt && large) {
-        z0 -= v[c];
-        if (pair) z1 -= v[c + 1];
-      }
-      v[c] = z0;
-      if (pair) v[c + 1] = z1;
+  // the rows' values (four right-hand sides' loads in flight), then D^-1 of
+  // each pivot block
+  for (int i = tid; i < (apply_lt ? f : p); i += kLvlNT) {
+    const int ri = rows[i];
+    for (int r0 = 0; r0 < nrhs; r0 += 4) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = r0 + q < nrhs ? x[(int64_t)(r0 + q) * P.n + ri] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (r0 + q < nrhs) sv[(r0 + q) * stride + i] = v[q];
     }
   }
-  if (apply_lt && large) return;  // the block kernels (k_bwd_dots / k_bwd_tri) go on
-  if (apply_lt)
-    for (int i = p + tid; i < f; i += kLvlNT)
-      for (int r = 0; r < nrhs; ++r) sv[r * stride + i] = x[(int64_t)r * P.n + rows[i]];
+  if (use_d) {
+    __syncthreads();
+    for (int c = tid; c < p; c += kLvlNT) {
+      const double *Lc = L + (size_t)c * sf;
+      for (int r = 0; r < nrhs; ++r) {
+        double *v = sv + r * stride;
+        double z0, z1;
+        bool pair;
+        // (a pair's values are read and written by its first column's thread)
+        if (c > 0 && Lc[c - 1] != 0.0) break;
+        pivot_value(Lc, f, c, p, true, v[c], c + 1 < p ? v[c + 1] : 0.0, z0, z1, pair);
+        v[c] = z0;
+        if (pair) v[c + 1] = z1;
+      }
+    }
+  }
   __syncthreads();
   if (apply_lt) {
     // strips of 32 columns from the last: their products with every row past
