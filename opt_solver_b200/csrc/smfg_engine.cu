@@ -716,6 +716,8 @@ static int level_at_most(const Plan &pl, int l, int v) {
 // 65..95; a warp below). Half as many: 9% slower on one small trajectory KKT;
 // twice as many: 12% slower on a batch of 256 (fewer fronts resident).
 constexpr int kSmallNT = 128, kUpperNT = 256;
+// Threads of an indefinite front of 96..128 rows.
+constexpr int kMediumNT = 256;
 
 // Rows of the largest front that is assembled, factored and stored by one
 // block (k_small_front): those below the blocked size.
@@ -771,10 +773,10 @@ static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, in
       case kSmall: k_small_front<kSmallNT, 64><<<k.n, kSmallNT, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
       case kUpper: k_small_front<kUpperNT, 96><<<k.n, kUpperNT, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
       case kMedium:
-        // SPD fronts take their updates with four times the threads (per
+        // SPD fronts take their updates in tiles with twice the threads (per
         // entry the same operations in the same order)
         if (c.posdef) k_factor<512, true><<<k.n, 512, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax);
-        else k_factor<128, true><<<k.n, 128, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax);
+        else k_factor<kMediumNT, true><<<k.n, kMediumNT, sm, q>>>(d, x, k.i0, prm, k.fmin, k.fmax);
         break;
       case kGlobal: k_factor<512, false><<<k.n, 512, 0, q>>>(d, x, k.i0, prm, k.fmin, k.fmax); break;
     }
@@ -1003,7 +1005,7 @@ static void set_kernel_attrs(int nb) {
   if (done_nb == nb) return;
   SMFG_CUDA(cudaFuncSetAttribute(k_tri_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem));
   // (the with-W size: launches ask for at most this)
-  for (auto kern : {k_factor<128, true>, k_factor<512, true>})
+  for (auto kern : {k_factor<kMediumNT, true>, k_factor<512, true>})
     SMFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)front_smem_bytes(kMediumMax, nb)));
   SMFG_CUDA(cudaFuncSetAttribute(k_small_front<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,

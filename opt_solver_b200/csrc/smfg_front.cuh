@@ -440,8 +440,8 @@ __device__ __forceinline__ void inverse_2x2(double d00, double d10, double d11, 
   i11 = __dmul_rn(a, inv);
 }
 
-// Thread layout of the block's update loops: kRB consecutive rows per pass
-// (coalesced column-major accesses), NT / kRB column groups.
+// Thread layout of the block's update loops: RB consecutive rows per pass
+// (coalesced column-major accesses), NT / RB column groups.
 template <int NT>
 struct Lay {
   static constexpr int RB = NT < 128 ? NT : 128;
@@ -450,6 +450,77 @@ struct Lay {
   static __device__ __forceinline__ int g() { return threadIdx.x / RB; }
 };
 
+
+// Fronts of one block of fewer than 512 threads are in shared memory (at most
+// 128 rows).
+template <int NT>
+constexpr bool kSmemFront = NT < 512;
+
+// Columns (k, jend) of a front in shared memory minus pivot k's products:
+// F(i, j) -= F(i, k) l_j, l_j = F(j, k) inv, for j <= i < f (no update where
+// l_j is zero); a warp four columns at a time, lanes over the rows.
+// skip: the entry (skip, skip) is left (the caller forms it itself).
+template <int NT>
+__device__ __forceinline__ void small_update1(double *F, int ld, int f, int k, int jend, double inv, int skip) {
+  constexpr int NW = NT / 32, G = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *ck = F + k * ld;
+  for (int j0 = k + 1 + warp; j0 < jend; j0 += G * NW) {
+    double l[G];
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const int j = j0 + u * NW;
+      l[u] = j < jend ? __dmul_rn(ck[j], inv) : 0.0;
+    }
+    for (int i = j0 + lane; i < f; i += 32) {
+      const double w = ck[i];
+      double x[G];
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const int j = j0 + u * NW;
+        x[u] = (j <= i && j < jend) ? F[j * ld + i] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const int j = j0 + u * NW;
+        if (j <= i && j < jend && l[u] != 0.0 && (i != skip || j != skip)) F[j * ld + i] = __dsub_rn(x[u], __dmul_rn(w, l[u]));
+      }
+    }
+  }
+}
+
+// The same for the 2x2 pivot (k, k + 1) with inverse (i00, i10, i11).
+template <int NT>
+__device__ __forceinline__ void small_update2(double *F, int ld, int f, int k, int jend, double i00, double i10, double i11) {
+  constexpr int NW = NT / 32, G = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *c0 = F + k * ld, *c1 = c0 + ld;
+  for (int j0 = k + 2 + warp; j0 < jend; j0 += G * NW) {
+    double l0[G], l1[G];
+#pragma unroll
+    for (int u = 0; u < G; ++u) {
+      const int j = j0 + u * NW;
+      const double a0 = j < jend ? c0[j] : 0.0, a1 = j < jend ? c1[j] : 0.0;
+      l0[u] = __dadd_rn(__dmul_rn(i00, a0), __dmul_rn(i10, a1));
+      l1[u] = __dadd_rn(__dmul_rn(i10, a0), __dmul_rn(i11, a1));
+    }
+    for (int i = j0 + lane; i < f; i += 32) {
+      const double w0 = c0[i], w1 = c1[i];
+      double x[G];
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const int j = j0 + u * NW;
+        x[u] = (j <= i && j < jend) ? F[j * ld + i] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        const int j = j0 + u * NW;
+        if (j <= i && j < jend && !(l0[u] == 0.0 && l1[u] == 0.0))
+          F[j * ld + i] = __dsub_rn(x[u], __dadd_rn(__dmul_rn(w0, l0[u]), __dmul_rn(w1, l1[u])));
+      }
+    }
+  }
+}
 
 // Panels of up to this many columns right of the pivot take the
 // row-at-a-time elimination path (global-memory fronts: blocks of 512).
@@ -474,7 +545,9 @@ static __device__ void eliminate_1x1_blk(const FrontRef &v, int k, int ucol_end,
     for (int i = k + 1 + rk * NT + (int)threadIdx.x; i < f; i += C * NT) w[i] = ck[i];
   }
   const int nj = ucol_end - (k + 1);
-  if (NT >= 512 && nj <= kElimCols) {
+  if constexpr (kSmemFront<NT>) {
+    small_update1<NT>(v.F, v.ld, f, k, ucol_end, inv_d, -1);
+  } else if (nj <= kElimCols) {
     // a panel: the multipliers once in shared memory, then each thread
     // one row of every column at a time (all loads of the row in flight)
     __shared__ double s_l[kElimCols];
@@ -539,7 +612,9 @@ static __device__ void eliminate_2x2_blk(const FrontRef &v, int k, int ucol_end,
     }
   }
   const int nj = ucol_end - (k + 2);
-  if (NT >= 512 && nj <= kElimCols) {
+  if constexpr (kSmemFront<NT>) {
+    small_update2<NT>(v.F, v.ld, f, k, ucol_end, i00, i10, i11);
+  } else if (nj <= kElimCols) {
     // as eliminate_1x1_blk: multipliers in shared memory, rows in flight
     __shared__ double s_l0[kElimCols], s_l1[kElimCols];
     for (int jj = threadIdx.x; jj < nj; jj += NT) {
@@ -867,6 +942,79 @@ static __device__ int cand_eval_warp(const FrontRef &v, int k, int limit, int ca
   return 0;
 }
 
+// Maximum over the warp of non-negative, non-NaN doubles.
+__device__ __forceinline__ double warp_max_bits(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+__device__ __forceinline__ double abs_no_nan(double v) {  // |v|, NaN (ignored by the searches) as 0
+  const double a = fabs(v);
+  return a == a ? a : 0.0;
+}
+
+// cand_eval_warp on a front of at most 32 NS rows in shared memory: 0 when
+// column cand gives no pivot, else kind | a << 2 | b << 10 (b: the partner).
+// The first-column shortcut of select_pivot is this test's first outcome for
+// cand = k (its column maximum is the larger of m1 and ext). A warp's maxima
+// are integer reductions (two redux a maximum) in place of five shuffle
+// rounds on doubles.
+template <int NS>
+__device__ __forceinline__ int small_cand(const double *F, int ld, int f, int ne, int k, int limit, int cand,
+                                          const PivotParams &prm) {
+  const int lane = threadIdx.x & 31;
+  double x[NS];
+  double in = 0.0, ex = 0.0;
+#pragma unroll
+  for (int u = 0; u < NS; ++u) {
+    const int i = lane + 32 * u;
+    const bool on = i >= k && i < f && i != cand;
+    x[u] = on ? abs_no_nan(i > cand ? F[cand * ld + i] : F[i * ld + cand]) : 0.0;
+    if (i < ne) in = fmax(in, x[u]);
+    else ex = fmax(ex, x[u]);
+  }
+  const double a_cand = fabs(F[cand * ld + cand]);
+  const double m1 = warp_max_bits(in), ext = warp_max_bits(ex);
+  bool weak = false;
+  double weak_growth = 0.0;
+  if (a_cand >= prm.eff_small && !(__dmul_rn(prm.u, m1) > a_cand)) {
+    if (!(__dmul_rn(prm.u, ext) > a_cand)) {
+      const double colmax = dmax_ref(m1, ext);
+      if (!(a_cand < __dmul_rn(kWeakPivotRatio, colmax))) return 1 | (cand << 2);
+      weak = true;
+      weak_growth = colmax / a_cand;
+    }
+  }
+  unsigned r0 = 0x7fffffffu;
+#pragma unroll
+  for (int u = NS - 1; u >= 0; --u)
+    if (lane + 32 * u < ne && x[u] == m1) r0 = (unsigned)(lane + 32 * u);
+  const int r = (int)__reduce_min_sync(0xffffffffu, r0);  // first row of the largest entry
+  if (m1 <= 0.0 || r >= limit) return weak ? (1 | (cand << 2)) : 0;
+  double second = 0.0, off = 0.0;
+#pragma unroll
+  for (int u = 0; u < NS; ++u) {
+    const int i = lane + 32 * u;
+    if (i < ne && i != r) second = fmax(second, x[u]);
+    if (i >= k && i < f && i != r && i != cand)
+      off = fmax(off, abs_no_nan(i > r ? F[r * ld + i] : F[i * ld + r]));
+  }
+  const double m2 = warp_max_bits(second), off1 = warp_max_bits(off);
+  const double om2 = fmax(off1, m1);  // column r's maximum holds its entry in row cand, which is m1
+  const double d00 = F[cand * ld + cand], d11 = F[r * ld + r];
+  const double d10 = r >= cand ? F[cand * ld + r] : F[r * ld + cand];
+  double growth2 = 0.0;
+  if (k + 1 < limit && two_by_two_ok_s(d00, d10, d11, dmax_ref(m2, ext), off1, prm, growth2) &&
+      (!weak || growth2 < weak_growth))
+    return 2 | (cand << 2) | (r << 10);
+  if (weak) return 1 | (cand << 2);
+  const double a_r = fabs(d11);
+  if (a_r >= prm.eff_small && (om2 == 0.0 || a_r >= __dmul_rn(prm.u, om2))) return 1 | (r << 2);
+  return 0;
+}
+
 template <int NT, int C = 1>
 static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, const PivotParams &prm,
                                  FrontShared &sh) {
@@ -885,6 +1033,31 @@ static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, con
       sh.kind = kind;
       sh.a = pa;
       sh.b = pb;
+    }
+    __syncthreads();
+    return;
+  }
+  if constexpr (kSmemFront<NT>) {
+    // a warp per candidate, NT / 32 at a time, one barrier a round; the
+    // first that gives a pivot wins (two result buffers alternate). With the
+    // updates four columns a warp and (L D) formed once per pivot, fronts of
+    // 96..128 rows of a 200-stage trajectory KKT went from 210 to 100 us a
+    // level (factor + 8 solves 2.38 -> 1.65 ms; 256 of them 10.3 -> 9.4).
+    constexpr int NW = NT / 32;
+    const int warp = threadIdx.x >> 5;
+    int pick = 0;
+    for (int c0 = k; c0 < limit && !pick; c0 += NW) {
+      const int cand = c0 + warp;
+      const int got = cand < limit ? small_cand<4>(F, v.ld, f, v.ne, k, limit, cand, prm) : 0;
+      int *se = ((c0 - k) / NW & 1) ? sh.cb : sh.ca;
+      if ((threadIdx.x & 31) == 0) se[warp] = got;
+      __syncthreads();
+      for (int w = NW - 1; w >= 0; --w) pick = se[w] ? se[w] : pick;
+    }
+    if (threadIdx.x == 0) {
+      sh.kind = pick & 3;
+      sh.a = pick ? (pick >> 2) & 255 : -1;
+      sh.b = (pick & 3) == 2 ? pick >> 10 : -1;
     }
     __syncthreads();
     return;
@@ -1125,57 +1298,70 @@ static __device__ void front_update_tiles(const FrontRef &v, int c0, int cend, i
   __syncthreads();
 }
 
+// Columns [c0, cend) of the lower part of rows [c0, f) of a front in shared
+// memory minus L(i, p0 + q) B(q, j), B = W's rows q < kk (a row per pivot,
+// stride f): a chain over the pivots in order per entry (b = 0 skipped), a
+// thread four columns of a row at a time.
 template <int NT>
-static __device__ void deferred_update_blk(const FrontRef &v, int p0, int p1, int c0, int e) {
+static __device__ __forceinline__ void smem_update(const FrontRef &v, int p0, int kk, int c0, int cend) {
   using LY = Lay<NT>;
-  const int jb = p1 - p0;
-  if (jb <= 0 || e - c0 <= 0) return;
-  if constexpr (NT == 512) {  // fronts in global memory: tiles staged in shared memory
-    front_update_tiles<false>(v, c0, e, p0, jb);
-    return;
-  }
-  const size_t sf = (size_t)v.ld;
-  const int f = v.f;
+  const int f = v.f, ld = v.ld;
   for (int i = c0 + LY::r(); i < f; i += LY::RB) {
-    const int jend = min(e, i + 1);
-    for (int j = c0 + LY::g(); j < jend; j += LY::G) {
-      double c = v.F[(size_t)j * sf + i];
-      for (int p = 0; p < jb; ++p) {
-        const double b = v.W[(size_t)p * f + j];
-        if (b == 0.0) continue;
-        c = fma(-v.F[(size_t)(p0 + p) * sf + i], b, c);
+    const int jend = min(cend, i + 1);
+    for (int j0 = c0 + LY::g(); j0 < jend; j0 += 4 * LY::G) {
+      double c[4];
+      int j[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        j[u] = min(j0 + u * LY::G, f - 1);
+        c[u] = v.F[j[u] * ld + i];
       }
-      v.F[(size_t)j * sf + i] = c;
+      for (int p = 0; p < kk; ++p) {
+        const double a = -v.F[(p0 + p) * ld + i];
+        const double *w = v.W + p * f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double b = w[j[u]];
+          const double t = fma(a, b, c[u]);
+          c[u] = b != 0.0 ? t : c[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j0 + u * LY::G < jend) v.F[j[u] * ld + i] = c[u];
     }
   }
   __syncthreads();
 }
 
+template <int NT>
+static __device__ void deferred_update_blk(const FrontRef &v, int p0, int p1, int c0, int e) {
+  const int jb = p1 - p0;
+  if (jb <= 0 || e - c0 <= 0) return;
+  if constexpr (kSmemFront<NT>) smem_update<NT>(v, p0, jb, c0, e);
+  else front_update_tiles<false>(v, c0, e, p0, jb);
+}
 
 // schur_update (ldlt_kernel.cpp:820-933): F[e:f, e:f] -= L LD^T over the
-// pivots [p0, p) in order.
+// pivots [p0, p) in order. In shared memory: (L D)'s rows formed in W, nb
+// pivots at a time (W's panel is done with).
 template <int NT>
-static __device__ void schur_update_blk(const FrontRef &v, int p0, int p, int e) {
-  using LY = Lay<NT>;
+static __device__ void schur_update_blk(const FrontRef &v, int p0, int p, int e, int nb) {
   const int f = v.f;
   if (p <= p0 || f - e <= 0) return;
-  if constexpr (NT == 512) {  // fronts in global memory: tiles staged in shared memory
-    front_update_tiles<true>(v, e, f, p0, p - p0);
-    return;
-  }
-  const size_t sf = (size_t)v.ld;
-  for (int i = e + LY::r(); i < f; i += LY::RB) {
-    for (int j = e + LY::g(); j <= i; j += LY::G) {
-      double c = v.F[(size_t)j * sf + i];
-      for (int cc = p0; cc < p; ++cc) {
-        const double b = ld_entry(v, cc, j);
-        if (b == 0.0) continue;
-        c = fma(-v.F[(size_t)cc * sf + i], b, c);
+  if constexpr (kSmemFront<NT>) {
+    for (int q0 = p0; q0 < p; q0 += nb) {
+      const int kk = min(nb, p - q0);
+      for (int t = threadIdx.x; t < kk * (f - e); t += NT) {
+        const int q = t / (f - e), j = e + t % (f - e);
+        v.W[q * f + j] = ld_entry(v, q0 + q, j);
       }
-      v.F[(size_t)j * sf + i] = c;
+      __syncthreads();
+      smem_update<NT>(v, q0, kk, e, f);
     }
+  } else {
+    front_update_tiles<true>(v, e, f, p0, p - p0);
   }
-  __syncthreads();
 }
 
 // State of the blocked path of ldlt_factor_front between its panel steps
@@ -1482,7 +1668,7 @@ static __device__ int ldlt_factor_front_blk(const FrontRef &v, const PivotParams
   TppState S;
   tpp_init(S, ne, prm.posdef != 0);
   while (tpp_step_blk<NT>(v, prm, sh, S)) deferred_update_blk<NT>(v, S.g_p0, S.g_p1, S.g_c0, S.g_e);
-  if (do_schur) schur_update_blk<NT>(v, 0, S.k, ne);
+  if (do_schur) schur_update_blk<NT>(v, 0, S.k, ne, prm.nb);
   return S.k;
 }
 

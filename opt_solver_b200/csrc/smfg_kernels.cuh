@@ -440,7 +440,7 @@ __device__ int spd_front_panels(FrontRef &v, const PivotParams &prm, FrontShared
   }
   // the contribution block: its Schur update over every pivot, as the
   // medium kernel takes it
-  schur_update_blk<NT>(v, 0, p, ne);
+  schur_update_blk<NT>(v, 0, p, ne, NB);
   return p;
 }
 

@@ -39,77 +39,6 @@ __device__ __forceinline__ void small_sync() {
   else __syncthreads();
 }
 
-// Maximum over the warp of non-negative, non-NaN doubles.
-__device__ __forceinline__ double warp_max_bits(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  return __hiloint2double((int)mh, (int)ml);
-}
-
-__device__ __forceinline__ double abs_no_nan(double v) {  // |v|, NaN (ignored by the searches) as 0
-  const double a = fabs(v);
-  return a == a ? a : 0.0;
-}
-
-// cand_eval_warp (smfg_front.cuh) on a front of at most 32 NS rows in shared
-// memory: 0 when column cand gives no pivot, else kind | a << 2 | b << 10.
-// The first-column shortcut of select_pivot is this test's first outcome for
-// cand = k (its column maximum is the larger of m1 and ext).
-template <int NS>
-__device__ __forceinline__ int small_cand(const double *F, int ld, int f, int ne, int k, int cand,
-                                          const PivotParams &prm) {
-  const int lane = threadIdx.x & 31;
-  double x[NS];
-  double in = 0.0, ex = 0.0;
-#pragma unroll
-  for (int u = 0; u < NS; ++u) {
-    const int i = lane + 32 * u;
-    const bool on = i >= k && i < f && i != cand;
-    x[u] = on ? abs_no_nan(i > cand ? F[cand * ld + i] : F[i * ld + cand]) : 0.0;
-    if (i < ne) in = fmax(in, x[u]);
-    else ex = fmax(ex, x[u]);
-  }
-  const double a_cand = fabs(F[cand * ld + cand]);
-  const double m1 = warp_max_bits(in), ext = warp_max_bits(ex);
-  bool weak = false;
-  double weak_growth = 0.0;
-  if (a_cand >= prm.eff_small && !(__dmul_rn(prm.u, m1) > a_cand)) {
-    if (!(__dmul_rn(prm.u, ext) > a_cand)) {
-      const double colmax = dmax_ref(m1, ext);
-      if (!(a_cand < __dmul_rn(kWeakPivotRatio, colmax))) return 1 | (cand << 2);
-      weak = true;
-      weak_growth = colmax / a_cand;
-    }
-  }
-  if (m1 <= 0.0) return weak ? (1 | (cand << 2)) : 0;
-  unsigned r0 = 0x7fffffffu;
-#pragma unroll
-  for (int u = NS - 1; u >= 0; --u)
-    if (lane + 32 * u < ne && x[u] == m1) r0 = (unsigned)(lane + 32 * u);
-  const int r = (int)__reduce_min_sync(0xffffffffu, r0);  // first row of the largest entry
-  double second = 0.0, off = 0.0;
-#pragma unroll
-  for (int u = 0; u < NS; ++u) {
-    const int i = lane + 32 * u;
-    if (i < ne && i != r) second = fmax(second, x[u]);
-    if (i >= k && i < f && i != r && i != cand)
-      off = fmax(off, abs_no_nan(i > r ? F[r * ld + i] : F[i * ld + r]));
-  }
-  const double m2 = warp_max_bits(second), off1 = warp_max_bits(off);
-  const double om2 = fmax(off1, m1);  // column r's maximum holds its entry in row cand, which is m1
-  const double d00 = F[cand * ld + cand], d11 = F[r * ld + r];
-  const double d10 = r >= cand ? F[cand * ld + r] : F[r * ld + cand];
-  double growth2 = 0.0;
-  if (k + 1 < ne && two_by_two_ok_s(d00, d10, d11, dmax_ref(m2, ext), off1, prm, growth2) &&
-      (!weak || growth2 < weak_growth))
-    return 2 | (cand << 2) | (r << 10);
-  if (weak) return 1 | (cand << 2);
-  const double a_r = fabs(d11);
-  if (a_r >= prm.eff_small && (om2 == 0.0 || a_r >= __dmul_rn(prm.u, om2))) return 1 | (r << 2);
-  return 0;
-}
-
 // Rows and columns p < q of the front exchanged (sym_swap_blk's pairs), then
 // a barrier.
 template <int NT>
@@ -146,71 +75,6 @@ __device__ __forceinline__ void small_swap(double *F, int ld, int f, int *rows, 
     *b = x;
   }
   small_sync<NT>();
-}
-
-// The trailing triangle minus pivot k's products: F(i, j) -= F(i, k) l_j,
-// l_j = F(j, k) inv, for k < j <= i < f (no update where l_j is zero).
-// skip: the entry (skip, skip) is left (the caller forms it itself).
-template <int NT>
-__device__ __forceinline__ void small_update1(double *F, int ld, int f, int k, double inv, int skip) {
-  constexpr int NW = NT / 32, G = 4;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double *ck = F + k * ld;
-  for (int j0 = k + 1 + warp; j0 < f; j0 += G * NW) {
-    double l[G];
-#pragma unroll
-    for (int u = 0; u < G; ++u) {
-      const int j = j0 + u * NW;
-      l[u] = j < f ? __dmul_rn(ck[j], inv) : 0.0;
-    }
-    for (int i = j0 + lane; i < f; i += 32) {
-      const double w = ck[i];
-      double x[G];
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const int j = j0 + u * NW;
-        x[u] = (j <= i) ? F[j * ld + i] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const int j = j0 + u * NW;
-        if (j <= i && l[u] != 0.0 && (i != skip || j != skip)) F[j * ld + i] = __dsub_rn(x[u], __dmul_rn(w, l[u]));
-      }
-    }
-  }
-}
-
-// The same for the 2x2 pivot (k, k + 1) with inverse (i00, i10, i11).
-template <int NT>
-__device__ __forceinline__ void small_update2(double *F, int ld, int f, int k, double i00, double i10, double i11) {
-  constexpr int NW = NT / 32, G = 4;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double *c0 = F + k * ld, *c1 = c0 + ld;
-  for (int j0 = k + 2 + warp; j0 < f; j0 += G * NW) {
-    double l0[G], l1[G];
-#pragma unroll
-    for (int u = 0; u < G; ++u) {
-      const int j = j0 + u * NW;
-      const double a0 = j < f ? c0[j] : 0.0, a1 = j < f ? c1[j] : 0.0;
-      l0[u] = __dadd_rn(__dmul_rn(i00, a0), __dmul_rn(i10, a1));
-      l1[u] = __dadd_rn(__dmul_rn(i10, a0), __dmul_rn(i11, a1));
-    }
-    for (int i = j0 + lane; i < f; i += 32) {
-      const double w0 = c0[i], w1 = c1[i];
-      double x[G];
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const int j = j0 + u * NW;
-        x[u] = (j <= i) ? F[j * ld + i] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const int j = j0 + u * NW;
-        if (j <= i && !(l0[u] == 0.0 && l1[u] == 0.0))
-          F[j * ld + i] = __dsub_rn(x[u], __dadd_rn(__dmul_rn(w0, l0[u]), __dmul_rn(w1, l1[u])));
-      }
-    }
-  }
 }
 
 // One front of rows fmin..FMAX of the level list P.lvl_sn[i0 + blockIdx.x]
@@ -339,7 +203,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
         dn = l != 0.0 ? v : dn;
         ivn = 1.0 / dn;
       }
-      small_update1<NT>(F, ld, f, p, iv, p + 1 < ne ? p + 1 : -1);
+      small_update1<NT>(F, ld, f, p, f, iv, p + 1 < ne ? p + 1 : -1);
       small_sync<NT>();
       d = dn;
       iv = ivn;
@@ -359,7 +223,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
       int pick = 0;
       for (int c0 = p; c0 < ne; c0 += NW) {
         const int cand = c0 + warp;
-        const int got = cand < ne ? small_cand<NS>(F, ld, f, ne, p, cand, prm) : 0;
+        const int got = cand < ne ? small_cand<NS>(F, ld, f, ne, p, ne, cand, prm) : 0;
         if constexpr (NW == 1) {
           pick = got;
         } else {
@@ -385,7 +249,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
           q0[p] = iv;
           tags[p] = 1;
         }
-        small_update1<NT>(F, ld, f, p, iv, -1);
+        small_update1<NT>(F, ld, f, p, f, iv, -1);
         p += 1;
       } else {
         int partner = pick >> 10;
@@ -403,7 +267,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
           tags[p] = 2;
           tags[p + 1] = -1;
         }
-        small_update2<NT>(F, ld, f, p, i00, i10, i11);
+        small_update2<NT>(F, ld, f, p, f, i00, i10, i11);
         p += 2;
       }
       small_sync<NT>();
