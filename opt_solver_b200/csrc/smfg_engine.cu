@@ -130,23 +130,44 @@ static void large_state(Plan &pl) {
   pl.aptp_q = dalloc<int>(pl, ml);
 }
 
-// Fronts that delays took to the APTP size outside the large-front path
-// join it (the caller redoes the factorization).
-static void add_large(Plan &pl, const std::vector<int> &sn) {
+// The lists of pl.h_large on the device, with the state they size.
+static void upload_large(Plan &pl) {
   // a captured graph holds the old lists' and states' addresses
   if (pl.graph_exec) {
     cudaGraphExecDestroy(pl.graph_exec);
     pl.graph_exec = nullptr;
     pl.graph_key.clear();
   }
-  for (int s : sn) pl.h_large[s] = 1;
   large_lists(pl);
   dfree(pl, pl.d.lvl_large);
   dfree(pl, pl.d.sn_large);
   pl.d.lvl_large = dupload(pl, pl.h_lvl_large);
   pl.d.sn_large = dupload(pl, pl.h_large);
   large_state(pl);
+  pl.spd_layout = false;
   SMFG_CUDA(cudaStreamSynchronize(pl.stream));
+}
+
+// Fronts that delays took to the APTP size outside the large-front path
+// join it (the caller redoes the factorization).
+static void add_large(Plan &pl, const std::vector<int> &sn) {
+  for (int s : sn) pl.h_large[s] = pl.h_grown[s] = 1;
+  upload_large(pl);
+}
+
+// The large fronts of an SPD or an indefinite factorization: by symbolic
+// rows, and for the latter the fronts that delays took to the APTP size.
+static void set_large_mode(Plan &pl, int posdef) {
+  if (pl.large_mode == (posdef ? 1 : 0)) return;
+  pl.large_mode = posdef ? 1 : 0;
+  const int lim = posdef ? kLargeMinSpd : kLargeMin;
+  for (int s = 0; s < pl.nsn; ++s) pl.h_large[s] = pl.h_fsym[s] >= lim || (!posdef && pl.h_grown[s]) ? 1 : 0;
+  for (void *p : {(void *)pl.x.tri_inv, (void *)pl.x.sn_ioff, (void *)pl.x.inv_items}) dfree(pl, p);
+  pl.x.tri_inv = nullptr;
+  pl.x.sn_ioff = nullptr;
+  pl.x.inv_items = nullptr;
+  pl.x.inv_nitems = 0;
+  upload_large(pl);
 }
 
 static void build_plan(Plan &pl, const smfg_analysis_t &a) {
@@ -184,14 +205,12 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   for (int l = 0; l < nl; ++l)
     std::stable_sort(lvl_sn.begin() + pl.lvl_ptr[l], lvl_sn.begin() + pl.lvl_ptr[l + 1],
                      [&](int x, int y) { return fsym[x] > fsym[y]; });
-  // large fronts (multi-block path): by symbolic rows; fronts that delays
-  // take to the APTP size join later (large_lists)
+  // the large fronts (multi-block path) are listed by the first factorization
   pl.h_large.assign(ns, 0);
-  for (int s = 0; s < ns; ++s) pl.h_large[s] = fsym[s] >= kLargeMin ? 1 : 0;
+  pl.h_grown.assign(ns, 0);
   pl.h_lvl_sn = lvl_sn;
   pl.h_width = width;
   pl.h_fsym = fsym;
-  large_lists(pl);
   pl.lvl_maxf.assign(nl, 0);
   pl.lvl_maxkids.assign(nl, 0);
   for (int s = 0; s < ns; ++s) {
@@ -308,8 +327,6 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   d.cpr_off = dupload(pl, cpr_off);
   d.cpr_idx = dupload(pl, cpr_idx);
   d.lvl_sn = dupload(pl, lvl_sn);
-  d.lvl_large = dupload(pl, pl.h_lvl_large);
-  d.sn_large = dupload(pl, pl.h_large);
   d.sn_level = dupload(pl, level);
   d.pcp = dupload(pl, std::vector<int>(a.perm_col_ptr, a.perm_col_ptr + n + 1));
   d.pri = dupload(pl, std::vector<int>(a.perm_row_idx, a.perm_row_idx + pl.nnz));
@@ -344,7 +361,6 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   SMFG_CUDA(cudaMemsetAsync(x.sn_mixed, 0, ns, pl.stream));
   x.tc_njobs = dalloc<int>(pl, 1);
   x.aptp_miss = dalloc<int>(pl, kAptpMissCap);
-  large_state(pl);
   x.arena = nullptr;
   x.arena_cap = 0;
   x.rows = nullptr;
@@ -368,7 +384,62 @@ static void ensure_arena(Plan &pl, int64_t arena_need, int64_t rows_need) {
     x.cbmap = dalloc<int>(pl, rows_need);
     x.ploc = dalloc<int>(pl, 2 * (size_t)rows_need);
     x.rows_cap = rows_need;
+    pl.spd_layout = false;
   }
+}
+
+// Doubles of an SPD front of symbolic rows f in the static layout: the front
+// and its W (large fronts: wcols rows; those factored in global memory by one
+// block: nb; none in shared memory).
+static int64_t spd_front_doubles(const Plan &pl, int s, int wcols) {
+  const int64_t f = pl.h_fsym[s];
+  return f * f + f * (pl.h_large[s] ? wcols : f > kMediumMax ? pl.nb : 0);
+}
+static int64_t spd_arena_doubles(const Plan &pl, int wcols) {
+  int64_t t = 0;
+  for (int s = 0; s < pl.nsn; ++s) t += spd_front_doubles(pl, s, wcols);
+  return t;
+}
+
+// The static layout of an SPD factorization: sizes, arena and row offsets,
+// assembly work items of every front, its rows and its children's row maps,
+// in place of two kernels a level on every factorization (k_level_setup is
+// one block: 119 us for the 33,000 leaves of the 64^3 operator).
+static void ensure_spd_layout(Plan &pl, int wcols, int fuse) {
+  if (pl.spd_layout && pl.spd_wcols == wcols && pl.spd_fuse == fuse) return;
+  DevFactor &x = pl.x;
+  const int ns = pl.nsn, nl = pl.nlevels;
+  std::vector<int64_t> off(ns), roff(ns);
+  std::vector<int> blk((size_t)ns + nl + 1, 0);
+  int64_t a = 0, r = 0;
+  for (int l = 0; l < nl; ++l) {
+    int b = 0;
+    for (int i = pl.lvl_ptr[l]; i < pl.lvl_ptr[l + 1]; ++i) {
+      const int s = pl.h_lvl_sn[i], f = pl.h_fsym[s];
+      off[s] = a;
+      roff[s] = r;
+      a += spd_front_doubles(pl, s, wcols);
+      r += f;
+      blk[i + l] = b;
+      b += (f <= fuse && !pl.h_large[s]) ? 0 : (f + kAsmCols - 1) / kAsmCols;
+    }
+    blk[pl.lvl_ptr[l + 1] + l] = b;
+  }
+  cudaStream_t st = pl.stream;
+  SMFG_CUDA(cudaMemcpyAsync(x.sn_off, off.data(), sizeof(int64_t) * ns, cudaMemcpyHostToDevice, st));
+  SMFG_CUDA(cudaMemcpyAsync(x.sn_roff, roff.data(), sizeof(int64_t) * ns, cudaMemcpyHostToDevice, st));
+  SMFG_CUDA(cudaMemcpyAsync(x.lvl_blk, blk.data(), sizeof(int) * blk.size(), cudaMemcpyHostToDevice, st));
+  SMFG_CUDA(cudaMemcpyAsync(x.sn_f, pl.d.sn_fsym, sizeof(int) * ns, cudaMemcpyDeviceToDevice, st));
+  SMFG_CUDA(cudaMemcpyAsync(x.sn_ne, pl.d.sn_width, sizeof(int) * ns, cudaMemcpyDeviceToDevice, st));
+  SMFG_CUDA(cudaMemsetAsync(x.sn_nd, 0, sizeof(int) * ns, st));
+  SMFG_CUDA(cudaMemsetAsync(x.child_doff, 0, sizeof(int) * std::max<size_t>(1, pl.h_child_idx.size()), st));
+  if (ns > 0) k_level_rows<<<ns, 128, 0, st>>>(pl.d, x, 0, 0);
+  SMFG_CUDA(cudaGetLastError());
+  SMFG_CUDA(cudaStreamSynchronize(st));  // the host arrays are read
+  pl.spd_arena = a;
+  pl.spd_layout = true;
+  pl.spd_wcols = wcols;
+  pl.spd_fuse = fuse;
 }
 
 // ---------------------------------------------------------------------------
@@ -799,10 +870,14 @@ static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, in
   // rows and assembly of the fronts past fuse rows
   const int na = exact ? at_most(fuse) - lo : hi - lo;
   if (na > 0) {
-    k_level_rows<<<na, 128, 0, st>>>(d, x, lo, fuse);
+    if (!x.spd_static) {
+      // (a large front's thousands of rows: more threads a front)
+      k_level_rows<<<na, pl.lvl_maxf[l] >= 1024 ? 512 : 128, 0, st>>>(d, x, lo, fuse);
+      lc.n += 1;
+    }
     // 32-column work items: a level of a few large fronts has hundreds
-    k_level_assemble<<<4 * sm_count(pl.device), 256, 0, st>>>(d, x, lo, hi, l);
-    lc.n += 2;
+    k_level_assemble<<<8 * sm_count(pl.device), 256, 0, st>>>(d, x, lo, hi, l);
+    lc.n += 1;
   }
   if (nc > first && !fused(cls[first])) {
     SMFG_CUDA(cudaEventRecord(pl.ev_asm, st));
@@ -839,7 +914,9 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
   k_values<<<vgrid, 256, 0, st>>>(
       d_values, pl.nnz_in, d.vptr, d.vsrc, pcol, d.pri, d.perm, scale, pl.nnz, x.pv, x.pv_raw,
       x.counters);
-  k_eff_small<<<1, 1, 0, st>>>(x.counters, c.small_pivot);
+  const bool fixed_layout = x.spd_static != 0;  // SPD: sizes and offsets laid out before
+  k_eff_small<<<1, 1, 0, st>>>(x.counters, c.small_pivot, fixed_layout ? pl.spd_arena : 0,
+                               fixed_layout ? pl.sum_f : 0);
   lc.n += 2;
   const bool aptp_on = aptp_active(c);
   // early stops (indefinite): max_negative_pivots, the work limit
@@ -855,8 +932,10 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
   const int fuse = fuse_rows(c);
   for (int l = 0; l < pl.nlevels; ++l) {
     const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
-    k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse);
-    lc.n += 1;
+    if (!fixed_layout) {
+      k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse);
+      lc.n += 1;
+    }
     const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
     const unsigned side = launch_level_fronts(pl, c, l, fuse, prm, nL > 0, lc);
     if (nL > 0) {
@@ -1028,12 +1107,15 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
   (void)team16_ok(pl.device);  // queried here, outside any stream capture
   pl.nb = std::max(2, c.nb);
   set_kernel_attrs(pl.nb);
+  set_large_mode(pl, c.posdef);
+  if (!c.posdef) pl.spd_layout = false;
+  const int wcols = w_rows(pl, c, c.profile != 0), fuse = fuse_rows(c);
+  bool use_static = c.posdef != 0;
   // arena: exact for SPD (no delays); head-room for delays, regrown on overflow
   // (look-ahead: a second W buffer, nb columns more per front)
   // (the symbolic sizes hold nb W rows per front; the SPD steps need more)
-  const int64_t base_a = pl.sum_f2 + pl.sum_f * (int64_t)(w_rows(pl, c, c.profile != 0) - c.nb),
-                base_r = pl.sum_f;
-  int64_t need_a = c.posdef ? base_a : base_a + base_a / 4 + (int64_t)pl.max_fsym * pl.max_fsym * 2 + 4096;
+  const int64_t base_a = pl.sum_f2 + pl.sum_f * (int64_t)(wcols - c.nb), base_r = pl.sum_f;
+  int64_t need_a = c.posdef ? (pl.spd_layout && pl.spd_wcols == wcols ? pl.spd_arena : spd_arena_doubles(pl, wcols)) : base_a + base_a / 4 + (int64_t)pl.max_fsym * pl.max_fsym * 2 + 4096;
   int64_t need_r = c.posdef ? base_r : base_r + base_r / 2 + 4096;
   // mixed fronts: large, at least min_front rows, allowed by the caller's mask
   const MixedCfg mc = mixed_cfg(c);
@@ -1089,6 +1171,7 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     put(&pl.x.tc_img, sizeof(pl.x.tc_img));
     put(&pl.x.tri_inv, sizeof(pl.x.tri_inv));
     if (pl.graph_exec && key == pl.graph_key) {
+      if (pl.graph_static) ensure_spd_layout(pl, wcols, fuse);
       if (c.scale)
         SMFG_CUDA(cudaMemcpyAsync(pl.x.scale, c.scale, sizeof(double) * pl.n, cudaMemcpyHostToDevice, pl.stream));
       SMFG_CUDA(cudaEventRecord(pl.ev0, pl.stream));
@@ -1099,13 +1182,18 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
       SMFG_CUDA(cudaStreamSynchronize(pl.stream));
       SMFG_CUDA(cudaEventElapsedTime(&ms, pl.ev0, pl.ev1));
       const unsigned fl = (unsigned)h_cnt[kCFlags];
-      replayed = !(fl & (kFArena | kFRows | kFTcCap | kFSteps | kFAptpMiss));
+      replayed = !(fl & (kFArena | kFRows | kFTcCap | kFSteps | kFAptpMiss | kFStatic));
+      if (fl & kFStatic) use_static = false;
       lc.n = pl.graph_launches;
     }
   }
   int attempt_extra = 0;
   for (int attempt = 0; attempt < 4 && !replayed; ++attempt) {
+    if (c.posdef && !use_static) need_a = std::max(need_a, base_a);
     ensure_arena(pl, std::max(need_a, pl.x.arena_cap), std::max(need_r, pl.x.rows_cap));
+    pl.x.spd_static = use_static ? 1 : 0;
+    if (use_static) ensure_spd_layout(pl, wcols, fuse);
+    else pl.spd_layout = false;
     if (pl.x.tc_img_cap < tc_need) {
       dfree(pl, pl.x.tc_img);
       pl.x.tc_img = dalloc<uint8_t>(pl, tc_need);
@@ -1126,6 +1214,13 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     SMFG_CUDA(cudaStreamSynchronize(pl.stream));
     SMFG_CUDA(cudaEventElapsedTime(&ms, pl.ev0, pl.ev1));
     const unsigned flags = (unsigned)h_cnt[kCFlags];
+    if (flags & kFStatic) {
+      // not positive definite: redone with the failed columns delayed, as the
+      // reference reports it
+      use_static = false;
+      --attempt;
+      continue;
+    }
     if (flags & (kFArena | kFRows)) {
       need_a = std::max<int64_t>(need_a * 2, (int64_t)h_cnt[kCArena] * 2);
       need_r = std::max<int64_t>(need_r * 2, (int64_t)h_cnt[kCRows] * 2);
@@ -1177,14 +1272,17 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
       cudaGraphDestroy(g);
       pl.graph_key = key;
       pl.graph_launches = glc.n + 1;
+      pl.graph_static = pl.x.spd_static != 0;
     } else {
       clear_stale_error();
     }
   }
   const unsigned flags = (unsigned)h_cnt[kCFlags];
-  // stored pivots of the large fronts by level (the solves' block counts)
-  pl.lvl_large_pmax.assign(pl.nlevels, 0);
-  if (!pl.h_lvl_large.empty()) {
+  // stored pivots of the large fronts by level (the solves' block counts);
+  // SPD: their widths
+  if (c.posdef) {
+    pl.lvl_large_pmax = pl.lvl_large_maxw;
+  } else if (pl.lvl_large_pmax.assign(pl.nlevels, 0); !pl.h_lvl_large.empty()) {
     std::vector<int> pst(pl.nsn);
     SMFG_CUDA(cudaMemcpy(pst.data(), pl.x.sn_pstore, sizeof(int) * pl.nsn, cudaMemcpyDeviceToHost));
     for (int l = 0; l < pl.nlevels; ++l)

@@ -59,6 +59,7 @@ struct DevFactor {
   int *cbmap = nullptr;       // CB row -> parent position, at the child's sn_roff + p
   int *ploc = nullptr;        // 2 x rows_cap: pivot-order tracking of global-memory fronts
   int64_t rows_cap = 0;
+  int spd_static = 0;         // SPD on the static layout: a failed pivot also sets kFStatic
   unsigned long long *counters = nullptr;  // [0] arena base, [1] rows base, [2] error flags, [3] max|A| bits, [4] blocks
   TppState *tpp = nullptr;    // per large front of a level: blocked-pivoting state
   unsigned *team_bar = nullptr;  // per large front of a level: its CTA team's barrier words
@@ -97,6 +98,15 @@ struct Plan {
   std::vector<int> lvl_large_pmax; // most stored pivots among them (last factorization)
   std::vector<int> h_lvl_large;    // host copy of the large-front lists
   std::vector<int8_t> h_large;     // per supernode: the large-front path (symbolic rows, or grown by delays)
+  std::vector<int8_t> h_grown;     // indefinite fronts that delays took to the APTP size
+  int large_mode = -1;             // the lists' factorization kind: 1 SPD, 0 indefinite, -1 none yet
+  // SPD fronts take no delays: their sizes, offsets, rows and row maps are
+  // the analysis', laid out once (spd_wcols: its W rows, spd_fuse: its
+  // fused class), until an indefinite factorization overwrites them
+  bool spd_layout = false;
+  int spd_wcols = 0, spd_fuse = 0;
+  int64_t spd_arena = 0;
+  bool graph_static = false;       // the captured graph runs on the static layout
   std::vector<int> h_lvl_sn, h_width;  // supernodes by level; pivot columns
   int max_large = 0;
   int64_t sum_f2 = 0, sum_f = 0; // symbolic
