@@ -430,7 +430,12 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
 
 // Fronts of at least this many symbolic rows take the multi-block path.
 constexpr int kLargeMin = 384;
-constexpr int kLargeMinSpd = 384;  // SPD factorizations
+// SPD fronts already from fewer: one block takes a front of 380 rows 400 us,
+// the multi-block steps 130 (one SM's FP64 rate bounds the block). Measured
+// with 384 / 256 / 192 / 144: 701 x 433 Laplacian 6.85 / 5.75 / 5.64 / 5.79 ms,
+// 23 x 19 x 21 operator 4.39 / 4.04 / 3.93 / 3.95, 64^3 36.8 / 37.1 / 37.2 / 37.7
+// (more fronts a level in the multi-block kernels).
+constexpr int kLargeMinSpd = 192;
 
 // In-place unit-LDL^T of the nbp x nbp lower block T (the SPD panels'
 // diagonal blocks), all threads of the block: pivot k's reciprocal to
