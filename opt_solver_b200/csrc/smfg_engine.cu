@@ -115,14 +115,11 @@ static void large_lists(Plan &pl) {
 // Device state sized by the most large fronts of a level.
 static void large_state(Plan &pl) {
   DevFactor &x = pl.x;
-  for (void *p : {(void *)x.tpp, (void *)x.team_bar, (void *)x.team_red, (void *)x.tc_jobs, (void *)x.tc_ipref,
+  for (void *p : {(void *)x.tpp, (void *)x.tc_jobs, (void *)x.tc_ipref,
                   (void *)x.tc_tpref, (void *)pl.aptp_sizes, (void *)pl.aptp_q})
     dfree(pl, p);
   const size_t ml = (size_t)std::max(1, pl.max_large);
   x.tpp = dalloc<TppState>(pl, 2 * ml);  // two buffers (SPD panels)
-  x.team_bar = dalloc<unsigned>(pl, 2 * ml);
-  SMFG_CUDA(cudaMemsetAsync(x.team_bar, 0, sizeof(unsigned) * 2 * ml, pl.stream));
-  x.team_red = dalloc<double>(pl, (size_t)kTeamRedDoubles * ml);
   x.tc_jobs = dalloc<tc::Job>(pl, ml);
   x.tc_ipref = dalloc<int64_t>(pl, ml + 1);
   x.tc_tpref = dalloc<int>(pl, ml + 1);
@@ -590,7 +587,7 @@ static int level_team(const Plan &pl, const smfg_control_t &c, int maxf) {
 template <int C>
 static void launch_panel_c(Plan &pl, const int *lg, int nL, const PivotParams &prm, int it) {
   if constexpr (C == 1) {
-    k_large_panel<512, 1><<<nL, 512, 0, pl.stream>>>(pl.d, pl.x, lg, prm, it, pl.x.team_bar);
+    k_large_panel<512, 1><<<nL, 512, 0, pl.stream>>>(pl.d, pl.x, lg, prm, it);
   } else {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nL * C), 1, 1);
@@ -604,7 +601,7 @@ static void launch_panel_c(Plan &pl, const int *lg, int nL, const PivotParams &p
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    SMFG_CUDA(cudaLaunchKernelEx(&cfg, k_large_panel<512, C>, pl.d, pl.x, lg, prm, it, pl.x.team_bar));
+    SMFG_CUDA(cudaLaunchKernelEx(&cfg, k_large_panel<512, C>, pl.d, pl.x, lg, prm, it));
   }
 }
 

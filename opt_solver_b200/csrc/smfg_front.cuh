@@ -36,6 +36,8 @@ struct FrontStats {
   double flops;
 };
 
+constexpr int kTeamMax = 16;  // CTAs of a team (a thread-block cluster)
+
 // Shared control block of a front kernel.
 struct FrontShared {
   double red[32];
@@ -52,6 +54,9 @@ struct FrontShared {
   double pin[64], pout[64];
   int pr[64];
   int tr_seq;  // team reductions so far (alike in every CTA of a team)
+  // the team's partial results, a row per CTA, written by each CTA into every
+  // one of the team (two buffers alternate)
+  double team[2][kTeamMax][6];
   FrontStats st;
 };
 
@@ -83,19 +88,25 @@ __device__ __forceinline__ void top2_add(Top2 &t, double v, int i) {
   }
 }
 
-__device__ __forceinline__ Top2 top2_merge(Top2 a, Top2 b) {
+
+// Maximum over the warp of non-negative, non-NaN doubles.
+__device__ __forceinline__ double warp_max_bits(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+__device__ __forceinline__ double warp_max(double v) { return warp_max_bits(v); }
+
+// The warp's Top2: the maximum, its lowest index, and the largest of the rest
+// (a lane's runner-up, or another lane's maximum).
+__device__ __forceinline__ Top2 warp_top2(Top2 t) {
   Top2 o;
-  if (a.m1 > b.m1) {
-    o.m1 = a.m1;
-    o.r = a.r;
-  } else if (b.m1 > a.m1) {
-    o.m1 = b.m1;
-    o.r = b.r;
-  } else {
-    o.m1 = a.m1;
-    o.r = (a.r < 0) ? b.r : ((b.r < 0) ? a.r : min(a.r, b.r));
-  }
-  o.m2 = fmax(fmin(a.m1, b.m1), fmax(a.m2, b.m2));
+  o.m1 = warp_max_bits(t.m1);
+  const unsigned r = __reduce_min_sync(0xffffffffu, t.m1 == o.m1 && t.r >= 0 ? (unsigned)t.r : 0x7fffffffu);
+  o.r = r == 0x7fffffffu ? -1 : (int)r;
+  o.m2 = warp_max_bits(t.m1 == o.m1 && t.r == o.r ? t.m2 : t.m1);
   return o;
 }
 
@@ -104,52 +115,22 @@ struct Block {
   static_assert(NT % 32 == 0 && NT <= 1024, "block size");
   static constexpr int NW = NT / 32;
 
-  // Max of non-negative values, NaN ignored (fmax).
+  // Max of non-negative values.
   static __device__ double max(double v, FrontShared &sh) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    v = warp_max(v);
     if (NW == 1) return v;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     __syncthreads();
     if (l == 0) sh.red[w] = v;
     __syncthreads();
-    v = (l < NW) ? sh.red[l] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-  }
-
-  // Two maxima at once.
-  static __device__ void max2(double &a, double &b, FrontShared &sh) {
-    for (int o = 16; o > 0; o >>= 1) {
-      a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-      b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    if (NW == 1) return;
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) {
-      sh.red[w] = a;
-      sh.red2[w] = b;
-    }
-    __syncthreads();
-    a = (l < NW) ? sh.red[l] : 0.0;
-    b = (l < NW) ? sh.red2[l] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) {
-      a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-      b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
+    return warp_max((l < NW) ? sh.red[l] : 0.0);
   }
 
   // A Top2 and two maxima in one pass (one shared-memory round).
   static __device__ void bundle(Top2 &t, double &a, double &b, FrontShared &sh) {
-    for (int o = 16; o > 0; o >>= 1) {
-      Top2 u;
-      u.m1 = __shfl_xor_sync(0xffffffffu, t.m1, o);
-      u.m2 = __shfl_xor_sync(0xffffffffu, t.m2, o);
-      u.r = __shfl_xor_sync(0xffffffffu, t.r, o);
-      t = top2_merge(t, u);
-      a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-      b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
+    t = warp_top2(t);
+    a = warp_max(a);
+    b = warp_max(b);
     if (NW == 1) return;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     __syncthreads();
@@ -161,75 +142,16 @@ struct Block {
       sh.pout[w] = b;
     }
     __syncthreads();
+    Top2 o{0.0, 0.0, -1};
+    double x = 0.0, y = 0.0;
     if (l < NW) {
-      t.m1 = sh.red[l];
-      t.m2 = sh.red2[l];
-      t.r = sh.redi[l];
-      a = sh.pin[l];
-      b = sh.pout[l];
-    } else {
-      t.m1 = 0.0;
-      t.m2 = 0.0;
-      t.r = -1;
-      a = 0.0;
-      b = 0.0;
+      o = Top2{sh.red[l], sh.red2[l], sh.redi[l]};
+      x = sh.pin[l];
+      y = sh.pout[l];
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      Top2 u;
-      u.m1 = __shfl_xor_sync(0xffffffffu, t.m1, o);
-      u.m2 = __shfl_xor_sync(0xffffffffu, t.m2, o);
-      u.r = __shfl_xor_sync(0xffffffffu, t.r, o);
-      t = top2_merge(t, u);
-      a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-      b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-  }
-
-  static __device__ Top2 top2(Top2 t, FrontShared &sh) {
-    for (int o = 16; o > 0; o >>= 1) {
-      Top2 u;
-      u.m1 = __shfl_xor_sync(0xffffffffu, t.m1, o);
-      u.m2 = __shfl_xor_sync(0xffffffffu, t.m2, o);
-      u.r = __shfl_xor_sync(0xffffffffu, t.r, o);
-      t = top2_merge(t, u);
-    }
-    if (NW == 1) return t;
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) {
-      sh.red[w] = t.m1;
-      sh.red2[w] = t.m2;
-      sh.redi[w] = t.r;
-    }
-    __syncthreads();
-    if (l < NW) {
-      t.m1 = sh.red[l];
-      t.m2 = sh.red2[l];
-      t.r = sh.redi[l];
-    } else {
-      t.m1 = 0.0;
-      t.m2 = 0.0;
-      t.r = -1;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      Top2 u;
-      u.m1 = __shfl_xor_sync(0xffffffffu, t.m1, o);
-      u.m2 = __shfl_xor_sync(0xffffffffu, t.m2, o);
-      u.r = __shfl_xor_sync(0xffffffffu, t.r, o);
-      t = top2_merge(t, u);
-    }
-    return t;
-  }
-
-  // First index i in [lo, hi) of the largest |col[i]| (> 0), the
-  // reference's "if (v > out_max)" scan; -1 when all are zero.
-  static __device__ void argmax(const double *col, int lo, int hi, double &m, int &r,
-                                FrontShared &sh) {
-    Top2 t{0.0, 0.0, -1};
-    for (int i = lo + (int)threadIdx.x; i < hi; i += NT) top2_add(t, fabs(col[i]), i);
-    t = top2(t, sh);
-    m = t.m1;
-    r = t.r;
+    t = warp_top2(o);
+    a = warp_max(x);
+    b = warp_max(y);
   }
 };
 
@@ -254,13 +176,6 @@ struct FrontRef {
   int *loc;  // assembly position of the row now at each position (null: untracked)
   int *inv = nullptr;  // position of each assembly position (kept with loc; null: untracked)
   PairScratch *pair = nullptr;  // shared-memory scratch of the tracked pairing swaps
-  // teams of several CTAs: the team's barrier counter, the error word a
-  // timed-out barrier sets, this CTA's abort flag
-  unsigned *team_bar = nullptr;  // this launch's arrival counter (monotone within the launch)
-  unsigned long long *err = nullptr;
-  int *abort = nullptr;
-  unsigned *bar_seq = nullptr;    // this CTA's barriers so far in the launch (shared memory)
-  double *team_red = nullptr;  // the team's reduction scratch: 2 buffers x C ranks x 4
 };
 
 // A team of C CTAs (a thread-block cluster; C = 1: the CTA alone) that runs
@@ -280,46 +195,33 @@ __device__ __forceinline__ int team_rank() {
   }
 }
 
-// Team barrier (C > 1): an arrival counter in global memory that only grows
-// during a launch (the launch's own slot, reset by the previous launch): the
-// i-th barrier adds 1 (acquire-release: the last arrival reads the others'
-// writes through it) and waits, with acquire loads, until the counter
-// reaches C (i + 1). The spin is bounded by the
-// global timer (2 s): a team whose CTAs did not all arrive sets bit 128 of
-// *err, and the CTA stops waiting at its later barriers (the host then
-// discards the factorization and reports the timeout). The team's CTAs are
-// co-scheduled (one cluster), so the wait only runs out if they took
-// different paths.
+// Team barrier (C > 1): the cluster's hardware barrier, which also orders the
+// team's global and shared memory accesses before it with those after it.
+// Every decision is taken alike by every CTA of the team from the same data
+// (the state of the front, never a flag that another kernel may set
+// meanwhile), so each thread reaches the same barriers; threads that have
+// left the kernel count as arrived. It replaced an arrival counter in global
+// memory with polled loads (about 1,500 cycles a barrier, several a pivot).
 template <int C>
-__device__ __forceinline__ void team_sync(const FrontRef &v) {
+__device__ __forceinline__ void team_sync() {
   if constexpr (C == 1) {
     __syncthreads();
   } else {
-    __syncthreads();
-    if (threadIdx.x == 0 && !*v.abort) {
-      const unsigned target = (unsigned)C * (*v.bar_seq + 1u);
-      *v.bar_seq += 1u;
-      unsigned seen;
-      asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(seen) : "l"(v.team_bar) : "memory");
-      seen += 1u;
-      if (seen < target) {
-        unsigned long long t0;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-        while (true) {
-          asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(v.team_bar) : "memory");
-          if (seen >= target) break;
-          unsigned long long t;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-          if (t - t0 > 2000000000ull) {
-            *v.abort = 1;
-            atomicOr(v.err, 128ull);
-            break;
-          }
-        }
-      }
-    }
-    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   }
+}
+
+// Stores v at the address that `p` (this CTA's shared memory) has in CTA
+// `rank` of the team.
+__device__ __forceinline__ void team_store(double *p, int rank, double v) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile(
+      "{\n"
+      ".reg .b32 r;\n"
+      "mapa.shared::cluster.u32 r, %0, %1;\n"
+      "st.shared::cluster.f64 [r], %2;\n"
+      "}\n" ::"r"(a), "r"(rank), "d"(v) : "memory");
 }
 
 __device__ __forceinline__ double fat(const FrontRef &v, int i, int j) {  // element (i, j), i >= j
@@ -338,7 +240,7 @@ static __device__ bool sym_swap_blk(const FrontRef &v, int p, int q, int w_cols,
   // no CTA of the team writes while another still reads (C > 1); a swap
   // that follows a team barrier (the previous swap's) needs no other
   if constexpr (C > 1) {
-    if (!synced) team_sync<C>(v);
+    if (!synced) team_sync<C>();
   }
   const size_t sf = (size_t)v.ld;
   double *F = v.F;
@@ -387,7 +289,7 @@ static __device__ bool sym_swap_blk(const FrontRef &v, int p, int q, int w_cols,
       W[q] = x;
     }
   }
-  team_sync<C>(v);
+  team_sync<C>();
   return true;
 }
 
@@ -534,7 +436,7 @@ static __device__ void eliminate_1x1_blk(const FrontRef &v, int k, int ucol_end,
   const int rk = team_rank<C>();
   // (a swap that just ended with a team barrier needs no second one)
   if constexpr (C > 1) {
-    if (!synced) team_sync<C>(v);
+    if (!synced) team_sync<C>();
   }
   const size_t sf = (size_t)v.ld;
   const int f = v.f;
@@ -581,7 +483,7 @@ static __device__ void eliminate_1x1_blk(const FrontRef &v, int k, int ucol_end,
       }
     }
   }
-  team_sync<C>(v);
+  team_sync<C>();
   for (int i = k + 1 + rk * NT + (int)threadIdx.x; i < f; i += C * NT) ck[i] = __dmul_rn(ck[i], inv_d);
   // no barrier after the scaling for a team: the next pivot search reads
   // only later columns, and the next swap or elimination starts with one
@@ -595,7 +497,7 @@ static __device__ void eliminate_2x2_blk(const FrontRef &v, int k, int ucol_end,
   const int rk = team_rank<C>();
   // (a swap that just ended with a team barrier needs no second one)
   if constexpr (C > 1) {
-    if (!synced) team_sync<C>(v);
+    if (!synced) team_sync<C>();
   }
   const size_t sf = (size_t)v.ld;
   const int f = v.f;
@@ -653,7 +555,7 @@ static __device__ void eliminate_2x2_blk(const FrontRef &v, int k, int ucol_end,
       }
     }
   }
-  team_sync<C>(v);
+  team_sync<C>();
   for (int i = k + 2 + rk * NT + (int)threadIdx.x; i < f; i += C * NT) {
     const double a0 = c0[i], a1 = c1[i];
     c0[i] = __dadd_rn(__dmul_rn(i00, a0), __dmul_rn(i10, a1));
@@ -685,21 +587,6 @@ __device__ __forceinline__ bool two_by_two_ok_s(double d00, double d10, double d
 }
 
 // select_pivot (ldlt_kernel.cpp:127-275). Result in sh.kind / sh.a / sh.b.
-__device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-__device__ __forceinline__ Top2 warp_top2(Top2 t) {
-  for (int o = 16; o > 0; o >>= 1) {
-    Top2 u;
-    u.m1 = __shfl_xor_sync(0xffffffffu, t.m1, o);
-    u.m2 = __shfl_xor_sync(0xffffffffu, t.m2, o);
-    u.r = __shfl_xor_sync(0xffffffffu, t.r, o);
-    t = top2_merge(t, u);
-  }
-  return t;
-}
 
 // |col[i]| for i in [lo, hi), thread tid of nth: 16-byte loads of aligned
 // pairs, eight pairs in flight; each thread visits its indexes in increasing
@@ -741,39 +628,39 @@ __device__ __forceinline__ void scanv(const double *__restrict__ col, int lo, in
 
 // Team-wide reduction of a bundle (a Top2 and two maxima): the block's
 // reduction, then for a team of C > 1 CTAs each CTA's partial to the team's
-// scratch, a team barrier and the C partials merged in rank order by every
-// CTA (the merges are exact and order-independent, so every CTA holds the
-// one-CTA result). Two buffers alternate: a buffer is rewritten only after
-// the barrier of the next reduction, which every CTA reaches after reading.
+// slots, a team barrier and the C partials merged by every warp (the merges
+// are exact and order-independent, so every CTA holds the one-CTA result).
+// Two buffers alternate: a buffer is rewritten only after the barrier of the
+// next reduction, which every CTA reaches after reading.
 template <int NT, int C>
 static __device__ void team_bundle(const FrontRef &v, FrontShared &sh, Top2 &t, double &x1, double &x2) {
   Block<NT>::bundle(t, x1, x2, sh);
   if constexpr (C > 1) {
-    const int buf = sh.tr_seq & 1;
-    double *slot = v.team_red + (size_t)buf * C * 6;  // per rank: Top2 (4), maxima (2)
+    // each CTA's partial into every CTA of the team; after the barrier a
+    // warp's lanes merge the C rows
+    double(*slot)[6] = sh.team[sh.tr_seq & 1];
     const int rank = team_rank<C>();
-    if (threadIdx.x == 0) {
-      slot[rank * 4 + 0] = t.m1;
-      slot[rank * 4 + 1] = t.m2;
-      slot[rank * 4 + 2] = __longlong_as_double((long long)t.r);
-      slot[rank * 4 + 3] = 0.0;
-      slot[C * 4 + rank * 2 + 0] = x1;
-      slot[C * 4 + rank * 2 + 1] = x2;
+    if ((int)threadIdx.x < C) {
+      double *row = slot[rank];
+      team_store(row + 0, threadIdx.x, t.m1);
+      team_store(row + 1, threadIdx.x, t.m2);
+      team_store(row + 2, threadIdx.x, __longlong_as_double((long long)t.r));
+      team_store(row + 3, threadIdx.x, x1);
+      team_store(row + 4, threadIdx.x, x2);
     }
-    team_sync<C>(v);
+    team_sync<C>();
+    const int lane = threadIdx.x & 31;
     Top2 o{0.0, 0.0, -1};
     double a = 0.0, b = 0.0;
-    for (int q = 0; q < C; ++q) {
-      Top2 u{__ldcg(slot + q * 4 + 0), __ldcg(slot + q * 4 + 1),
-             (int)__double_as_longlong(__ldcg(slot + q * 4 + 2))};
-      o = top2_merge(o, u);
-      a = fmax(a, __ldcg(slot + C * 4 + q * 2 + 0));
-      b = fmax(b, __ldcg(slot + C * 4 + q * 2 + 1));
+    if (lane < C) {
+      const double *row = slot[lane];
+      o = Top2{row[0], row[1], (int)__double_as_longlong(row[2])};
+      a = row[3];
+      b = row[4];
     }
-    t = o;
-    x1 = a;
-    x2 = b;
-    __syncthreads();
+    t = warp_top2(o);
+    x1 = warp_max(a);
+    x2 = warp_max(b);
     if (threadIdx.x == 0) sh.tr_seq += 1;
     __syncthreads();
   }
@@ -942,14 +829,6 @@ static __device__ int cand_eval_warp(const FrontRef &v, int k, int limit, int ca
   return 0;
 }
 
-// Maximum over the warp of non-negative, non-NaN doubles.
-__device__ __forceinline__ double warp_max_bits(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  return __hiloint2double((int)mh, (int)ml);
-}
-
 __device__ __forceinline__ double abs_no_nan(double v) {  // |v|, NaN (ignored by the searches) as 0
   const double a = fabs(v);
   return a == a ? a : 0.0;
@@ -1095,19 +974,19 @@ static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, con
       const int cand = c0 + rank;
       int tk = 0, ta = -1, tb = -1;
       if (cand < limit) tk = cand_eval_team<NT, 1>(v, k, limit, cand, prm, sh, ta, tb);
-      double *slot = v.team_red + (size_t)(sh.tr_seq & 1) * C * 6;
-      if (threadIdx.x == 0) {
-        slot[rank * 4 + 0] = (double)tk;
-        slot[rank * 4 + 1] = (double)ta;
-        slot[rank * 4 + 2] = (double)tb;
+      double(*slot)[6] = sh.team[sh.tr_seq & 1];
+      if ((int)threadIdx.x < C) {
+        team_store(slot[rank] + 0, threadIdx.x, (double)tk);
+        team_store(slot[rank] + 1, threadIdx.x, (double)ta);
+        team_store(slot[rank] + 2, threadIdx.x, (double)tb);
       }
-      team_sync<C>(v);
+      team_sync<C>();
       for (int q = 0; q < C; ++q) {
-        const int qk = (int)__ldcg(slot + q * 4 + 0);
+        const int qk = (int)slot[q][0];
         if (qk) {
           kind = qk;
-          pa = (int)__ldcg(slot + q * 4 + 1);
-          pb = (int)__ldcg(slot + q * 4 + 2);
+          pa = (int)slot[q][1];
+          pb = (int)slot[q][2];
           done = true;
           break;
         }

@@ -62,8 +62,6 @@ struct DevFactor {
   int spd_static = 0;         // SPD on the static layout: a failed pivot also sets kFStatic
   unsigned long long *counters = nullptr;  // [0] arena base, [1] rows base, [2] error flags, [3] max|A| bits, [4] blocks
   TppState *tpp = nullptr;    // per large front of a level: blocked-pivoting state
-  unsigned *team_bar = nullptr;  // per large front of a level: its CTA team's barrier words
-  double *team_red = nullptr;    // per large front of a level: its team's reduction scratch
   int *aptp_miss = nullptr;   // fronts that reached the APTP size outside the large-front path
   double *work = nullptr;     // solve / refinement scratch
   int64_t work_cap = 0;

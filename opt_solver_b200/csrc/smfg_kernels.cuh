@@ -16,8 +16,6 @@ enum : int { kCArena = 0, kCRows = 1, kCFlags = 2, kCMaxAbs = 3, kCAux = 4, kCEf
 enum : unsigned { kFArena = 1u, kFRows = 2u, kFNonfinite = 4u, kFNotPosdef = 8u, kFNonfiniteD = 16u,
                   kFMap = 32u, kFInternal = 64u, kFTcWait = 128u, kFTcCap = 256u, kFSteps = 512u,
                   kFAptpMiss = 1024u, kFInertia = 2048u, kFWork = 4096u, kFStatic = 8192u };
-// team reduction scratch per large front (2 buffers x 16 CTAs x 6 doubles)
-constexpr int kTeamRedDoubles = 256;
 // flags after which the rest of a factorization is skipped (retried with
 // more room, or reported)
 constexpr unsigned kFAbort = kFArena | kFRows | kFTcWait | kFTcCap | kFAptpMiss | kFInertia | kFWork | kFStatic;
@@ -741,12 +739,17 @@ __device__ __forceinline__ FrontRef large_view(DevPlan &P, DevFactor &X, int s) 
 
 __global__ void k_large_init(DevPlan P, DevFactor X, const int *__restrict__ large, int nlarge,
                              int posdef, int nbo) {
-  if (X.counters[kCFlags] & kFAbort) return;
-  const int s = large[blockIdx.x];
-  if (threadIdx.x == 0) {  // arrival counters of the front's team (both launch parities)
-    X.team_bar[2 * blockIdx.x] = 0u;
-    X.team_bar[2 * blockIdx.x + 1] = 0u;
+  if (X.counters[kCFlags] & kFAbort) {
+    // the pivoting kernel takes its decisions from the state alone: done
+    if (threadIdx.x == 0) {
+      TppState S;
+      tpp_init(S, 0, posdef != 0);
+      S.phase = 2;
+      X.tpp[blockIdx.x] = S;
+    }
+    return;
   }
+  const int s = large[blockIdx.x];
   const int f = X.sn_f[s];
   int *loc = X.ploc + X.sn_roff[s];
   int *inv = X.ploc + X.rows_cap + X.sn_roff[s];
@@ -845,14 +848,14 @@ __global__ void k_aptp_to_tpp(const aptp::Front *__restrict__ fr, const aptp::St
 // front is taken by a team of C CTAs launched as one thread-block cluster
 // (blockIdx.x / C = the front), the pivot decisions taken by every CTA of
 // the team alike and the swaps and panel eliminations split over it.
+// (No test of the abort flags here: a kernel beside this one may set one
+// while a team reads it, and the team's CTAs must agree; k_large_init closes
+// the fronts of an aborted factorization.)
 template <int NT, int C>
 __global__ void __launch_bounds__(NT) k_large_panel(DevPlan P, DevFactor X, const int *__restrict__ large,
-                                                    PivotParams prm, int iter, unsigned *__restrict__ team_bar) {
+                                                    PivotParams prm, int iter) {
   __shared__ FrontShared sh;
-  __shared__ int s_abort;
-  __shared__ unsigned s_bar_seq;
   __shared__ PairScratch s_pair;
-  if (X.counters[kCFlags] & kFAbort) return;
   const int q = blockIdx.x / C;
   const bool lead = team_rank<C>() == 0 && threadIdx.x == 0;
   const int s = large[q];
@@ -863,24 +866,14 @@ __global__ void __launch_bounds__(NT) k_large_panel(DevPlan P, DevFactor X, cons
   }
   prm.eff_small = __longlong_as_double((long long)X.counters[kCEffSmall]);
   FrontRef v = large_view(P, X, s);
-  // arrival counters: one per launch parity; this launch resets the other
-  // (the previous launch's, finished; the next launch's, not started)
-  v.team_bar = team_bar + 2 * q + (iter & 1);
-  if (lead) team_bar[2 * q + ((iter + 1) & 1)] = 0u;
-  v.err = X.counters + kCFlags;
-  v.abort = &s_abort;
-  v.bar_seq = &s_bar_seq;
   v.pair = &s_pair;
-  v.team_red = X.team_red + (size_t)q * kTeamRedDoubles;
   if (threadIdx.x == 0) {
     sh.st = S.st;
     sh.tr_seq = 0;
-    s_abort = 0;
-    s_bar_seq = 0;
   }
   __syncthreads();
   // every CTA has read the state before the leader may write it back
-  if constexpr (C > 1) team_sync<C>(v);
+  if constexpr (C > 1) team_sync<C>();
   const bool more = tpp_step_blk<NT, C>(v, prm, sh, S);
   __syncthreads();
   if (lead) {
