@@ -200,40 +200,36 @@ __global__ void __launch_bounds__(256) k_apply(const Front *__restrict__ fr, Sta
         }
       }
     }
-    // D^-1 and the check, pivot by pivot (every lane computes the values)
+    // D^-1 and the check, every lane its own columns (a 2x2 pivot's other
+    // column from the neighbouring lane); the first failing pivot is the
+    // lowest. (Pivot by pivot with broadcasts it was most of the kernel: 810
+    // us a launch on fronts of up to 6,800 rows.)
 #pragma unroll
     for (int q = 0; q < kRW; ++q) {
       const int rr = wid * kRW + q;
       int fl = ne_t;
-      for (int t = 0; t < ne_t; ++t) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sm.x[rr][lane + 32 * u] = x[q][u];
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int t = lane + 32 * u;
+        if (t >= ne_t) continue;
         const int8_t tg = tb[t];
-        double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (u == (t >> 5)) a0 = x[q][u];
-        a0 = __shfl_sync(0xffffffffu, a0, t & 31);
-        if (tg == 2) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (u == ((t + 1) >> 5)) a1 = x[q][u];
-          a1 = __shfl_sync(0xffffffffu, a1, (t + 1) & 31);
-          const double i00 = S.dinv[2 * t], i10 = S.dinv[2 * t + 1], i11 = S.dinv[2 * (t + 1)];
-          const double l0 = fma(i00, a0, __dmul_rn(i10, a1)), l1 = fma(i10, a0, __dmul_rn(i11, a1));
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            if (lane + 32 * u == t) x[q][u] = l0;
-            if (lane + 32 * u == t + 1) x[q][u] = l1;
-          }
-          if (fl == ne_t && (!l_ok(l0, inv_u) || !l_ok(l1, inv_u))) fl = t;
-          ++t;
+        const int p0 = tg == -1 ? t - 1 : t;  // the pivot's first column
+        double l;
+        if (tg == 2 || tg == -1) {
+          const double a0 = sm.x[rr][p0], a1 = sm.x[rr][p0 + 1];
+          const double i00 = S.dinv[2 * p0], i10 = S.dinv[2 * p0 + 1], i11 = S.dinv[2 * (p0 + 1)];
+          l = tg == 2 ? fma(i00, a0, __dmul_rn(i10, a1)) : fma(i10, a0, __dmul_rn(i11, a1));
         } else {
-          const double l = __dmul_rn(a0, S.dinv[2 * t]);
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (lane + 32 * u == t) x[q][u] = l;
-          if (fl == ne_t && !l_ok(l, inv_u)) fl = t;
+          l = __dmul_rn(x[q][u], S.dinv[2 * t]);
         }
+        x[q][u] = l;
+        if (!l_ok(l, inv_u)) fl = min(fl, p0);
       }
+      __syncwarp();
+      fl = (int)__reduce_min_sync(0xffffffffu, (unsigned)fl);
       if (rr < nr) fail = min(fail, fl);
     }
     // back to shared memory, then out (coalesced)

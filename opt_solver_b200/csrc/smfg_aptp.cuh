@@ -28,7 +28,11 @@
 namespace smfg {
 namespace aptp {
 
-constexpr int kTileNT = 256;
+// Threads of the tile kernel. One CTA factors a 256-column tile, its data in
+// L2: latency, so that more threads (loads in flight) help. 256 threads with
+// the search as a pass of its own took 2.0 ms a tile of which most columns
+// fail the inner sweep (see below for the measured time).
+constexpr int kTileNT = 512;
 
 __device__ __forceinline__ size_t ix(int j, int ld) { return (size_t)j * (size_t)ld; }
 
@@ -70,8 +74,8 @@ struct TileShared {
   int cp_lp[kNb];
   int itmp[kNb];
   double rv[32];
-  int ri[32], rj[32];
-  int kind, a, b, ok, nq1, nmin, nelim;
+  int ri[32];
+  int nq1, nmin;
 };
 
 // Symmetric transposition of view positions p < q (ldlt_aptp.cpp:67-80);
@@ -129,68 +133,43 @@ __device__ __forceinline__ double sym_at(const double *A, int ld, int i, int j) 
   return (i >= j) ? A[ix(j, ld) + i] : A[ix(i, ld) + j];
 }
 
-// Block-wide argmax of |A| over the lower triangle of rows / columns [k, n):
-// the first maximum in column-major order, NaNs never chosen
-// (ldlt_aptp.cpp:108-122).
-static __device__ void cta_argmax(const double *A, int ld, int n, int k, TileShared &sh, double &amax, int &bi, int &bj) {
-  double best = -1.0;
-  int bii = -1, bjj = -1;
-  // a warp per column, its lanes down the rows; every lane keeps its first
-  // maximum in (column, row) order
-  const int lane0 = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int j = k + (threadIdx.x >> 5); j < n; j += nw) {
-    const double *col = A + ix(j, ld);
-    for (int i = j + lane0; i < n; i += 32) {
-      const double v = fabs(col[i]);
-      if (v > best) {
-        best = v;
-        bii = i;
-        bjj = j;
-      }
+// A thread's share of an argmax of |A|: its first maximum in (column, row)
+// order, NaNs never chosen (ldlt_aptp.cpp:108-122).
+struct ArgMax {
+  double v = -1.0;
+  unsigned at = 0xffffffffu;  // column << 16 | row
+  __device__ __forceinline__ void add(double x, int i, int j) {
+    const double a = fabs(x);
+    if (a > v) {
+      v = a;
+      at = (unsigned)j << 16 | (unsigned)i;
     }
   }
-  // larger value wins; equal values: the lower column, then the lower row
-  auto better = [](double v1, int j1, int i1, double v2, int j2, int i2) {
-    if (v1 > v2) return true;
-    if (v1 < v2 || j1 < 0) return false;
-    if (j2 < 0) return true;
-    return j1 < j2 || (j1 == j2 && i1 < i2);
-  };
-  for (int o = 16; o > 0; o >>= 1) {
-    const double v2 = __shfl_down_sync(0xffffffffu, best, o);
-    const int i2 = __shfl_down_sync(0xffffffffu, bii, o);
-    const int j2 = __shfl_down_sync(0xffffffffu, bjj, o);
-    if (better(v2, j2, i2, best, bjj, bii)) {
-      best = v2;
-      bii = i2;
-      bjj = j2;
-    }
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+};
+
+// The larger value wins; of equal values the lower column, then the lower row.
+__device__ __forceinline__ void warp_argmax(double &v, unsigned &at) {
+  const double m = warp_max_bits(v >= 0.0 ? v : 0.0);
+  at = __reduce_min_sync(0xffffffffu, v == m ? at : 0xffffffffu);
+  v = at == 0xffffffffu ? -1.0 : m;
+}
+
+// The block's argmax; ends with every thread holding it (two barriers).
+static __device__ void cta_argmax(ArgMax t, TileShared &sh, double &amax, int &bi, int &bj) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  warp_argmax(t.v, t.at);
   if (lane == 0) {
-    sh.rv[wid] = best;
-    sh.ri[wid] = bii;
-    sh.rj[wid] = bjj;
+    sh.rv[wid] = t.v;
+    sh.ri[wid] = (int)t.at;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double bv = sh.rv[0];
-    int b_i = sh.ri[0], b_j = sh.rj[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      if (better(sh.rv[w], sh.rj[w], sh.ri[w], bv, b_j, b_i)) {
-        bv = sh.rv[w];
-        b_i = sh.ri[w];
-        b_j = sh.rj[w];
-      }
-    sh.rv[0] = bv;
-    sh.ri[0] = b_i;
-    sh.rj[0] = b_j;
-  }
+  double v = lane < nw ? sh.rv[lane] : -1.0;
+  unsigned at = lane < nw ? (unsigned)sh.ri[lane] : 0xffffffffu;
+  warp_argmax(v, at);
   __syncthreads();
-  amax = sh.rv[0];
-  bi = sh.ri[0];
-  bj = sh.rj[0];
-  __syncthreads();
+  amax = v;
+  bi = (int)(at & 0xffffu);
+  bj = (int)(at >> 16);
 }
 
 // Complete pivoting on an n x n view (ldlt_aptp.cpp:101-210); returns the
@@ -203,29 +182,29 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
   }
   __syncthreads();
   int k = 0;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // the largest entry of the view, then with each pivot's update that of what
+  // is left: a warp per column, its lanes down the rows, four in flight
+  ArgMax best;
+  for (int j = wid; j < n; j += nw)
+    for (int i = j + lane; i < n; i += 32) best.add(A[ix(j, ld) + i], i, j);
   while (k < n) {
     double amax;
     int bi, bj;
-    cta_argmax(A, ld, n, k, sh, amax, bi, bj);
+    cta_argmax(best, sh, amax, bi, bj);
     if (!(amax >= small) || !isfinite(amax)) break;
-    if (threadIdx.x == 0) {
-      int kind = 1, a = bj, b = -1;
-      if (bi != bj) {
-        const double amm = A[ix(bj, ld) + bj], att = A[ix(bi, ld) + bi], amt = A[ix(bj, ld) + bi];
-        const double delta = fma(amm, att, -__dmul_rn(amt, amt));
-        if (fabs(delta) >= __dmul_rn(__dmul_rn(0.5, amt), amt)) {
-          kind = 2;
-          b = bi;
-        } else {
-          a = (fabs(att) > fabs(amm)) ? bi : bj;
-        }
+    // every thread takes the decision
+    int kind = 1, a = bj, b = -1;
+    if (bi != bj) {
+      const double amm = A[ix(bj, ld) + bj], att = A[ix(bi, ld) + bi], amt = A[ix(bj, ld) + bi];
+      const double delta = fma(amm, att, -__dmul_rn(amt, amt));
+      if (fabs(delta) >= __dmul_rn(__dmul_rn(0.5, amt), amt)) {
+        kind = 2;
+        b = bi;
+      } else {
+        a = (fabs(att) > fabs(amm)) ? bi : bj;
       }
-      sh.kind = kind;
-      sh.a = a;
-      sh.b = b;
     }
-    __syncthreads();
-    const int kind = sh.kind, a = sh.a, b = sh.b;
     // a posteriori bound inside the view
     bool bad = false;
     if (kind == 1) {
@@ -249,11 +228,27 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
       const double inv_d = 1.0 / ck[k];
       // entries (i, j), k < j <= i < n: one fused step each (a warp per
       // column)
-      for (int jj = k + 1 + (threadIdx.x >> 5); jj < n; jj += (blockDim.x >> 5)) {
+      best = ArgMax{};
+      for (int jj = k + 1 + wid; jj < n; jj += nw) {
         const double lj = __dmul_rn(ck[jj], inv_d);
-        if (lj == 0.0) continue;
         double *cj = A + ix(jj, ld);
-        for (int ii = jj + (threadIdx.x & 31); ii < n; ii += 32) cj[ii] = fma(-ck[ii], lj, cj[ii]);
+        for (int i0 = jj + lane; i0 < n; i0 += 4 * 32) {
+          double x[4], y[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            x[u] = i0 + 32 * u < n ? cj[i0 + 32 * u] : 0.0;
+            y[u] = i0 + 32 * u < n ? ck[i0 + 32 * u] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (i0 + 32 * u < n) {
+              if (lj != 0.0) {
+                x[u] = fma(-y[u], lj, x[u]);
+                cj[i0 + 32 * u] = x[u];
+              }
+              best.add(x[u], i0 + 32 * u, jj);
+            }
+        }
       }
       __syncthreads();
       double *ckw = A + ix(k, ld);
@@ -271,13 +266,30 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
       double *c0 = A + ix(k, ld), *c1 = A + ix(k + 1, ld);
       double i00, i10, i11;
       inv2(c0[k], c0[k + 1], c1[k + 1], i00, i10, i11);
-      for (int jj = k + 2 + (threadIdx.x >> 5); jj < n; jj += (blockDim.x >> 5)) {
+      best = ArgMax{};
+      for (int jj = k + 2 + wid; jj < n; jj += nw) {
         const double a0 = c0[jj], a1 = c1[jj];
         const double l0 = fma(i00, a0, __dmul_rn(i10, a1)), l1 = fma(i10, a0, __dmul_rn(i11, a1));
-        if (l0 == 0.0 && l1 == 0.0) continue;
+        const bool upd = !(l0 == 0.0 && l1 == 0.0);
         double *cj = A + ix(jj, ld);
-        for (int ii = jj + (threadIdx.x & 31); ii < n; ii += 32)
-          cj[ii] = __dsub_rn(cj[ii], fma(c0[ii], l0, __dmul_rn(c1[ii], l1)));
+        for (int i0 = jj + lane; i0 < n; i0 += 4 * 32) {
+          double x[4], y0[4], y1[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            x[u] = i0 + 32 * u < n ? cj[i0 + 32 * u] : 0.0;
+            y0[u] = i0 + 32 * u < n ? c0[i0 + 32 * u] : 0.0;
+            y1[u] = i0 + 32 * u < n ? c1[i0 + 32 * u] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (i0 + 32 * u < n) {
+              if (upd) {
+                x[u] = __dsub_rn(x[u], fma(y0[u], l0, __dmul_rn(y1[u], l1)));
+                cj[i0 + 32 * u] = x[u];
+              }
+              best.add(x[u], i0 + 32 * u, jj);
+            }
+        }
       }
       __syncthreads();
       for (int i = k + 2 + threadIdx.x; i < n; i += blockDim.x) {
