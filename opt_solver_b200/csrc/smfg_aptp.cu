@@ -165,37 +165,34 @@ __global__ void __launch_bounds__(256) k_apply(const Front *__restrict__ fr, Sta
         const int j = lane + 32 * u;
         if (j < ne_t) x[q][u] = sm.x[wid * kRW + q][j];
       }
-    for (int p0 = 0; p0 < ne_t; p0 += 32) {
+    // (unrolled over the 32-column groups: the rows' registers by constant
+    // index, only the groups still to come updated)
+#pragma unroll
+    for (int up = 0; up < 8; ++up) {
+      const int p0 = 32 * up;
+      if (p0 >= ne_t) break;
       __syncthreads();
-      for (int e = threadIdx.x; e < 32 * ne_t; e += blockDim.x) {
-        const int pp = e / ne_t, j = e % ne_t, p = p0 + pp;
-        double l = 0.0;
-        if (p < ne_t && j > p && !(tb[p] == 2 && j == p + 1)) l = T[ix(p, F.f) + j];
-        sm.L[pp][j] = l;
+      for (int pp = wid; pp < 32; pp += 8) {
+        const int p = p0 + pp;
+        const bool pair = p < ne_t && tb[p] == 2;
+        for (int j = p0 + lane; j < ne_t; j += 32)
+          sm.L[pp][j] = (p < ne_t && j > p && !(pair && j == p + 1)) ? T[ix(p, F.f) + j] : 0.0;
       }
       __syncthreads();
       const int pend = min(32, ne_t - p0);
       for (int pp = 0; pp < pend; ++pp) {
-        const int p = p0 + pp;
-        const int up = p >> 5;
         double xp[kRW];
 #pragma unroll
-        for (int q = 0; q < kRW; ++q) {
-          double v = 0.0;
+        for (int q = 0; q < kRW; ++q) xp[q] = __shfl_sync(0xffffffffu, x[q][up], pp);
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (u == up) v = x[q][u];
-          xp[q] = __shfl_sync(0xffffffffu, v, p & 31);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = up; u < 8; ++u) {
           const int j = lane + 32 * u;
-          if (j > p && j < ne_t) {
-            const double l = sm.L[pp][j];
-            if (l != 0.0) {
+          // (zero at and above the diagonal, and past the tile's pivots)
+          const double l = j < ne_t ? sm.L[pp][j] : 0.0;
 #pragma unroll
-              for (int q = 0; q < kRW; ++q) x[q][u] = fma(-xp[q], l, x[q][u]);
-            }
+          for (int q = 0; q < kRW; ++q) {
+            const double y = fma(-xp[q], l, x[q][u]);
+            x[q][u] = l != 0.0 ? y : x[q][u];
           }
         }
       }

@@ -28,10 +28,8 @@
 namespace smfg {
 namespace aptp {
 
-// Threads of the tile kernel. One CTA factors a 256-column tile, its data in
-// L2: latency, so that more threads (loads in flight) help. 256 threads with
-// the search as a pass of its own took 2.0 ms a tile of which most columns
-// fail the inner sweep (see below for the measured time).
+// Threads of the tile kernel: one CTA factors a 256-column tile, a chain of
+// pivots; 1,024 threads would spill its rows' solves.
 constexpr int kTileNT = 512;
 
 __device__ __forceinline__ size_t ix(int j, int ld) { return (size_t)j * (size_t)ld; }
@@ -66,8 +64,22 @@ __device__ __forceinline__ double ld_of(const double *T, int ld, const int8_t *t
 // CTA-level pieces of the diagonal tile's factorization (one CTA of
 // kTileNT threads per tile; the tile lives in global memory / L2).
 
+// Complete pivoting runs on a copy of its view in shared memory (the lower
+// triangle packed by columns) when it has at most this many columns: the
+// inner blocks, and the tile's failed columns at the end of its sweep.
+constexpr int kPackCols = 224;
+constexpr int kPackDoubles = kPackCols * (kPackCols + 1) / 2;
+
 struct TileShared {
-  double bk1[kNb * kIb];   // inner block backup: column t at bk1 + t * kNb (tile rows)
+  // the inner block's backup (column t at bk1 + t * kNb, tile rows) and its
+  // packed view; at the end of the sweep one packed view over both
+  union {
+    struct {
+      double bk1[kNb * kIb];
+      double pk1[kIb * (kIb + 1) / 2];
+    };
+    double pk[kPackDoubles];
+  };
   double dinv1[2 * kIb];
   int q1[kNb];
   int lpc1[kIb];
@@ -78,9 +90,23 @@ struct TileShared {
   int nq1, nmin;
 };
 
+// A view of a symmetric block by columns of its lower triangle: entry (i, j)
+// at col(j)[i]. In place (leading dimension ld), or packed.
+struct FullView {
+  double *A;
+  int ld;
+  __device__ __forceinline__ double *col(int j) const { return A + ix(j, ld); }
+};
+struct PackView {
+  double *A;
+  int n;
+  __device__ __forceinline__ double *col(int j) const { return A + j * (2 * n - j - 1) / 2; }
+};
+
 // Symmetric transposition of view positions p < q (ldlt_aptp.cpp:67-80);
 // tags, rows, lp and loc follow. Callers synchronize before.
-static __device__ void cta_swap(double *A, int ld, int m, int p, int q, int8_t *tags, int *rows, int *lp, int *loc) {
+template <typename View>
+static __device__ void cta_swap(const View &V, int m, int p, int q, int8_t *tags, int *rows, int *lp, int *loc) {
   if (p == q) return;
   if (p > q) {
     const int t = p;
@@ -89,26 +115,26 @@ static __device__ void cta_swap(double *A, int ld, int m, int p, int q, int8_t *
   }
   const int items = m - 1;  // p diag pair + (c < p) + (p < c < q) + (r > q)
   for (int t = threadIdx.x; t < items; t += blockDim.x) {
-    size_t e1, e2;
+    double *e1, *e2;
     if (t == 0) {
-      e1 = ix(p, ld) + p;
-      e2 = ix(q, ld) + q;
+      e1 = V.col(p) + p;
+      e2 = V.col(q) + q;
     } else if (t <= p) {
       const int c = t - 1;
-      e1 = ix(c, ld) + p;
-      e2 = ix(c, ld) + q;
+      e1 = V.col(c) + p;
+      e2 = V.col(c) + q;
     } else if (t < q) {
       const int c = t;  // p < c < q
-      e1 = ix(p, ld) + c;
-      e2 = ix(c, ld) + q;
+      e1 = V.col(p) + c;
+      e2 = V.col(c) + q;
     } else {
       const int r = t + 1;  // r > q
-      e1 = ix(p, ld) + r;
-      e2 = ix(q, ld) + r;
+      e1 = V.col(p) + r;
+      e2 = V.col(q) + r;
     }
-    const double x = A[e1];
-    A[e1] = A[e2];
-    A[e2] = x;
+    const double x = *e1;
+    *e1 = *e2;
+    *e2 = x;
   }
   if (threadIdx.x == 0) {
     const int8_t tg = tags[p];
@@ -129,8 +155,9 @@ static __device__ void cta_swap(double *A, int ld, int m, int p, int q, int8_t *
   __syncthreads();
 }
 
-__device__ __forceinline__ double sym_at(const double *A, int ld, int i, int j) {
-  return (i >= j) ? A[ix(j, ld) + i] : A[ix(i, ld) + j];
+template <typename View>
+__device__ __forceinline__ double sym_at(const View &V, int i, int j) {
+  return (i >= j) ? V.col(j)[i] : V.col(i)[j];
 }
 
 // A thread's share of an argmax of |A|: its first maximum in (column, row)
@@ -174,8 +201,9 @@ static __device__ void cta_argmax(ArgMax t, TileShared &sh, double &amax, int &b
 
 // Complete pivoting on an n x n view (ldlt_aptp.cpp:101-210); returns the
 // pivots taken. lp: the view's permutation record.
-static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *rows, int *lp, int *loc, double inv_u,
-                            double small, TileShared &sh) {
+template <typename View>
+static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *rows, int *lp, int *loc, double inv_u,
+                                      double small, TileShared &sh) {
   for (int t = threadIdx.x; t < n; t += blockDim.x) {
     lp[t] = t;
     tags[t] = 0;
@@ -187,7 +215,7 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
   // is left: a warp per column, its lanes down the rows, four in flight
   ArgMax best;
   for (int j = wid; j < n; j += nw)
-    for (int i = j + lane; i < n; i += 32) best.add(A[ix(j, ld) + i], i, j);
+    for (int i = j + lane; i < n; i += 32) best.add(V.col(j)[i], i, j);
   while (k < n) {
     double amax;
     int bi, bj;
@@ -196,7 +224,7 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
     // every thread takes the decision
     int kind = 1, a = bj, b = -1;
     if (bi != bj) {
-      const double amm = A[ix(bj, ld) + bj], att = A[ix(bi, ld) + bi], amt = A[ix(bj, ld) + bi];
+      const double amm = V.col(bj)[bj], att = V.col(bi)[bi], amt = V.col(bj)[bi];
       const double delta = fma(amm, att, -__dmul_rn(amt, amt));
       if (fabs(delta) >= __dmul_rn(__dmul_rn(0.5, amt), amt)) {
         kind = 2;
@@ -208,30 +236,30 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
     // a posteriori bound inside the view
     bool bad = false;
     if (kind == 1) {
-      const double lim = __dmul_rn(inv_u, fabs(A[ix(a, ld) + a]));
+      const double lim = __dmul_rn(inv_u, fabs(V.col(a)[a]));
       for (int r = k + threadIdx.x; r < n; r += blockDim.x)
-        if (r != a && !(fabs(sym_at(A, ld, r, a)) <= lim)) bad = true;
+        if (r != a && !(fabs(sym_at(V, r, a)) <= lim)) bad = true;
     } else {
       double i00, i10, i11;
-      inv2(A[ix(a, ld) + a], A[ix(a, ld) + b], A[ix(b, ld) + b], i00, i10, i11);
+      inv2(V.col(a)[a], V.col(a)[b], V.col(b)[b], i00, i10, i11);
       for (int r = k + threadIdx.x; r < n; r += blockDim.x) {
         if (r == a || r == b) continue;
-        const double x0 = sym_at(A, ld, r, a), x1 = sym_at(A, ld, r, b);
+        const double x0 = sym_at(V, r, a), x1 = sym_at(V, r, b);
         if (!l_ok(fma(i00, x0, __dmul_rn(i10, x1)), inv_u) || !l_ok(fma(i10, x0, __dmul_rn(i11, x1)), inv_u))
           bad = true;
       }
     }
     if (__syncthreads_or(bad)) break;
     if (kind == 1) {
-      cta_swap(A, ld, n, k, a, tags, rows, lp, loc);
-      const double *ck = A + ix(k, ld);
+      cta_swap(V, n, k, a, tags, rows, lp, loc);
+      const double *ck = V.col(k);
       const double inv_d = 1.0 / ck[k];
       // entries (i, j), k < j <= i < n: one fused step each (a warp per
       // column)
       best = ArgMax{};
       for (int jj = k + 1 + wid; jj < n; jj += nw) {
         const double lj = __dmul_rn(ck[jj], inv_d);
-        double *cj = A + ix(jj, ld);
+        double *cj = V.col(jj);
         for (int i0 = jj + lane; i0 < n; i0 += 4 * 32) {
           double x[4], y[4];
 #pragma unroll
@@ -251,7 +279,7 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
         }
       }
       __syncthreads();
-      double *ckw = A + ix(k, ld);
+      double *ckw = V.col(k);
       for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) ckw[i] = __dmul_rn(ckw[i], inv_d);
       if (threadIdx.x == 0) tags[k] = 1;
       __syncthreads();
@@ -259,11 +287,11 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
     } else {
       int partner = b;
       if (a != k) {
-        cta_swap(A, ld, n, k, a, tags, rows, lp, loc);
+        cta_swap(V, n, k, a, tags, rows, lp, loc);
         if (partner == k) partner = a;
       }
-      if (partner != k + 1) cta_swap(A, ld, n, k + 1, partner, tags, rows, lp, loc);
-      double *c0 = A + ix(k, ld), *c1 = A + ix(k + 1, ld);
+      if (partner != k + 1) cta_swap(V, n, k + 1, partner, tags, rows, lp, loc);
+      double *c0 = V.col(k), *c1 = V.col(k + 1);
       double i00, i10, i11;
       inv2(c0[k], c0[k + 1], c1[k + 1], i00, i10, i11);
       best = ArgMax{};
@@ -271,7 +299,7 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
         const double a0 = c0[jj], a1 = c1[jj];
         const double l0 = fma(i00, a0, __dmul_rn(i10, a1)), l1 = fma(i10, a0, __dmul_rn(i11, a1));
         const bool upd = !(l0 == 0.0 && l1 == 0.0);
-        double *cj = A + ix(jj, ld);
+        double *cj = V.col(jj);
         for (int i0 = jj + lane; i0 < n; i0 += 4 * 32) {
           double x[4], y0[4], y1[4];
 #pragma unroll
@@ -307,6 +335,26 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
   }
   __syncthreads();
   return k;
+}
+
+// The same in place at A (leading dimension ld), through a packed copy at pk
+// when there is one: a pivot's pass over the view is then bound by its
+// barriers, not by L2's latency.
+static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *rows, int *lp, int *loc, double inv_u,
+                                   double small, TileShared &sh, double *pk) {
+  const FullView G{A, ld};
+  if (!pk) return cta_complete_on(G, n, tags, rows, lp, loc, inv_u, small, sh);
+  const PackView S{pk, n};
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  __syncthreads();
+  for (int j = threadIdx.x >> 5; j < n; j += nw)
+    for (int i = j + lane; i < n; i += 32) S.col(j)[i] = G.col(j)[i];
+  __syncthreads();
+  const int p = cta_complete_on(S, n, tags, rows, lp, loc, inv_u, small, sh);
+  for (int j = threadIdx.x >> 5; j < n; j += nw)
+    for (int i = j + lane; i < n; i += 32) G.col(j)[i] = S.col(j)[i];
+  __syncthreads();
+  return p;
 }
 
 // Rows [r0, r0 + w) of columns [0, ncols): new row r0 + t takes old row
@@ -381,7 +429,7 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
   __syncthreads();
   // 2. complete pivoting on the diagonal block
   const int ne_t = cta_complete(T + ix(c0, ld) + c0, ld, w1, tags + c0, rows + c0, sh.lpc1, loc ? loc + c0 : nullptr,
-                                inv_u, small, sh);
+                                inv_u, small, sh, sh.pk1);
   // 3. its permutation on the rest of the tile
   if (!cta_identity(sh.lpc1, w1)) {
     cta_permute_rows(T, ld, c0, c0, w1, sh.lpc1);
@@ -496,27 +544,45 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
     }
     // UpdateNT / TN: the earlier failed columns, tile rows [e0, w) and their
     // block among themselves; each entry one chain from zero, then one
-    // subtraction
-    for (int jq = 0; jq < nq; ++jq) {
-      const int qj = sh.q1[jq];
-      const double *lq = T + ix(qj, ld) + c0;  // the column's L row for the pivots
-      for (int r = e0 + threadIdx.x; r < w; r += blockDim.x) {
-        double acc = 0.0;
+    // subtraction. (L D) of the failed columns' rows first, into bk1 (the
+    // backup is done with): formed per entry it was most of the kernel, 2.0
+    // of 2.4 ms a tile with 200 failed columns. A warp takes four columns,
+    // lanes the rows.
+    double(*ldq)[kIb] = reinterpret_cast<double(*)[kIb]>(sh.bk1);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nq * nelim; e += blockDim.x) {
+      const int jq = e / nelim, p = e % nelim;
+      const double *lq = T + ix(sh.q1[jq], ld) + c0;
+      ldq[jq][p] = (tb[p] == -1) ? ld_of(Tb, ld, tb, p, lq[p - 1], lq[p])
+                                 : ld_of(Tb, ld, tb, p, lq[p], tb[p] == 2 ? lq[p + 1] : 0.0);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int j0 = 4 * wid; j0 < nq; j0 += 4 * nw) {
+      const int nj = min(4, nq - j0);
+      // rows [e0, w) of the tile, then the failed columns' rows from j0 on
+      const int nr = w - e0;
+      for (int t = lane; t < nr + nq - j0; t += 32) {
+        const bool in = t < nr;
+        const int r = in ? e0 + t : sh.q1[j0 + t - nr];
+        const double *row = in ? T + ix(c0, ld) + r : T + ix(r, ld) + c0;
+        const size_t stride = in ? (size_t)ld : 1;
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
         for (int p = 0; p < nelim; ++p) {
-          const double bw = (tb[p] == -1) ? ld_of(Tb, ld, tb, p, lq[p - 1], lq[p]) : ld_of(Tb, ld, tb, p, lq[p], tb[p] == 2 ? lq[p + 1] : 0.0);
-          if (bw != 0.0) acc = fma(T[ix(c0 + p, ld) + r], bw, acc);
+          const double l = row[p * stride];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const double bw = u < nj ? ldq[j0 + u][p] : 0.0;
+            const double y = fma(l, bw, acc[u]);
+            acc[u] = bw != 0.0 ? y : acc[u];
+          }
         }
-        T[ix(qj, ld) + r] = __dsub_rn(T[ix(qj, ld) + r], acc);
-      }
-      for (int iq = jq + threadIdx.x; iq < nq; iq += blockDim.x) {
-        const int qi = sh.q1[iq];
-        const double *li = T + ix(qi, ld) + c0;
-        double acc = 0.0;
-        for (int p = 0; p < nelim; ++p) {
-          const double bw = (tb[p] == -1) ? ld_of(Tb, ld, tb, p, lq[p - 1], lq[p]) : ld_of(Tb, ld, tb, p, lq[p], tb[p] == 2 ? lq[p + 1] : 0.0);
-          if (bw != 0.0) acc = fma(li[p], bw, acc);
-        }
-        T[ix(qj, ld) + qi] = __dsub_rn(T[ix(qj, ld) + qi], acc);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < nj && (in || t - nr >= u)) {  // (of the failed block its lower part)
+            double *c = T + ix(sh.q1[j0 + u], ld) + r;
+            *c = __dsub_rn(*c, acc[u]);
+          }
       }
     }
   }
@@ -534,7 +600,7 @@ static __device__ void cta_compact(double *A, int ld, int m, int ne, int8_t *tag
   int dst = 0;
   for (int src = 0; src < ne; ++src) {
     if (tags[src] == 0) continue;
-    if (src != dst) cta_swap(A, ld, m, dst, src, tags, rows, lp, loc);
+    if (src != dst) cta_swap(FullView{A, ld}, m, dst, src, tags, rows, lp, loc);
     ++dst;
   }
   __syncthreads();
@@ -545,7 +611,7 @@ static __device__ void cta_compact(double *A, int ld, int m, int ne, int8_t *tag
 // permutation record. Returns the tile's pivots.
 static __device__ int tile_factor(double *T, int ld, int w, int8_t *tags, int *rows, int *lp, int *loc, double inv_u,
                            double small, TileShared &sh) {
-  if (w <= kIb) return cta_complete(T, ld, w, tags, rows, lp, loc, inv_u, small, sh);
+  if (w <= kIb) return cta_complete(T, ld, w, tags, rows, lp, loc, inv_u, small, sh, sh.pk1);
   for (int t = threadIdx.x; t < w; t += blockDim.x) {
     lp[t] = t;
     tags[t] = 0;
@@ -559,7 +625,7 @@ static __device__ int tile_factor(double *T, int ld, int w, int8_t *tags, int *r
   if (ne1 < w) {
     const int n2 = w - ne1;
     const int ne2 = cta_complete(T + ix(ne1, ld) + ne1, ld, n2, tags + ne1, rows + ne1, sh.cp_lp,
-                                 loc ? loc + ne1 : nullptr, inv_u, small, sh);
+                                 loc ? loc + ne1 : nullptr, inv_u, small, sh, n2 <= kPackCols ? sh.pk : nullptr);
     if (!cta_identity(sh.cp_lp, n2)) {
       cta_permute_rows(T, ld, ne1, ne1, n2, sh.cp_lp);
       if ((int)threadIdx.x < n2) sh.itmp[threadIdx.x] = lp[ne1 + sh.cp_lp[threadIdx.x]];

@@ -1055,7 +1055,8 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
         if (lvl_mixed) enqueue_tc(pl, mc, lg, nL, x.tpp, c.posdef, lc, gp);
       }
       gp.mark(st, 3);
-      k_large_schur<<<ggrid, 256, sizeof(TileSmem), st>>>(d, x, lg, nL, fin);
+      if (c.posdef) k_large_schur<true><<<ggrid, 256, sizeof(TileSmem), st>>>(d, x, lg, nL, fin);
+      else k_large_schur<false><<<ggrid, 256, sizeof(TileSmem), st>>>(d, x, lg, nL, fin);
       gp.mark(st, 3);
       k_large_finish<512><<<nL, 512, 0, st>>>(d, x, lg, fin, prm);
       k_large_store<<<ggrid, 256, 0, st>>>(d, x, lg, nL, c.posdef);
@@ -1095,7 +1096,8 @@ static void set_kernel_attrs(int nb) {
                                  (int)sizeof(tc::Smem)));
   SMFG_CUDA(cudaFuncSetAttribute(tc::k_tc_syrk<tc::kBF16x3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(tc::Smem)));
-  SMFG_CUDA(cudaFuncSetAttribute(k_large_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
+  for (auto kern : {k_large_schur<true>, k_large_schur<false>})
+    SMFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem)));
   done_nb = nb;
 }
 

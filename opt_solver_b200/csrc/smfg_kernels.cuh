@@ -896,6 +896,31 @@ __global__ void __launch_bounds__(NT) k_large_panel(DevPlan P, DevFactor X, cons
   }
 }
 
+// pref[q + 1] = counts of items 0..q of a launch's fronts (pref[0] = 0), one
+// front a thread: count(q) by threads q < cnt <= NT, a block scan; ends at a
+// barrier. (One thread adding them up waited for each front's loads in turn:
+// 100 us and more a launch on a level of a few hundred fronts.)
+template <int NT, typename Count>
+__device__ __forceinline__ void front_prefix(int cnt, int *pref, Count count) {
+  __shared__ int wsum[NT / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __syncthreads();  // the chunk before is done with pref
+  int v = tid < cnt ? count(tid) : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
+  }
+  if (lane == 31) wsum[warp] = v;
+  __syncthreads();
+  int base = 0;
+  for (int w = 0; w < warp; ++w) base += wsum[w];
+  if (tid < cnt) pref[tid + 1] = base + v;
+  if (tid == 0) pref[0] = 0;
+  __syncthreads();
+}
+constexpr int kFrontChunk = 256;  // fronts a chunk (a thread each)
+
 // Work items of a level's tiled GEMMs: each large front contributes tiles of
 // kGT x kGT over a lower-trapezoidal region [r0, f) x [r0, c1) with tile
 // (ti, tj) needed when ti >= tj.
@@ -931,118 +956,166 @@ __device__ __forceinline__ double ld_entry_g(const double *F, size_t sf, const i
 
 // One 128 x 64 tile of C -= A B^T (lower part: i >= j, i < rmax, j < cmax)
 // over K = kk pivots in order: A(i, p) = F(i, a0 + p); B(j, p) = W(j, p)
-// (deferred update) or (L D)(j, a0 + p) (Schur update). 256 threads, 8 x 4
-// entries each, K in chunks of 16 staged in shared memory with the next
-// chunk prefetched in registers. Every entry takes one fused multiply-add
-// per pivot in pivot order, a zero B(j, p) skipped, as the reference's
-// GEMM loops do.
+// (deferred update) or (L D)(j, a0 + p) (Schur update). 8 warps of 32 x 32
+// entries each, K in chunks of 16 staged in shared memory with the next chunk
+// prefetched in registers. Every entry takes one fused multiply-add per pivot
+// in pivot order, a zero B(j, p) skipped, as the reference's GEMM loops do.
+//
+// The multiply-adds are FP64 matrix instructions (mma.m8n8k4): on this GPU
+// they round as a chain of fused multiply-adds over k in ascending order
+// (tests/test_front_classes.py checks it against such chains), so the result
+// is the scalar loop's bit for bit; they take one operand load per 8
+// multiply-adds in place of 3 (the scalar loop, bound by its shared-memory
+// reads and by waiting for a chunk's loads before the one before it was used,
+// ran at 12 TFLOP/s of the 33 the FP64 units give). A skipped update and a
+// product with zero agree unless the sum is -0 or A is not finite: a warp that
+// meets either in a chunk with a zero B entry takes that chunk in scalar steps
+// (a sum that underflows to -0 inside the chunk may keep the other sign of
+// zero). A is negated as it is read; the padding of a last chunk is -0 x 0,
+// which leaves every sum as it is.
 constexpr int kTM = 128, kTN = 64, kTK = 16;
+constexpr int kTAS = kTM + 4, kTBS = kTN + 4;  // row strides: the fragments' reads hit distinct banks
 
 struct TileSmem {
-  double A[2][kTK][kTM];
-  double B[2][kTK][kTN];
+  double A[2][kTK][kTAS];
+  double B[2][kTK][kTBS];
 };
 
-template <bool SCHUR>
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// KIND 0: B = W; 1: B = (L D) with the pivots' tags; 2: B = L D, every pivot
+// 1 x 1 (SPD).
+template <int KIND>
 __device__ __forceinline__ void tile_update(double *F, size_t sf, const double *W, int wld, const int8_t *tags,
                                             int i0, int j0, int rmax, int cmax, int a0, int kk, TileSmem &sm) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double c[8][4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t4 = lane & 3;  // fragment coordinates
+  const int wr = 32 * (warp & 3), wc = 32 * (warp >> 2);
+  // fragment (mi, ni): rows wr + 8 mi + g, columns wc + 8 ni + 2 t4 + e
+  double c[4][4][2];
 #pragma unroll
-  for (int r = 0; r < 8; ++r)
+  for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * q;
-      c[r][q] = (i < rmax && j < cmax && i >= j) ? F[(size_t)j * sf + i] : 0.0;
-    }
-  double pa[8], pb[4];
-  int zb = 0;  // a zero among the fetched chunk's B values (a skipped update)
-  auto fetch = [&](int k0) {
-    zb = 0;
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int i = i0 + wr + 8 * mi + g, j = j0 + wc + 8 * ni + 2 * t4 + e;
+        c[mi][ni][e] = (i < rmax && j < cmax && i >= j) ? F[(size_t)j * sf + i] : 0.0;
+      }
+  // (a warp wholly above the diagonal or past the edge has nothing to do)
+  const bool idle = i0 + wr + 31 < j0 + wc || i0 + wr >= rmax || j0 + wc >= cmax;
+  double pb[4], pd[4];
+  // chunk k0: A copied asynchronously (zero past its edges), B's factors into
+  // registers; nothing here waits for a load
+  auto fetch = [&](int k0, int buf) {
     const int kc = min(kTK, kk - k0);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const int t = threadIdx.x + 256 * u;
-      const int p = t / kTM, r = t % kTM;
-      pa[u] = (p < kc && i0 + r < rmax) ? F[(size_t)(a0 + k0 + p) * sf + i0 + r] : 0.0;
+      const int p = (threadIdx.x >> 7) + 2 * u, r = threadIdx.x & 127;
+      const bool in = p < kc && i0 + r < rmax;
+      const double *src = in ? F + (size_t)(a0 + k0 + p) * sf + i0 + r : F;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(&sm.A[buf][p][r]);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(in ? 8 : 0) : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int t = threadIdx.x + 256 * u;
-      const int p = t / kTN, r = t % kTN;
-      double bv = 0.0;
-      if (p < kc && j0 + r < cmax) {
-        if (SCHUR) bv = ld_entry_g(F, sf, tags, a0 + k0 + p, j0 + r);
-        else bv = W[(size_t)(k0 + p) * wld + j0 + r];
-        zb |= bv == 0.0 ? 1 : 0;
+      const int p = (threadIdx.x >> 6) + 4 * u, j = j0 + (int)(threadIdx.x & 63), c = a0 + k0 + p;
+      const bool in = p < kc && j < cmax;
+      if (KIND == 0) pb[u] = in ? W[(size_t)(k0 + p) * wld + j] : 0.0;
+      else if (KIND == 1) pb[u] = in ? ld_entry_g(F, sf, tags, c, j) : 0.0;
+      else {
+        pb[u] = in ? F[(size_t)c * sf + j] : 0.0;
+        pd[u] = in ? F[(size_t)c * sf + c] : 0.0;
       }
-      pb[u] = bv;
     }
   };
-  auto stash = [&](int buf) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int t = threadIdx.x + 256 * u;
-      sm.A[buf][t / kTM][t % kTM] = pa[u];
-    }
+  // B of the fetched chunk into buffer buf; whether a real one is zero (the
+  // padding's zeros only reach entries that are not stored)
+  auto stash = [&](int k0, int buf) {
+    const int kc = min(kTK, kk - k0);
+    int zb = 0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int t = threadIdx.x + 256 * u;
-      sm.B[buf][t / kTN][t % kTN] = pb[u];
+      const int p = (threadIdx.x >> 6) + 4 * u, r = threadIdx.x & 63;
+      const double b = KIND == 2 ? __dmul_rn(pb[u], pd[u]) : pb[u];
+      sm.B[buf][p][r] = b;
+      zb |= (b == 0.0 && p < kc && j0 + r < cmax) ? 1 : 0;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return zb;
   };
   int buf = 0;
-  fetch(0);
-  __syncthreads();
-  stash(0);
-  // whether the chunk in sm has a zero B value: without one every update
-  // applies and the loop takes no tests (the padding's zeros only reach
-  // entries that are not stored)
-  int anyz = __syncthreads_or(zb);
+  fetch(0, 0);
+  int anyz = __syncthreads_or(stash(0, 0));
   for (int k0 = 0; k0 < kk; k0 += kTK) {
     const int kc = min(kTK, kk - k0);
-    if (k0 + kTK < kk) fetch(k0 + kTK);
-    if (!anyz) {
-      for (int p = 0; p < kc; ++p) {
-        double av[8], bv[4];
+    if (k0 + kTK < kk) fetch(k0 + kTK, buf ^ 1);
+    bool scalar = false;
+    if (anyz && !idle) {
+      // a skipped update matters where the sum is -0 or A is not finite
 #pragma unroll
-        for (int r = 0; r < 8; ++r) av[r] = sm.A[buf][p][tx + 16 * r];
+      for (int mi = 0; mi < 4; ++mi) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) bv[q] = sm.B[buf][p][ty + 16 * q];
+        for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+          for (int e = 0; e < 2; ++e)
+            scalar = scalar || __double_as_longlong(c[mi][ni][e]) == (long long)0x8000000000000000ull;
 #pragma unroll
-          for (int r = 0; r < 8; ++r) c[r][q] = fma(-av[r], bv[q], c[r][q]);
+        for (int p4 = 0; p4 < kTK; p4 += 4) scalar = scalar || !isfinite(sm.A[buf][p4 + t4][wr + 8 * mi + g]);
+      }
+      scalar = __any_sync(0xffffffffu, scalar);
+    }
+    if (idle) {
+    } else if (!scalar) {
+#pragma unroll
+      for (int p4 = 0; p4 < kTK; p4 += 4) {
+        double av[4], bv[4];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi) av[mi] = -sm.A[buf][p4 + t4][wr + 8 * mi + g];
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) bv[ni] = sm.B[buf][p4 + t4][wc + 8 * ni + g];
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+          for (int ni = 0; ni < 4; ++ni) dmma884(c[mi][ni], av[mi], bv[ni]);
       }
     } else {
       for (int p = 0; p < kc; ++p) {
-        double av[8], bv[4];
+        double av[4];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) av[r] = sm.A[buf][p][tx + 16 * r];
+        for (int mi = 0; mi < 4; ++mi) av[mi] = -sm.A[buf][p][wr + 8 * mi + g];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) bv[q] = sm.B[buf][p][ty + 16 * q];
+        for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (bv[q] != 0.0) {
+          for (int e = 0; e < 2; ++e) {
+            const double bv = sm.B[buf][p][wc + 8 * ni + 2 * t4 + e];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) c[r][q] = fma(-av[r], bv[q], c[r][q]);
+            for (int mi = 0; mi < 4; ++mi) {
+              const double x = fma(av[mi], bv, c[mi][ni][e]);
+              c[mi][ni][e] = bv != 0.0 ? x : c[mi][ni][e];
+            }
           }
-        }
       }
     }
     if (k0 + kTK < kk) {
-      stash(buf ^ 1);
-      anyz = __syncthreads_or(zb);
+      anyz = __syncthreads_or(stash(k0 + kTK, buf ^ 1));
       buf ^= 1;
     }
   }
 #pragma unroll
-  for (int r = 0; r < 8; ++r)
+  for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * q;
-      if (i < rmax && j < cmax && i >= j) F[(size_t)j * sf + i] = c[r][q];
-    }
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int i = i0 + wr + 8 * mi + g, j = j0 + wc + 8 * ni + 2 * t4 + e;
+        if (i < rmax && j < cmax && i >= j) F[(size_t)j * sf + i] = c[mi][ni][e];
+      }
   __syncthreads();
 }
 
@@ -1078,22 +1151,15 @@ __global__ void __launch_bounds__(256) k_large_gemm(DevPlan P, DevFactor X, cons
                                                     int nlarge, const TppState *__restrict__ tpp) {
   extern __shared__ __align__(16) double dsm_g[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(dsm_g);
-  __shared__ int pref[129];
+  __shared__ int pref[kFrontChunk + 1];
   if (X.counters[kCFlags] & kFAbort) return;
-  for (int chunk = 0; chunk < nlarge; chunk += 128) {
-    const int cnt = min(128, nlarge - chunk);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) {
-        const TppState &S = tpp[chunk + q];
-        int nt = 0;
-        if (S.pad[0] && S.g_p1 > S.g_p0 && S.g_e > S.g_c0)
-          nt = trap_tiles2(X.sn_f[large[chunk + q]] - S.g_c0, S.g_e - S.g_c0);
-        pref[q + 1] = pref[q] + nt;
-      }
-    }
-    __syncthreads();
+  for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
+    const int cnt = min(kFrontChunk, nlarge - chunk);
+    front_prefix<256>(cnt, pref, [&](int q) {
+      const TppState &S = tpp[chunk + q];
+      return S.pad[0] && S.g_p1 > S.g_p0 && S.g_e > S.g_c0
+                 ? trap_tiles2(X.sn_f[large[chunk + q]] - S.g_c0, S.g_e - S.g_c0) : 0;
+    });
     const int total = pref[cnt];
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
       int a = 0, b = cnt;
@@ -1110,7 +1176,7 @@ __global__ void __launch_bounds__(256) k_large_gemm(DevPlan P, DevFactor X, cons
       double *F = X.arena + X.sn_off[s];
       int ti, tj;
       trap_tile2(w - pref[a], f - S.g_c0, S.g_e - S.g_c0, ti, tj);
-      tile_update<false>(F, sf, F + sf * sf, f, nullptr, S.g_c0 + ti * kTM, S.g_c0 + tj * kTN, f, S.g_e,
+      tile_update<0>(F, sf, F + sf * sf, f, nullptr, S.g_c0 + ti * kTM, S.g_c0 + tj * kTN, f, S.g_e,
                          S.g_p0, S.g_p1 - S.g_p0, sm);
     }
   }
@@ -1298,27 +1364,23 @@ __global__ void __launch_bounds__(256, kDBlocksPerSM) k_large_defer(DevPlan P, D
 
 // Schur updates of all large fronts of a level (schur_update,
 // ldlt_kernel.cpp:820-933): F[e:f, e:f] -= L LD^T over pivots [0, k).
-__global__ void __launch_bounds__(256) k_large_schur(DevPlan P, DevFactor X, const int *__restrict__ large,
+template <bool POSDEF>
+__global__ void __launch_bounds__(256, 2) k_large_schur(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                      int nlarge, const TppState *__restrict__ tpp) {
   extern __shared__ __align__(16) double dsm_g[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(dsm_g);
-  __shared__ int pref[129];
+  __shared__ int pref[kFrontChunk + 1];
   if (X.counters[kCFlags] & kFAbort) return;
-  for (int chunk = 0; chunk < nlarge; chunk += 128) {
-    const int cnt = min(128, nlarge - chunk);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) {
-        const int s = large[chunk + q];
-        // pivots [pad[3], k): an APTP front's trailing update covered its own
-        const int e = X.sn_ne[s], f = X.sn_f[s], k = tpp[chunk + q].k, k0 = tpp[chunk + q].pad[3];
-        // mixed fronts: the tensor-core updates covered the contribution block
-        const bool fp64 = !tpp[chunk + q].mixed;
-        pref[q + 1] = pref[q] + ((f > e && k > k0 && fp64) ? trap_tiles2(f - e, f - e) : 0);
-      }
-    }
-    __syncthreads();
+  for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
+    const int cnt = min(kFrontChunk, nlarge - chunk);
+    front_prefix<256>(cnt, pref, [&](int q) {
+      const int s = large[chunk + q];
+      // pivots [pad[3], k): an APTP front's trailing update covered its own
+      const int e = X.sn_ne[s], f = X.sn_f[s], k = tpp[chunk + q].k, k0 = tpp[chunk + q].pad[3];
+      // mixed fronts: the tensor-core updates covered the contribution block
+      const bool fp64 = !tpp[chunk + q].mixed;
+      return (f > e && k > k0 && fp64) ? trap_tiles2(f - e, f - e) : 0;
+    });
     const int total = pref[cnt];
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
       int a = 0, b = cnt;
@@ -1334,7 +1396,8 @@ __global__ void __launch_bounds__(256) k_large_schur(DevPlan P, DevFactor X, con
       double *F = X.arena + X.sn_off[s];
       int ti, tj;
       trap_tile2(w - pref[a], f - e, f - e, ti, tj);
-      tile_update<true>(F, sf, nullptr, 0, X.tags + X.sn_roff[s], e + ti * kTM, e + tj * kTN, f, f, k0, kk, sm);
+      tile_update<POSDEF ? 2 : 1>(F, sf, nullptr, 0, X.tags + X.sn_roff[s], e + ti * kTM, e + tj * kTN, f, f, k0, kk,
+                                  sm);
     }
   }
 }
@@ -1406,16 +1469,12 @@ __global__ void __launch_bounds__(NT) k_large_finish(DevPlan P, DevFactor X, con
 // slot k_large_finish filled). Work items: 32 columns of one front.
 __global__ void __launch_bounds__(256) k_large_store(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                      int nlarge, int posdef) {
-  __shared__ int pref[65];
+  __shared__ int pref[kFrontChunk + 1];
   __shared__ double sdv[32];
   if (X.counters[kCFlags] & kFAbort) return;
-  for (int chunk = 0; chunk < nlarge; chunk += 64) {
-    const int cnt = min(64, nlarge - chunk);
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) pref[q + 1] = pref[q] + (X.sn_pstore[large[chunk + q]] + 31) / 32;
-    }
-    __syncthreads();
+  for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
+    const int cnt = min(kFrontChunk, nlarge - chunk);
+    front_prefix<256>(cnt, pref, [&](int q) { return (X.sn_pstore[large[chunk + q]] + 31) / 32; });
     const int total = pref[cnt];
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
       int a = 0, b = cnt;
@@ -2052,19 +2111,14 @@ __global__ void __launch_bounds__(256) k_bwd_l21(DevPlan P, DevFactor X, const i
                                                  int64_t rows_total, int nrhs) {
   constexpr int CW = kL21Cols / 8;  // columns a warp
   constexpr int TILE = R == 1 ? 1024 : 512;
-  __shared__ int pref[65];
+  __shared__ int pref[kFrontChunk + 1];
   __shared__ double xs[R][TILE];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_wait();
   pdl_trigger();
-  for (int chunk = 0; chunk < nlarge; chunk += 64) {
-    const int cnt = min(64, nlarge - chunk);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) pref[q + 1] = pref[q] + (X.sn_pstore[large[chunk + q]] + kL21Cols - 1) / kL21Cols;
-    }
-    __syncthreads();
+  for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
+    const int cnt = min(kFrontChunk, nlarge - chunk);
+    front_prefix<256>(cnt, pref, [&](int q) { return (X.sn_pstore[large[chunk + q]] + kL21Cols - 1) / kL21Cols; });
     const int total = pref[cnt];
     for (int wi = blockIdx.x; wi < total; wi += gridDim.x) {
       int a = 0, b = cnt;
@@ -2529,21 +2583,16 @@ __global__ void __launch_bounds__(256) k_fwd_gemv(DevPlan P, DevFactor X, const 
                                                   int nrhs) {
   __shared__ __align__(16) double ws[R][kSB];
   __shared__ double part[8][R][33];
-  __shared__ int pref[65];
+  __shared__ int pref[kFrontChunk + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bool waited = false;
-  for (int chunk = 0; chunk < nlarge; chunk += 64) {
-    const int cnt = min(64, nlarge - chunk);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) {
-        const int s = large[chunk + q];
-        const int f = X.sn_f[s], p = X.sn_pstore[s], j1 = min(p, (b + 1) * kSB);
-        pref[q + 1] = pref[q] + ((b * kSB < p && f > j1) ? (f - j1 + 31) / 32 : 0);
-      }
-    }
-    __syncthreads();
+  for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
+    const int cnt = min(kFrontChunk, nlarge - chunk);
+    front_prefix<256>(cnt, pref, [&](int q) {
+      const int s = large[chunk + q];
+      const int f = X.sn_f[s], p = X.sn_pstore[s], j1 = min(p, (b + 1) * kSB);
+      return (b * kSB < p && f > j1) ? (f - j1 + 31) / 32 : 0;
+    });
     const int total = pref[cnt];
     for (int wi = blockIdx.x; wi < total; wi += gridDim.x) {
       int a = 0, bb = cnt;
@@ -2609,23 +2658,17 @@ __global__ void __launch_bounds__(256) k_bwd_dots(DevPlan P, DevFactor X, const 
                                                   int nlarge, int b, double *wk, int64_t rows_total,
                                                   int nrhs) {
   constexpr int CW = R == 1 ? 1 : 2, AHEAD = R == 1 ? 8 : 2;
-  __shared__ int pref[65];
+  __shared__ int pref[kFrontChunk + 1];
   __shared__ double red[8][CW * R];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_wait();
   pdl_trigger();
-  for (int chunk = 0; chunk < nlarge; chunk += 64) {
-    const int cnt = min(64, nlarge - chunk);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      pref[0] = 0;
-      for (int q = 0; q < cnt; ++q) {
-        const int s = large[chunk + q];
-        const int p = X.sn_pstore[s], j0 = b * kSB, j1 = min(p, j0 + kSB);
-        pref[q + 1] = pref[q] + ((j0 < p && j1 < p) ? (j1 - j0 + CW - 1) / CW : 0);
-      }
-    }
-    __syncthreads();
+  for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
+    const int cnt = min(kFrontChunk, nlarge - chunk);
+    front_prefix<256>(cnt, pref, [&](int q) {
+      const int p = X.sn_pstore[large[chunk + q]], j0 = b * kSB, j1 = min(p, j0 + kSB);
+      return (j0 < p && j1 < p) ? (j1 - j0 + CW - 1) / CW : 0;
+    });
     const int total = pref[cnt];
     for (int wi = blockIdx.x; wi < total; wi += gridDim.x) {
       int a = 0, bb = cnt;

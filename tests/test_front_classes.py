@@ -180,3 +180,34 @@ def test_solve_trees(kind, nrhs):
         _, _, om, steps = sv.refine(b[r], one, omega_target=1e-12)
         assert om <= 1e-12 and steps <= 1
     sv.close()
+
+
+@pytest.mark.parametrize("n,ne", [(330, 130), (520, 260), (700, 77)])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_schur_matrix_instructions(n, ne, zeros):
+    """The contribution block of a large front against chains of fused
+    multiply-adds in pivot order (the oracle's): odd sizes, chunks with and
+    without zero multipliers, an infinity-free but wide range of magnitudes."""
+    rng = np.random.default_rng(n)
+    A = _spd(n, rng)
+    s = 10.0 ** rng.uniform(-6, 6, n)
+    if zeros:  # rows without entries in some of the pivots' columns
+        A[ne:, : ne // 2] *= rng.random((n - ne, 1)) < 0.6
+        A[: ne // 2, ne:] = A[ne:, : ne // 2].T
+        A[np.arange(n), np.arange(n)] += n
+    A = A * s[:, None] * s[None, :]
+    n, cp, ri, v = dense_lower(A)
+    # two supernodes: the first ne columns, whose update the second takes
+    a = smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL)
+    arrays = {k: getattr(a, k).copy() for k in smfg._ANALYSIS_FIELDS}
+    arrays["sn_start"], arrays["sn_end"] = np.int32([0, ne]), np.int32([ne, n])
+    arrays["sn_parent"], arrays["postorder"] = np.int32([1, -1]), np.int32([0, 1])
+    arrays["child_ptr"], arrays["child_idx"] = np.int32([0, 0, 1]), np.int32([0])
+    arrays["front_row_ptr"] = np.int32([0, n, 2 * n - ne])
+    arrays["front_row_idx"] = np.concatenate([np.arange(n), np.arange(ne, n)]).astype(np.int32)
+    b = smfg.Analysis(n, arrays)
+    for posdef in (True, False):
+        sv = smfg.Solver(b, device=0)
+        info = sv.factor(v, posdef=posdef, aptp_min_rows=0)
+        _compare(b, sv, info, v, posdef, aptp_min_rows=0)
+        sv.close()
