@@ -969,7 +969,8 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
       if (c.posdef && c.nb == 16) {
         // no delays, no search: one multi-block step per panel, states
         // double-buffered; the closing step leaves phase 2
-        const dim3 pgrid((pl.lvl_large_maxf[l] + 255) / 256, nL);
+        const int rpb = (int64_t)nL * ((pl.lvl_large_maxf[l] + 127) / 128) <= 2 * sms ? 128 : 256;
+        const dim3 pgrid((pl.lvl_large_maxf[l] + rpb - 1) / rpb, nL);
         // two panels (32 pivots) per step and one rank-32 deferred update.
         // Look-ahead (unless profiling): the step's update of the next
         // step's 32 columns runs on the stream before the next step, the
@@ -983,7 +984,7 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
           TppState *cur = x.tpp + (size_t)(it & 1) * pl.max_large;
           TppState *nxt = x.tpp + (size_t)((it + 1) & 1) * pl.max_large;
           gp.mark(st, 2);
-          k_large_panel_spd2<16><<<pgrid, 256, 0, st>>>(d, x, lg, cur, nxt, it, ahead ? 1 : 0);
+          k_large_panel_spd2<16><<<pgrid, 256, 0, st>>>(d, x, lg, cur, nxt, it, ahead ? 1 : 0, rpb);
           gp.mark(st, 2);
           if (ahead) {
             SMFG_CUDA(cudaEventRecord(pl.ev_panel, st));
@@ -2477,6 +2478,8 @@ extern "C" SMFG_API int smfg_kernel_bench_defer(int f, int ne, int k, int reps, 
     S.g_p1 = k;
     S.g_c0 = 16;
     S.g_e = ne;
+    S.f = f;
+    S.ne = ne;
     SMFG_CUDA(cudaMemcpy(tpp, &S, sizeof S, cudaMemcpyHostToDevice));
     DevPlan P{};
     DevFactor X{};

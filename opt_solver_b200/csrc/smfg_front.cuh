@@ -1258,6 +1258,8 @@ struct TppState {
   // are current; every column from there on has the pivots [0, tc_done)
   // applied and waits for a tensor-core update by [tc_done, k)
   int mixed, tc_done, se, flush;
+  int f, ne;        // the front's realized rows and eligible columns
+  long long off;    // its arena offset
   FrontStats st;
 };
 
@@ -1281,6 +1283,8 @@ __device__ __forceinline__ void tpp_init(TppState &S, int ne, bool posdef, bool 
   // block, nbo pivots at a time
   S.se = (mixed && posdef) ? nbo : (1 << 30);
   S.flush = 0;
+  S.f = S.ne = 0;
+  S.off = 0;
   S.st = FrontStats{0, 0, 0, 0, 0.0};
 }
 

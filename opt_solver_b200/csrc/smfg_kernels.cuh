@@ -435,43 +435,131 @@ constexpr int kLargeMin = 384;
 // (more fronts a level in the multi-block kernels).
 constexpr int kLargeMinSpd = 192;
 
-// In-place unit-LDL^T of the nbp x nbp lower block T (the SPD panels'
-// diagonal blocks), all threads of the block: pivot k's reciprocal to
-// linv[k], its multipliers l_kj = t_jk / d_k to lm[k][j], then every entry
-// (i, j), k < j <= i, takes t_ij - t_ik l_kj (skipped for l_kj = 0) -- per
-// entry the one-warp loop's operations in its order. The strictly lower
-// part keeps the unscaled values (its multipliers are lm; the callers read
-// only the diagonal of T afterwards). Stops at the first pivot that is not
+// Unit-LDL^T of the nbp x nbp lower block T (the SPD panels' diagonal
+// blocks), all 256 threads or more: pivot k's value to dv[k], its reciprocal
+// to linv[k], its multipliers l_kj = t_jk / d_k to lm[k][j]; every entry (i, j),
+// k < j <= i, takes t_ij - t_ik l_kj (skipped for l_kj = 0) in pivot order,
+// multiply and subtract rounded separately. Columns past the pivots taken
+// keep their updated values in T. Stops at the first pivot that is not
 // positive and finite; returns the pivots taken. Starts and ends at a
 // barrier. `zero` (shared, optional) is set to 1 when a multiplier is zero.
-template <int NB, int NT = 256>
-__device__ __forceinline__ int spd_diag_factor(double (*T)[NB + 1], double (*lm)[NB], double *linv, int nbp,
-                                               int *zero = nullptr) {
-  const int t = threadIdx.x;
+//
+// A chain of pivots, bound by latency: two pivots a barrier (each thread
+// forms the second pivot's column entries it needs itself, from the two
+// columns as they stood), a block of 16 in 6,700 cycles of a launch against
+// 7,300. With EXT the 16 rows below the block (T rows NB..) and the second
+// panel's diagonal block ride along: the rows take the same eliminations,
+// their unscaled values w to Wr[row][pivot] and multipliers to Lr, and v2, the
+// thread's entry of the second block, its fused chain c = fma(-l, w, c) (w = 0
+// skipped) -- in place of a chain of 16 steps on 16 threads after the block
+// (3,600 cycles). One pivot a barrier with the same additions: 19.6 us a
+// launch on the 64^3 operator against 17.1.
+template <int NB, bool EXT, int NT = 256>
+__device__ __forceinline__ int spd_diag_factor(double (*T)[NB + 1], double (*lm)[NB], double *linv, double *dv, int nbp,
+                                               int *zero = nullptr, int next = 0, double (*Wr)[NB] = nullptr,
+                                               double (*Lr)[NB] = nullptr, double *v2 = nullptr) {
+  static_assert(NB * NB <= NT, "an entry a thread");
+  const int t = threadIdx.x, ti = t / NB, tj = t % NB;
+  const bool mine = t < NB * NB;
   __syncthreads();
-  int np = 0;
-  for (int k = 0; k < nbp; ++k) {
+  int k = 0;
+  while (k < nbp) {
     const double d = T[k][k];
     if (!(d > 0.0 && isfinite(d))) break;
     const double inv = __drcp_rn(d);  // 1.0 / d, correctly rounded
-    if (t == 0) linv[k] = inv;
-    // each entry's thread forms the multiplier it needs itself (column k
-    // is read, not written, in this step): one barrier a pivot
-    for (int e = t; e < NB * NB; e += NT) {
-      const int ti = e / NB, tj = e % NB;
-      if (tj > k && tj <= ti && ti < nbp) {
-        const double l = __dmul_rn(T[tj][k], inv);
-        if (ti == tj) {
-          lm[k][tj] = l;
-          if (zero && l == 0.0) *zero = 1;
+    // columns k and k + 1 at this thread's rows
+    double ci = 0.0, cj = 0.0, cr = 0.0, cq = 0.0, bi = 0.0, bj = 0.0, br = 0.0, bq = 0.0;
+    const bool pair = k + 1 < nbp;
+    double lp = 0.0, d1 = 0.0;
+    if (pair) {
+      const double cp = T[k + 1][k], bp = T[k + 1][k + 1];
+      lp = __dmul_rn(cp, inv);
+      const double u = __dsub_rn(bp, __dmul_rn(cp, lp));
+      d1 = lp != 0.0 ? u : bp;
+    }
+    const bool two = pair && d1 > 0.0 && isfinite(d1);
+    if (mine) {
+      ci = T[ti][k];
+      cj = T[tj][k];
+      bi = T[ti][k + 1 < NB ? k + 1 : k];
+      bj = T[tj][k + 1 < NB ? k + 1 : k];
+      if (EXT) {
+        cr = T[NB + ti][k];
+        cq = T[NB + tj][k];
+        br = T[NB + ti][k + 1 < NB ? k + 1 : k];
+        bq = T[NB + tj][k + 1 < NB ? k + 1 : k];
+      }
+    }
+    // (the second failed: column k + 1, which every thread has read, is
+    // written below)
+    if (pair && !two) __syncthreads();
+    const double inv1 = two ? __drcp_rn(d1) : 0.0;
+    if (mine) {
+      const double lj = __dmul_rn(cj, inv);
+      // pivot k on column k + 1 (its entries as pivot k + 1 finds them)
+      auto step = [&](double b, double c) {
+        const double u = __dsub_rn(b, __dmul_rn(c, lp));
+        return lp != 0.0 ? u : b;
+      };
+      bi = step(bi, ci);
+      bj = step(bj, cj);
+      if (EXT) {
+        br = step(br, cr);
+        bq = step(bq, cq);
+      }
+      const double lj1 = __dmul_rn(bj, inv1);
+      const int last = two ? k + 1 : k;
+      auto entry = [&](double v, double c, double b) {
+        const double u = __dsub_rn(v, __dmul_rn(c, lj));
+        v = lj != 0.0 ? u : v;
+        const double w = __dsub_rn(v, __dmul_rn(b, lj1));
+        return two && lj1 != 0.0 ? w : v;
+      };
+      // (the columns of the pivots taken are not needed any more; column
+      // k + 1 alone when it failed)
+      if (tj > last && tj <= ti && ti < nbp) T[ti][tj] = entry(T[ti][tj], ci, bi);
+      if (EXT && tj > last && tj < nbp && ti < next) T[NB + ti][tj] = entry(T[NB + ti][tj], cr, br);
+      if (ti == 0) {
+        if (tj > k && tj < nbp) {
+          lm[k][tj] = lj;
+          if (zero && lj == 0.0) *zero = 1;
         }
-        if (l != 0.0) T[ti][tj] = __dsub_rn(T[ti][tj], __dmul_rn(T[ti][k], l));
+        if (two && tj > k + 1 && tj < nbp) {
+          lm[k + 1][tj] = lj1;
+          if (zero && lj1 == 0.0) *zero = 1;
+        }
+        if (tj == k) {
+          linv[k] = inv;
+          dv[k] = d;
+        }
+        if (two && tj == k + 1) {
+          linv[k + 1] = inv1;
+          dv[k + 1] = d1;
+        }
+      }
+      if (EXT) {
+        const double a0 = __dmul_rn(cr, inv), a1 = __dmul_rn(br, inv1);
+        if (tj == 0 && ti < next) {
+          Wr[ti][k] = cr;
+          Lr[ti][k] = a0;
+          if (cr == 0.0) *zero = 1;
+          if (two) {
+            Wr[ti][k + 1] = br;
+            Lr[ti][k + 1] = a1;
+            if (br == 0.0) *zero = 1;
+          }
+        }
+        const double y0 = fma(-a0, cq, *v2);
+        if (cq != 0.0) *v2 = y0;
+        const double y1 = fma(-a1, bq, *v2);
+        if (two && bq != 0.0) *v2 = y1;
       }
     }
     __syncthreads();
-    ++np;
+    k += two ? 2 : 1;
+    if (pair && !two) break;
   }
-  return np;
+  return k;
 }
 
 // SPD fronts of the blocked size classes (nb = 16, at least
@@ -487,7 +575,7 @@ __device__ __forceinline__ int spd_diag_factor(double (*T)[NB + 1], double (*lm)
 template <int NT>
 __device__ int spd_front_panels(FrontRef &v, const PivotParams &prm, FrontShared &sh) {
   constexpr int NB = 16;
-  __shared__ double T[NB][NB + 1], lm[NB][NB], linv[NB];
+  __shared__ double T[NB][NB + 1], lm[NB][NB], linv[NB], dv[NB];
   const int f = v.f, ne = v.ne;
   const size_t sf = (size_t)v.ld;
   double *F = v.F, *W = v.W;  // W row q (f doubles): w of the panel's pivot q
@@ -498,7 +586,7 @@ __device__ int spd_front_panels(FrontRef &v, const PivotParams &prm, FrontShared
       const int r = t / NB, c = t % NB;
       T[r][c] = (r < nbp && c <= r) ? F[(size_t)(ps + c) * sf + ps + r] : 0.0;
     }
-    const int np = spd_diag_factor<NB, NT>(T, lm, linv, nbp);
+    const int np = spd_diag_factor<NB, false, NT>(T, lm, linv, dv, nbp);
     for (int i = ps + threadIdx.x; i < f; i += NT) {
       double a[NB];
 #pragma unroll
@@ -525,7 +613,7 @@ __device__ int spd_front_panels(FrontRef &v, const PivotParams &prm, FrontShared
     if (threadIdx.x == 0) {
       for (int k = 0; k < np; ++k) {
         v.tags[ps + k] = 1;
-        inertia_1x1(T[k][k], prm.eff_small, sh.st);
+        inertia_1x1(dv[k], prm.eff_small, sh.st);
         const double rem = (double)(f - (ps + k + 1));
         sh.st.flops += rem + rem * (rem + 1.0);
       }
@@ -762,6 +850,9 @@ __global__ void k_large_init(DevPlan P, DevFactor X, const int *__restrict__ lar
     const bool mixed = X.sn_mixed != nullptr && X.sn_mixed[s] != 0 && nbo > 0;
     tpp_init(S, X.sn_ne[s], posdef != 0, mixed, nbo);
     S.pad[0] = 0;  // deferred update pending
+    S.f = f;
+    S.ne = X.sn_ne[s];
+    S.off = X.sn_off[s];
     X.tpp[blockIdx.x] = S;
   }
 }
@@ -1239,8 +1330,7 @@ __global__ void __launch_bounds__(256, kDBlocksPerSM) k_large_defer(DevPlan P, D
     int nt = 0;
     if (tid < cnt) {
       const TppState &S = tpp[chunk + tid];
-      const int s = large[chunk + tid];
-      const int f = X.sn_f[s];
+      const int f = S.f;
       // the columns of this launch's share of the update
       const int split = min(S.g_e, S.g_c0 + kDK);  // the next step's 32 columns
       const int cs = mode == 2 ? split : S.g_c0, ce = mode == 1 ? split : S.g_e;
@@ -1251,7 +1341,7 @@ __global__ void __launch_bounds__(256, kDBlocksPerSM) k_large_defer(DevPlan P, D
       m_p0[tid] = S.g_p0;
       m_kk[tid] = S.g_p1 - S.g_p0;
       // (W of the panel: the second buffer for odd look-ahead panels)
-      m_off[tid] = (long long)X.sn_off[s];
+      m_off[tid] = S.off;
       m_wo[tid] = S.pad[1];
     }
     // inclusive block scan of the tile counts
@@ -1543,24 +1633,27 @@ __global__ void __launch_bounds__(256) k_large_store(DevPlan P, DevFactor X, con
 // update would (c = fma(-l_p, w_p, c) over its pivots in order, w_p = 0
 // skipped) before the second panel's eliminations, and the columns past
 // both take one chain over the 32 pivots in order. Every block factors both
-// diagonal blocks itself: the first, then the first panel's pivots on the
-// second panel's 16 rows (their unscaled values w and multipliers l to
-// shared memory), the second block updated from them and factored. A
-// failing pivot in the first panel ends the front there (as the one-panel
-// path ends it).
+// diagonal blocks itself: the first with the second panel's 16 rows (their
+// unscaled values w and multipliers l to shared memory) and diagonal block
+// beside it, then the second. A failing pivot in the first panel ends the
+// front there (as the one-panel path ends it). rpb rows a block: 128 when the
+// launch has few blocks (the rows' chains are bound by one SM's FP64 rate:
+// 8,000 cycles for 256 rows, 4,700 for 128). The front's sizes come with its
+// state, two dependent loads fewer ahead of everything else.
 template <int NB>
 __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                           const TppState *__restrict__ cur,
-                                                          TppState *__restrict__ nxt, int iter, int w2) {
-  __shared__ double T[NB][NB + 1], T2[NB][NB + 1];
-  __shared__ double lm[NB][NB], lm2[NB][NB];
-  __shared__ double linv[NB], linv2[NB];
-  __shared__ double Wr[NB][NB], Lr[NB][NB];  // [row of panel 2][pivot of panel 1]
-  __shared__ int np2_sh, zero_sh;
-  if (X.counters[kCFlags] & kFAbort) return;
+                                                          TppState *__restrict__ nxt, int iter, int w2, int rpb) {
+  __shared__ double T[2 * NB][NB + 1], T2[NB][NB + 1];
+  // (rows of multipliers and of w read two at a time)
+  __shared__ __align__(16) double lm[NB][NB], lm2[NB][NB];
+  __shared__ double linv[NB], linv2[NB], dv[NB], dv2[NB];
+  __shared__ __align__(16) double Wr[NB][NB];  // [row of panel 2][pivot of panel 1]
+  __shared__ double Lr[NB][NB];
+  __shared__ int zero_sh;
   const int q = blockIdx.y;
-  const int s = large[q];
   const TppState S = cur[q];
+  if (X.counters[kCFlags] & kFAbort) return;
   const bool lead = blockIdx.x == 0;
   if (S.phase == 2) {
     if (lead && threadIdx.x == 0) {
@@ -1570,13 +1663,13 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
     }
     return;
   }
-  const int f = X.sn_f[s], ne = X.sn_ne[s];
+  const int f = S.f, ne = S.ne;
   const int ps = S.k, pl = min(ne, ps + NB), nbp = pl - ps;
   const int ps2 = pl, pl2 = min(ne, ps2 + NB), nbp2 = pl2 - ps2;
-  const int r0 = ps + blockIdx.x * 256;
+  const int r0 = ps + blockIdx.x * rpb;  // rows [r0, r0 + rpb), a thread each
   if (r0 >= f) return;
   const size_t sf = (size_t)f;
-  double *F = X.arena + X.sn_off[s];
+  double *F = X.arena + S.off;
   // W: rows [0, 16) panel 1, [16, 32) panel 2; w2 (look-ahead): two such
   // buffers alternating by step
   const int wpar = w2 ? (iter & 1) : 0;
@@ -1587,66 +1680,30 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
   // written in this launch before it is read (the panels' diagonal rows are
   // staged in W, and each row below belongs to one thread, which writes
   // panel 1's columns only after reading panel 2's).
-  const int i = r0 + threadIdx.x;
+  const int i = (int)threadIdx.x < rpb ? r0 + (int)threadIdx.x : f;
   static_assert(NB * NB == 256, "one entry of T and T2 per thread");
   const int tr = threadIdx.x / NB, tc = threadIdx.x % NB;
   const double t1v = (tr < nbp && tc <= tr) ? F[(size_t)(ps + tc) * sf + ps + tr] : 0.0;
   const double t2v = (tr < nbp2 && tc <= tr) ? F[(size_t)(ps2 + tc) * sf + ps2 + tr] : 0.0;
-  double ra[NB], rb[NB], wa[NB];
+  const double txv = (tr < nbp2 && tc < nbp) ? F[(size_t)(ps + tc) * sf + ps2 + tr] : 0.0;
+  double ra[NB], rb[NB];
 #pragma unroll
   for (int c = 0; c < NB; ++c) {
     ra[c] = (i < f && c < nbp && ps + c <= i) ? F[(size_t)(ps + c) * sf + i] : 0.0;
     rb[c] = (i < f && c < nbp2 && ps2 + c <= i) ? F[(size_t)(ps2 + c) * sf + i] : 0.0;
-    wa[c] = (threadIdx.x < nbp2 && nbp == NB) ? F[(size_t)(ps + c) * sf + ps2 + threadIdx.x] : 0.0;
   }
-  // panel 1's diagonal block
+  // panel 1's diagonal block, with panel 2's rows and diagonal block
   T[tr][tc] = t1v;
+  T[NB + tr][tc] = txv;
   if (threadIdx.x == 0) zero_sh = 0;
-  const int np1 = spd_diag_factor<NB>(T, lm, linv, nbp, &zero_sh);
+  double v2 = t2v;
+  const int np1 = spd_diag_factor<NB, true>(T, lm, linv, dv, nbp, &zero_sh, nbp2, Wr, Lr, &v2);
   const bool two = np1 == NB && nbp == NB && nbp2 > 0;
+  int np2 = 0;
   if (two) {
-    // panel 1's pivots on panel 2's rows (threads 0..15: one row each)
-    if (threadIdx.x < nbp2) {
-      double a[NB];
-#pragma unroll
-      for (int c = 0; c < NB; ++c) a[c] = wa[c];
-      bool zw = false;
-#pragma unroll
-      for (int k = 0; k < NB; ++k) {
-        const double w = a[k];
-        Wr[threadIdx.x][k] = w;
-        zw = zw || w == 0.0;
-#pragma unroll
-        for (int j = k + 1; j < NB; ++j) {
-          const double l = lm[k][j];
-          const double u = __dsub_rn(a[j], __dmul_rn(w, l));
-          a[j] = l != 0.0 ? u : a[j];
-        }
-        a[k] = __dmul_rn(w, linv[k]);
-        Lr[threadIdx.x][k] = a[k];
-      }
-      if (zw) zero_sh = 1;
-    }
-    // panel 2's diagonal block, panel 1's update applied as the deferred
-    // update applies it
-    __syncthreads();
-    if (tr < nbp2 && tc <= tr) {
-      double v = t2v;
-#pragma unroll
-      for (int p = 0; p < NB; ++p) {
-        const double bw = Wr[tc][p];
-        const double u = fma(-Lr[tr][p], bw, v);
-        v = bw != 0.0 ? u : v;
-      }
-      T2[tr][tc] = v;
-    } else {
-      T2[tr][tc] = 0.0;
-    }
-    const int n2 = spd_diag_factor<NB>(T2, lm2, linv2, nbp2, &zero_sh);
-    if (threadIdx.x == 0) np2_sh = n2;
+    T2[tr][tc] = (tr < nbp2 && tc <= tr) ? v2 : 0.0;
+    np2 = spd_diag_factor<NB, false>(T2, lm2, linv2, dv2, nbp2, &zero_sh);
   }
-  __syncthreads();
-  const int np2 = two ? np2_sh : 0;
   // warps whose rows all lie past the panels' diagonal blocks, with every
   // pivot taken and no zero multiplier or w: each entry takes every update
   // (no tests), the same operations in the same order
@@ -1661,7 +1718,11 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
       const double w = a[k];
       W[(size_t)k * f + i] = w;
 #pragma unroll
-      for (int j = k + 1; j < NB; ++j) a[j] = __dsub_rn(a[j], __dmul_rn(w, lm[k][j]));
+      for (int j = (k + 1) / 2 * 2; j < NB; j += 2) {  // (two multipliers a load)
+        const double2 l = *reinterpret_cast<const double2 *>(&lm[k][j]);
+        if (j > k) a[j] = __dsub_rn(a[j], __dmul_rn(w, l.x));
+        a[j + 1] = __dsub_rn(a[j + 1], __dmul_rn(w, l.y));
+      }
       a[k] = __dmul_rn(w, linv[k]);
     }
 #pragma unroll
@@ -1672,7 +1733,11 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
       for (int c = 0; c < NB; ++c) {
         double v = rb[c];
 #pragma unroll
-        for (int p = 0; p < NB; ++p) v = fma(-a[p], Wr[c][p], v);
+        for (int p = 0; p < NB; p += 2) {
+          const double2 w = *reinterpret_cast<const double2 *>(&Wr[c][p]);
+          v = fma(-a[p], w.x, v);
+          v = fma(-a[p + 1], w.y, v);
+        }
         b[c] = v;
       }
 #pragma unroll
@@ -1680,7 +1745,11 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
         const double w = b[k];
         W[(size_t)(NB + k) * f + i] = w;
 #pragma unroll
-        for (int j = k + 1; j < NB; ++j) b[j] = __dsub_rn(b[j], __dmul_rn(w, lm2[k][j]));
+        for (int j = (k + 1) / 2 * 2; j < NB; j += 2) {
+          const double2 l = *reinterpret_cast<const double2 *>(&lm2[k][j]);
+          if (j > k) b[j] = __dsub_rn(b[j], __dmul_rn(w, l.x));
+          b[j + 1] = __dsub_rn(b[j + 1], __dmul_rn(w, l.y));
+        }
         b[k] = __dmul_rn(w, linv2[k]);
       }
 #pragma unroll
@@ -1696,14 +1765,14 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
     if (r < NB) {
 #pragma unroll
       for (int c = 0; c < NB; ++c)
-        if (c < nbp && c <= r) W[(size_t)c * f + i] = (c < r && c < np1) ? lm[c][r] : T[r][c];
+        if (c < nbp && c <= r) W[(size_t)c * f + i] = c >= np1 ? T[r][c] : c < r ? lm[c][r] : dv[c];
     } else {
       const int r2 = r - NB;
 #pragma unroll
       for (int c = 0; c < NB; ++c) W[(size_t)c * f + i] = Lr[r2][c];
 #pragma unroll
       for (int c = 0; c < NB; ++c)
-        if (c < nbp2 && c <= r2) W[(size_t)(NB + c) * f + i] = (c < r2 && c < np2) ? lm2[c][r2] : T2[r2][c];
+        if (c < nbp2 && c <= r2) W[(size_t)(NB + c) * f + i] = c >= np2 ? T2[r2][c] : c < r2 ? lm2[c][r2] : dv2[c];
     }
   } else if (i < f) {
     double a[NB];
@@ -1782,17 +1851,17 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
     // shuffles -- the same totals as a pivot-by-pivot loop
     const int lane = threadIdx.x;
     const bool p1 = lane < np1, p2 = lane >= NB && lane - NB < np2;
-    double dv = 0.0, term = 0.0;
+    double dpv = 0.0, term = 0.0;
     if (p1 || p2) {
       const int col = p1 ? ps + lane : ps2 + lane - NB;
-      X.tags[X.sn_roff[s] + col] = 1;
-      dv = p1 ? T[lane][lane] : T2[lane - NB][lane - NB];
+      X.tags[X.sn_roff[large[q]] + col] = 1;
+      dpv = p1 ? dv[lane] : dv2[lane - NB];
       const double rem = (double)(f - (col + 1));
       term = rem + rem * (rem + 1.0);
     }
-    const bool zr = (p1 || p2) && (!isfinite(dv) || fabs(dv) < eff_small);
-    const bool po = (p1 || p2) && !zr && dv > 0.0;
-    const bool ng = (p1 || p2) && !zr && !(dv > 0.0);
+    const bool zr = (p1 || p2) && (!isfinite(dpv) || fabs(dpv) < eff_small);
+    const bool po = (p1 || p2) && !zr && dpv > 0.0;
+    const bool ng = (p1 || p2) && !zr && !(dpv > 0.0);
     const int nzr = __popc(__ballot_sync(0xffffffffu, zr)), npo = __popc(__ballot_sync(0xffffffffu, po)),
               nng = __popc(__ballot_sync(0xffffffffu, ng));
 #pragma unroll
