@@ -87,7 +87,22 @@ struct TileShared {
   int itmp[kNb];
   double rv[32];
   int ri[32];
-  int nq1, nmin;
+  int nq1, nmin, np;
+  double lt[kIb][kIb];  // L of an inner block for its rows' solves: column p at lt[p]
+};
+
+// The threads that work on a view: the block, or (small views) one warp of it.
+template <bool WARP>
+struct Group {
+  static __device__ __forceinline__ int tid() { return WARP ? (int)(threadIdx.x & 31) : (int)threadIdx.x; }
+  static __device__ __forceinline__ int size() { return WARP ? 32 : (int)blockDim.x; }
+  static __device__ __forceinline__ void sync() {
+    if (WARP) __syncwarp();
+    else __syncthreads();
+  }
+  static __device__ __forceinline__ bool any(bool b) {
+    return WARP ? __any_sync(0xffffffffu, b) != 0 : __syncthreads_or(b) != 0;
+  }
 };
 
 // A view of a symmetric block by columns of its lower triangle: entry (i, j)
@@ -105,7 +120,7 @@ struct PackView {
 
 // Symmetric transposition of view positions p < q (ldlt_aptp.cpp:67-80);
 // tags, rows, lp and loc follow. Callers synchronize before.
-template <typename View>
+template <bool WARP, typename View>
 static __device__ void cta_swap(const View &V, int m, int p, int q, int8_t *tags, int *rows, int *lp, int *loc) {
   if (p == q) return;
   if (p > q) {
@@ -114,7 +129,7 @@ static __device__ void cta_swap(const View &V, int m, int p, int q, int8_t *tags
     q = t;
   }
   const int items = m - 1;  // p diag pair + (c < p) + (p < c < q) + (r > q)
-  for (int t = threadIdx.x; t < items; t += blockDim.x) {
+  for (int t = Group<WARP>::tid(); t < items; t += Group<WARP>::size()) {
     double *e1, *e2;
     if (t == 0) {
       e1 = V.col(p) + p;
@@ -136,7 +151,7 @@ static __device__ void cta_swap(const View &V, int m, int p, int q, int8_t *tags
     *e1 = *e2;
     *e2 = x;
   }
-  if (threadIdx.x == 0) {
+  if (Group<WARP>::tid() == 0) {
     const int8_t tg = tags[p];
     tags[p] = tags[q];
     tags[q] = tg;
@@ -152,7 +167,7 @@ static __device__ void cta_swap(const View &V, int m, int p, int q, int8_t *tags
       loc[q] = u;
     }
   }
-  __syncthreads();
+  Group<WARP>::sync();
 }
 
 template <typename View>
@@ -181,8 +196,18 @@ __device__ __forceinline__ void warp_argmax(double &v, unsigned &at) {
   v = at == 0xffffffffu ? -1.0 : m;
 }
 
-// The block's argmax; ends with every thread holding it (two barriers).
+// The group's argmax; ends with every thread holding it (a block: two
+// barriers).
+template <bool WARP>
 static __device__ void cta_argmax(ArgMax t, TileShared &sh, double &amax, int &bi, int &bj) {
+  if (WARP) {
+    warp_argmax(t.v, t.at);
+    __syncwarp();
+    amax = t.v;
+    bi = (int)(t.at & 0xffffu);
+    bj = (int)(t.at >> 16);
+    return;
+  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   warp_argmax(t.v, t.at);
   if (lane == 0) {
@@ -201,16 +226,17 @@ static __device__ void cta_argmax(ArgMax t, TileShared &sh, double &amax, int &b
 
 // Complete pivoting on an n x n view (ldlt_aptp.cpp:101-210); returns the
 // pivots taken. lp: the view's permutation record.
-template <typename View>
+template <bool WARP, typename View>
 static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *rows, int *lp, int *loc, double inv_u,
                                       double small, TileShared &sh) {
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+  using GR = Group<WARP>;
+  for (int t = GR::tid(); t < n; t += GR::size()) {
     lp[t] = t;
     tags[t] = 0;
   }
-  __syncthreads();
+  GR::sync();
   int k = 0;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, wid = WARP ? 0 : threadIdx.x >> 5, nw = GR::size() >> 5;
   // the largest entry of the view, then with each pivot's update that of what
   // is left: a warp per column, its lanes down the rows, four in flight
   ArgMax best;
@@ -219,7 +245,7 @@ static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *r
   while (k < n) {
     double amax;
     int bi, bj;
-    cta_argmax(best, sh, amax, bi, bj);
+    cta_argmax<WARP>(best, sh, amax, bi, bj);
     if (!(amax >= small) || !isfinite(amax)) break;
     // every thread takes the decision
     int kind = 1, a = bj, b = -1;
@@ -237,26 +263,47 @@ static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *r
     bool bad = false;
     if (kind == 1) {
       const double lim = __dmul_rn(inv_u, fabs(V.col(a)[a]));
-      for (int r = k + threadIdx.x; r < n; r += blockDim.x)
+      for (int r = k + GR::tid(); r < n; r += GR::size())
         if (r != a && !(fabs(sym_at(V, r, a)) <= lim)) bad = true;
     } else {
       double i00, i10, i11;
       inv2(V.col(a)[a], V.col(a)[b], V.col(b)[b], i00, i10, i11);
-      for (int r = k + threadIdx.x; r < n; r += blockDim.x) {
+      for (int r = k + GR::tid(); r < n; r += GR::size()) {
         if (r == a || r == b) continue;
         const double x0 = sym_at(V, r, a), x1 = sym_at(V, r, b);
         if (!l_ok(fma(i00, x0, __dmul_rn(i10, x1)), inv_u) || !l_ok(fma(i10, x0, __dmul_rn(i11, x1)), inv_u))
           bad = true;
       }
     }
-    if (__syncthreads_or(bad)) break;
+    if (GR::any(bad)) break;
     if (kind == 1) {
-      cta_swap(V, n, k, a, tags, rows, lp, loc);
+      cta_swap<WARP>(V, n, k, a, tags, rows, lp, loc);
       const double *ck = V.col(k);
       const double inv_d = 1.0 / ck[k];
       // entries (i, j), k < j <= i < n: one fused step each (a warp per
       // column)
       best = ArgMax{};
+      if (WARP) {  // (n <= 32: a row a lane, four columns in flight)
+        const double y = lane < n ? ck[lane > k ? lane : k] : 0.0;
+        for (int j0 = k + 1; j0 < n; j0 += 4) {
+          double x[4], l[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int jj = min(j0 + u, n - 1);
+            l[u] = __dmul_rn(ck[jj], inv_d);
+            x[u] = (lane >= jj && lane < n) ? V.col(jj)[lane] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (j0 + u < n && lane >= j0 + u && lane < n) {
+              if (l[u] != 0.0) {
+                x[u] = fma(-y, l[u], x[u]);
+                V.col(j0 + u)[lane] = x[u];
+              }
+              best.add(x[u], lane, j0 + u);
+            }
+        }
+      } else
       for (int jj = k + 1 + wid; jj < n; jj += nw) {
         const double lj = __dmul_rn(ck[jj], inv_d);
         double *cj = V.col(jj);
@@ -278,23 +325,47 @@ static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *r
             }
         }
       }
-      __syncthreads();
+      GR::sync();
       double *ckw = V.col(k);
-      for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) ckw[i] = __dmul_rn(ckw[i], inv_d);
-      if (threadIdx.x == 0) tags[k] = 1;
-      __syncthreads();
+      for (int i = k + 1 + GR::tid(); i < n; i += GR::size()) ckw[i] = __dmul_rn(ckw[i], inv_d);
+      if (GR::tid() == 0) tags[k] = 1;
+      GR::sync();
       k += 1;
     } else {
       int partner = b;
       if (a != k) {
-        cta_swap(V, n, k, a, tags, rows, lp, loc);
+        cta_swap<WARP>(V, n, k, a, tags, rows, lp, loc);
         if (partner == k) partner = a;
       }
-      if (partner != k + 1) cta_swap(V, n, k + 1, partner, tags, rows, lp, loc);
+      if (partner != k + 1) cta_swap<WARP>(V, n, k + 1, partner, tags, rows, lp, loc);
       double *c0 = V.col(k), *c1 = V.col(k + 1);
       double i00, i10, i11;
       inv2(c0[k], c0[k + 1], c1[k + 1], i00, i10, i11);
       best = ArgMax{};
+      if (WARP) {
+        const int lr = lane > k + 1 && lane < n ? lane : k + 1;
+        const double y0 = c0[lr], y1 = c1[lr];
+        for (int j0 = k + 2; j0 < n; j0 += 4) {
+          double x[4], l0[4], l1[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int jj = min(j0 + u, n - 1);
+            const double a0 = c0[jj], a1 = c1[jj];
+            l0[u] = fma(i00, a0, __dmul_rn(i10, a1));
+            l1[u] = fma(i10, a0, __dmul_rn(i11, a1));
+            x[u] = (lane >= jj && lane < n) ? V.col(jj)[lane] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (j0 + u < n && lane >= j0 + u && lane < n) {
+              if (!(l0[u] == 0.0 && l1[u] == 0.0)) {
+                x[u] = __dsub_rn(x[u], fma(y0, l0[u], __dmul_rn(y1, l1[u])));
+                V.col(j0 + u)[lane] = x[u];
+              }
+              best.add(x[u], lane, j0 + u);
+            }
+        }
+      } else
       for (int jj = k + 2 + wid; jj < n; jj += nw) {
         const double a0 = c0[jj], a1 = c1[jj];
         const double l0 = fma(i00, a0, __dmul_rn(i10, a1)), l1 = fma(i10, a0, __dmul_rn(i11, a1));
@@ -319,21 +390,21 @@ static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *r
             }
         }
       }
-      __syncthreads();
-      for (int i = k + 2 + threadIdx.x; i < n; i += blockDim.x) {
+      GR::sync();
+      for (int i = k + 2 + GR::tid(); i < n; i += GR::size()) {
         const double a0 = c0[i], a1 = c1[i];
         c0[i] = fma(i00, a0, __dmul_rn(i10, a1));
         c1[i] = fma(i10, a0, __dmul_rn(i11, a1));
       }
-      if (threadIdx.x == 0) {
+      if (GR::tid() == 0) {
         tags[k] = 2;
         tags[k + 1] = -1;
       }
-      __syncthreads();
+      GR::sync();
       k += 2;
     }
   }
-  __syncthreads();
+  GR::sync();
   return k;
 }
 
@@ -343,14 +414,25 @@ static __device__ int cta_complete_on(const View &V, int n, int8_t *tags, int *r
 static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *rows, int *lp, int *loc, double inv_u,
                                    double small, TileShared &sh, double *pk) {
   const FullView G{A, ld};
-  if (!pk) return cta_complete_on(G, n, tags, rows, lp, loc, inv_u, small, sh);
+  if (!pk) return cta_complete_on<false>(G, n, tags, rows, lp, loc, inv_u, small, sh);
   const PackView S{pk, n};
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   __syncthreads();
   for (int j = threadIdx.x >> 5; j < n; j += nw)
     for (int i = j + lane; i < n; i += 32) S.col(j)[i] = G.col(j)[i];
   __syncthreads();
-  const int p = cta_complete_on(S, n, tags, rows, lp, loc, inv_u, small, sh);
+  int p;
+  if (n <= 32) {
+    // one warp: no block barriers in the chain
+    if (threadIdx.x < 32) {
+      p = cta_complete_on<true>(S, n, tags, rows, lp, loc, inv_u, small, sh);
+      if (lane == 0) sh.np = p;
+    }
+    __syncthreads();
+    p = sh.np;
+  } else {
+    p = cta_complete_on<false>(S, n, tags, rows, lp, loc, inv_u, small, sh);
+  }
   for (int j = threadIdx.x >> 5; j < n; j += nw)
     for (int i = j + lane; i < n; i += 32) G.col(j)[i] = S.col(j)[i];
   __syncthreads();
@@ -358,15 +440,22 @@ static __device__ int cta_complete(double *A, int ld, int n, int8_t *tags, int *
 }
 
 // Rows [r0, r0 + w) of columns [0, ncols): new row r0 + t takes old row
-// r0 + perm[t] (ldlt_aptp.cpp:214-221); w <= blockDim.x.
+// r0 + perm[t] (ldlt_aptp.cpp:214-221); w <= 256.
 static __device__ void cta_permute_rows(double *A, int ld, int ncols, int r0, int w, const int *perm) {
-  for (int c = 0; c < ncols; ++c) {
-    double v = 0.0;
-    if ((int)threadIdx.x < w) v = A[ix(c, ld) + r0 + perm[threadIdx.x]];
-    __syncthreads();
-    if ((int)threadIdx.x < w) A[ix(c, ld) + r0 + threadIdx.x] = v;
-    __syncthreads();
+  const int lane = threadIdx.x & 31;
+  int src[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) src[u] = lane + 32 * u < w ? perm[lane + 32 * u] : 0;
+  for (int c = threadIdx.x >> 5; c < ncols; c += blockDim.x >> 5) {  // a warp per column
+    double v[8], *col = A + ix(c, ld) + r0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = lane + 32 * u < w ? col[src[u]] : 0.0;
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (lane + 32 * u < w) col[lane + 32 * u] = v[u];
   }
+  __syncthreads();
 }
 
 static __device__ bool cta_identity(const int *perm, int w) {
@@ -376,12 +465,12 @@ static __device__ bool cta_identity(const int *perm, int w) {
 }
 
 // x := x L^-T for one row (x holds its first k entries, k <= KMAX), L the
-// unit lower triangle of the tile at T (2x2 off-diagonals read as zero): per
+// unit lower triangle, column p at lt[p] (2x2 off-diagonals zero): per
 // entry one fused chain over the earlier columns in order, a zero L entry
 // skipped; then the D^-1 scaling, returning the first pivot whose
 // multipliers exceed 1/u, or k (ldlt_aptp.cpp:232-265, :292-304).
 template <int KMAX>
-__device__ __forceinline__ int row_solve_scale(double (&x)[KMAX], int k, const double *T, int ld, const int8_t *tags,
+__device__ __forceinline__ int row_solve_scale(double (&x)[KMAX], int k, const double (*lt)[KMAX], const int8_t *tags,
                                                const double *dinv, double inv_u) {
 #pragma unroll
   for (int j = 1; j < KMAX; ++j) {
@@ -389,8 +478,9 @@ __device__ __forceinline__ int row_solve_scale(double (&x)[KMAX], int k, const d
       double xj = x[j];
 #pragma unroll
       for (int p = 0; p < j; ++p) {
-        const double l = (tags[p] == 2 && j == p + 1) ? 0.0 : T[ix(p, ld) + j];
-        if (l != 0.0) xj = fma(-x[p], l, xj);
+        const double l = lt[p][j];
+        const double y = fma(-x[p], l, xj);
+        xj = l != 0.0 ? y : xj;
       }
       x[j] = xj;
     }
@@ -424,8 +514,11 @@ __device__ __forceinline__ int row_solve_scale(double (&x)[KMAX], int k, const d
 static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1, int8_t *tags, int *rows, int *lp,
                                 int *loc, double inv_u, double small, TileShared &sh) {
   // 1. backup: column c0 + t, tile rows [c0 + t, w)
-  for (int t = 0; t < w1; ++t)
-    for (int r = c0 + t + threadIdx.x; r < w; r += blockDim.x) sh.bk1[t * kNb + r] = T[ix(c0 + t, ld) + r];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll 2
+  for (int t = wid; t < w1; t += nw)
+#pragma unroll 4
+    for (int r = c0 + t + lane; r < w; r += 32) sh.bk1[t * kNb + r] = T[ix(c0 + t, ld) + r];
   __syncthreads();
   // 2. complete pivoting on the diagonal block
   const int ne_t = cta_complete(T + ix(c0, ld) + c0, ld, w1, tags + c0, rows + c0, sh.lpc1, loc ? loc + c0 : nullptr,
@@ -433,8 +526,8 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
   // 3. its permutation on the rest of the tile
   if (!cta_identity(sh.lpc1, w1)) {
     cta_permute_rows(T, ld, c0, c0, w1, sh.lpc1);
-    for (int t = 0; t < w1; ++t)
-      for (int r = c0 + w1 + threadIdx.x; r < w; r += blockDim.x) T[ix(c0 + t, ld) + r] = sh.bk1[sh.lpc1[t] * kNb + r];
+    for (int t = wid; t < w1; t += nw)
+      for (int r = c0 + w1 + lane; r < w; r += 32) T[ix(c0 + t, ld) + r] = sh.bk1[sh.lpc1[t] * kNb + r];
     if ((int)threadIdx.x < w1) sh.itmp[threadIdx.x] = lp[c0 + sh.lpc1[threadIdx.x]];
     __syncthreads();
     if ((int)threadIdx.x < w1) lp[c0 + threadIdx.x] = sh.itmp[threadIdx.x];
@@ -442,23 +535,25 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
   }
   const double *Tb = T + ix(c0, ld) + c0;  // the block's diagonal tile
   const int8_t *tb = tags + c0;
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < ne_t; ++j) {
-      if (tb[j] == 2) {
-        double i00, i10, i11;
-        inv2(Tb[ix(j, ld) + j], Tb[ix(j, ld) + j + 1], Tb[ix(j + 1, ld) + j + 1], i00, i10, i11);
-        sh.dinv1[2 * j] = i00;
-        sh.dinv1[2 * j + 1] = i10;
-        sh.dinv1[2 * (j + 1)] = i11;
-        sh.dinv1[2 * (j + 1) + 1] = 0.0;
-        ++j;
-      } else {
-        sh.dinv1[2 * j] = 1.0 / Tb[ix(j, ld) + j];
-        sh.dinv1[2 * j + 1] = 0.0;
-      }
+  if ((int)threadIdx.x < ne_t) {
+    const int j = threadIdx.x;
+    if (tb[j] == 2) {
+      double i00, i10, i11;
+      inv2(Tb[ix(j, ld) + j], Tb[ix(j, ld) + j + 1], Tb[ix(j + 1, ld) + j + 1], i00, i10, i11);
+      sh.dinv1[2 * j] = i00;
+      sh.dinv1[2 * j + 1] = i10;
+      sh.dinv1[2 * (j + 1)] = i11;
+      sh.dinv1[2 * (j + 1) + 1] = 0.0;
+    } else if (tb[j] == 1) {
+      sh.dinv1[2 * j] = 1.0 / Tb[ix(j, ld) + j];
+      sh.dinv1[2 * j + 1] = 0.0;
     }
-    sh.nmin = ne_t;
   }
+  for (int e = threadIdx.x; e < kIb * kIb; e += blockDim.x) {
+    const int p = e / kIb, j = e % kIb;
+    sh.lt[p][j] = (p < ne_t && j > p && j < w1 && !(tb[p] == 2 && j == p + 1)) ? Tb[ix(p, ld) + j] : 0.0;
+  }
+  if (threadIdx.x == 0) sh.nmin = ne_t;
   __syncthreads();
   // 4. ApplyN on the tile rows below the block and ApplyT (check pass) on
   // the earlier failed columns: the first failing pivot over all rows
@@ -474,7 +569,7 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
       const size_t stride = below ? (size_t)ld : 1;
 #pragma unroll
       for (int u = 0; u < kIb; ++u) x[u] = (u < ne_t) ? src[u * stride] : 0.0;
-      const int fl = row_solve_scale<kIb>(x, ne_t, Tb, ld, tb, sh.dinv1, inv_u);
+      const int fl = row_solve_scale<kIb>(x, ne_t, sh.lt, tb, sh.dinv1, inv_u);
       if (below) {
 #pragma unroll
         for (int u = 0; u < kIb; ++u)
@@ -510,44 +605,61 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
       double *src = T + ix(sh.q1[t], ld) + c0;
 #pragma unroll
       for (int u = 0; u < kIb; ++u) x[u] = (u < nelim) ? src[u] : 0.0;
-      row_solve_scale<kIb>(x, nelim, Tb, ld, tb, sh.dinv1, inv_u);
+      row_solve_scale<kIb>(x, nelim, sh.lt, tb, sh.dinv1, inv_u);
 #pragma unroll
       for (int u = 0; u < kIb; ++u)
         if (u < nelim) src[u] = x[u];
     }
     // UpdateNN: W = (L D)^T of the columns [e0, w) into their strict upper
-    // triangle rows [c0, c0 + nelim)
+    // triangle rows [c0, c0 + nelim), and with the rows' L in shared memory
+    // (past the backup, which is done with; row r of pivot p at [p][r])
     const int e0 = c0 + nelim;
-    for (int col = e0 + threadIdx.x; col < w; col += blockDim.x) {
-      for (int t = 0; t < nelim; ++t) {
+    double(*Lp)[kNb] = reinterpret_cast<double(*)[kNb]>(sh.pk);
+    double(*Wp)[kNb] = reinterpret_cast<double(*)[kNb]>(sh.pk + kIb * kNb);
+    static_assert(2 * kIb * kNb <= kPackDoubles, "L and W panels");
+    __syncthreads();  // (the restore has read the backup)
+    for (int t = wid; t < nelim; t += nw)
+      for (int col = e0 + lane; col < w; col += 32) {
         const double l0 = T[ix(c0 + t, ld) + col];
+        double v;
         if (tb[t] == 2) {
           const double l1 = T[ix(c0 + t + 1, ld) + col];
-          T[ix(col, ld) + c0 + t] = fma(l1, Tb[ix(t, ld) + t + 1], __dmul_rn(l0, Tb[ix(t, ld) + t]));
-          T[ix(col, ld) + c0 + t + 1] = fma(l0, Tb[ix(t, ld) + t + 1], __dmul_rn(l1, Tb[ix(t + 1, ld) + t + 1]));
-          ++t;
+          v = fma(l1, Tb[ix(t, ld) + t + 1], __dmul_rn(l0, Tb[ix(t, ld) + t]));
+        } else if (tb[t] == -1) {
+          const double lm1 = T[ix(c0 + t - 1, ld) + col];
+          v = fma(lm1, Tb[ix(t - 1, ld) + t], __dmul_rn(l0, Tb[ix(t, ld) + t]));
         } else {
-          T[ix(col, ld) + c0 + t] = __dmul_rn(l0, Tb[ix(t, ld) + t]);
+          v = __dmul_rn(l0, Tb[ix(t, ld) + t]);
         }
+        T[ix(col, ld) + c0 + t] = v;
+        Wp[t][col] = v;
+        Lp[t][col] = l0;
       }
-    }
     __syncthreads();
-    for (int cj = e0 + (threadIdx.x >> 5); cj < w; cj += (blockDim.x >> 5)) {
-      for (int ri = cj + (threadIdx.x & 31); ri < w; ri += 32) {
-        double c = T[ix(cj, ld) + ri];
+    // a warp four columns at a time, lanes over the rows
+    for (int j0 = e0 + 4 * wid; j0 < w; j0 += 4 * nw) {
+      for (int ri = j0 + lane; ri < w; ri += 32) {
+        double c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = (j0 + u <= ri) ? T[ix(j0 + u, ld) + ri] : 0.0;
         for (int p = 0; p < nelim; ++p) {
-          const double bw = T[ix(cj, ld) + c0 + p];
-          if (bw != 0.0) c = fma(-T[ix(c0 + p, ld) + ri], bw, c);
+          const double a = -Lp[p][ri];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const double bw = Wp[p][min(j0 + u, w - 1)];
+            const double y = fma(a, bw, c[u]);
+            c[u] = bw != 0.0 ? y : c[u];
+          }
         }
-        T[ix(cj, ld) + ri] = c;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (j0 + u <= ri) T[ix(j0 + u, ld) + ri] = c[u];
       }
     }
     // UpdateNT / TN: the earlier failed columns, tile rows [e0, w) and their
     // block among themselves; each entry one chain from zero, then one
     // subtraction. (L D) of the failed columns' rows first, into bk1 (the
-    // backup is done with): formed per entry it was most of the kernel, 2.0
-    // of 2.4 ms a tile with 200 failed columns. A warp takes four columns,
-    // lanes the rows.
+    // panels are done with). A warp takes four columns, lanes the rows.
     double(*ldq)[kIb] = reinterpret_cast<double(*)[kIb]>(sh.bk1);
     __syncthreads();
     for (int e = threadIdx.x; e < nq * nelim; e += blockDim.x) {
@@ -557,7 +669,6 @@ static __device__ int tile_inner_block(double *T, int ld, int w, int c0, int w1,
                                  : ld_of(Tb, ld, tb, p, lq[p], tb[p] == 2 ? lq[p + 1] : 0.0);
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int j0 = 4 * wid; j0 < nq; j0 += 4 * nw) {
       const int nj = min(4, nq - j0);
       // rows [e0, w) of the tile, then the failed columns' rows from j0 on
@@ -600,7 +711,7 @@ static __device__ void cta_compact(double *A, int ld, int m, int ne, int8_t *tag
   int dst = 0;
   for (int src = 0; src < ne; ++src) {
     if (tags[src] == 0) continue;
-    if (src != dst) cta_swap(FullView{A, ld}, m, dst, src, tags, rows, lp, loc);
+    if (src != dst) cta_swap<false>(FullView{A, ld}, m, dst, src, tags, rows, lp, loc);
     ++dst;
   }
   __syncthreads();
