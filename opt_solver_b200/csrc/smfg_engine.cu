@@ -798,16 +798,17 @@ static int fuse_rows(const smfg_control_t &c) { return std::min(kFuseMax, c.bloc
 // last on the plan's stream unless the large fronts come there. Returns the
 // side streams used, whose events the caller waits for.
 // A class is a range of the level's list (largest symbolic front first).
-// SPD: exact. Indefinite: delays may have grown any smaller front into it, so
-// the range runs to the end of the list (level 0 has no children: exact);
-// the kernels test the realized rows.
+// On the static SPD layout: exact. Otherwise delays (of an SPD factorization's
+// failed pivots too) may have grown any smaller front into it, so the range
+// runs to the end of the list (level 0 has no children: exact); the kernels
+// test the realized rows.
 static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, int fuse, const PivotParams &prm,
                                     bool has_large, LaunchCount &lc) {
   DevPlan &d = pl.d;
   DevFactor &x = pl.x;
   cudaStream_t st = pl.stream;
   const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
-  const bool exact = c.posdef || l == 0;
+  const bool exact = x.spd_static || l == 0;
   auto at_most = [&](int v) { return level_at_most(pl, l, v); };
   enum Kind { kGlobal, kMedium, kUpper, kSmall, kWarp };
   struct Class { Kind kind; int fmin, fmax, i0, n; };

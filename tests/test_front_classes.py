@@ -211,3 +211,26 @@ def test_schur_matrix_instructions(n, ne, zeros):
         info = sv.factor(v, posdef=posdef, aptp_min_rows=0)
         _compare(b, sv, info, v, posdef, aptp_min_rows=0)
         sv.close()
+
+
+@pytest.mark.parametrize("m", [6, 12, 20])
+def test_not_positive_definite_tree(m):
+    """Failed pivots all over a tree: the columns they delay grow the fronts
+    above past their symbolic size class, and the factorization still reports
+    NOT_POSDEF, twice the same; the next one of good values is the oracle's."""
+    n, cp, ri, good = W.varcoef_3d(m, seed=m)
+    v = good.copy()
+    v[W.diagonal_slots(n, cp, ri)[np.random.default_rng(m).choice(n, 3)]] *= -1
+    a = smfg.analyse(n, cp, ri)
+    sv = smfg.Solver(a, device=0)
+    runs = []
+    for _ in range(2):
+        info = sv.factor(v, posdef=True)
+        assert info.factor_status == smfg.SMFG_FACTOR_NOT_POSDEF
+        assert sum(info.inertia) + info.delayed_pivots >= n
+        runs.append((info.inertia, info.delayed_pivots, info.flops, sv.front_stats().tolist()))
+    assert runs[0] == runs[1]
+    assert runs[0][1] > 0
+    gi = sv.factor(good, posdef=True)
+    _compare(a, sv, gi, good, True)
+    sv.close()
