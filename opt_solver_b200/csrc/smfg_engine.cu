@@ -210,6 +210,17 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   pl.h_fsym = fsym;
   pl.lvl_maxf.assign(nl, 0);
   pl.lvl_maxkids.assign(nl, 0);
+  pl.lvl_cols.assign(nl, kAsmCols);
+  {
+    // (the 701 x 433 grid's upper levels of a few fronts: with this, two children
+    // in flight and the division-free store, its factorization 5.48 -> 5.15 ms;
+    // 64^3 operator 32.92 -> 32.79 ms, 23^3 3.85 -> 3.66 ms with its transfers)
+    std::vector<int64_t> items(nl, 0);
+    for (int s = 0; s < ns; ++s)
+      if (fsym[s] > kFuseMax) items[level[s]] += (fsym[s] + kAsmCols - 1) / kAsmCols;
+    for (int l = 0; l < nl; ++l)
+      if (items[l] < 4 * sm_count(pl.device)) pl.lvl_cols[l] = kAsmColsFew;
+  }
   for (int s = 0; s < ns; ++s) {
     pl.lvl_maxf[level[s]] = std::max(pl.lvl_maxf[level[s]], fsym[s]);
     pl.lvl_maxkids[level[s]] = std::max(pl.lvl_maxkids[level[s]], a.child_ptr[s + 1] - a.child_ptr[s]);
@@ -418,7 +429,7 @@ static void ensure_spd_layout(Plan &pl, int wcols, int fuse) {
       a += spd_front_doubles(pl, s, wcols);
       r += f;
       blk[i + l] = b;
-      b += (f <= fuse && !pl.h_large[s]) ? 0 : (f + kAsmCols - 1) / kAsmCols;
+      b += (f <= fuse && !pl.h_large[s]) ? 0 : (f + pl.lvl_cols[l] - 1) / pl.lvl_cols[l];
     }
     blk[pl.lvl_ptr[l + 1] + l] = b;
   }
@@ -873,8 +884,7 @@ static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, in
       k_level_rows<<<na, pl.lvl_maxf[l] >= 1024 ? 512 : 128, 0, st>>>(d, x, lo, fuse);
       lc.n += 1;
     }
-    // 32-column work items: a level of a few large fronts has hundreds
-    k_level_assemble<<<8 * sm_count(pl.device), 256, 0, st>>>(d, x, lo, hi, l);
+    k_level_assemble<<<8 * sm_count(pl.device), 256, 0, st>>>(d, x, lo, hi, l, pl.lvl_cols[l]);
     lc.n += 1;
   }
   if (nc > first && !fused(cls[first])) {
@@ -931,7 +941,7 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
   for (int l = 0; l < pl.nlevels; ++l) {
     const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
     if (!fixed_layout) {
-      k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse);
+      k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse, pl.lvl_cols[l]);
       lc.n += 1;
     }
     const int nL = pl.lvl_large_ptr[l + 1] - pl.lvl_large_ptr[l];
@@ -963,7 +973,8 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
       bool tpp_work = true;
       if (!aq.empty()) tpp_work = aptp_sweep(pl, c, asz, aq, nL, lc);
       const int team = level_team(pl, c, pl.lvl_large_maxf[l]);
-      SMFG_CUDA(cudaMemsetAsync(x.counters + kCActive, 0, sizeof(unsigned long long), st));
+      // (the steps asked for: read by the indefinite batches)
+      if (!c.posdef) SMFG_CUDA(cudaMemsetAsync(x.counters + kCActive, 0, sizeof(unsigned long long), st));
       const int ggrid = 2 * sms;
       int it = 0;
       TppState *fin = x.tpp;  // where the final state of the level's fronts ends up

@@ -16,7 +16,9 @@ namespace smfg {
 constexpr int kFuseMax = 95;     // assembled, factored and stored by one block (smfg_small.cuh), below
                                  // the blocked size (blocked_min_front, 96)
 constexpr int kMediumMax = 128;  // one block, front in shared memory
-constexpr int kAsmCols = 32;     // columns per assembly work item
+// Columns per assembly work item: 32, or 8 on levels that would not give every
+// SM a few items (Plan::lvl_cols).
+constexpr int kAsmCols = 32, kAsmColsFew = 8;
 
 // Device copies of the analysis-derived arrays (one per plan).
 struct DevPlan {
@@ -90,6 +92,7 @@ struct Plan {
   std::vector<int> lvl_ptr;      // host copy: level l = lvl_sn[lvl_ptr[l] .. lvl_ptr[l+1])
   std::vector<int> lvl_maxf;     // symbolic max front per level
   std::vector<int> lvl_maxkids;
+  std::vector<int> lvl_cols;     // columns per assembly work item
   std::vector<int> lvl_large_ptr;  // level l's large fronts: d.lvl_large[lvl_large_ptr[l] ..]
   std::vector<int> lvl_large_maxw; // widest large front per level
   std::vector<int> lvl_large_maxf; // largest symbolic front among them

@@ -84,7 +84,7 @@ __global__ void k_eff_small(unsigned long long *cnt, double small_pivot, long lo
 // offsets by exclusive scan, delay offsets of the children in the parent's
 // row list (multifrontal_serial.cpp:510-545), assembly work items.
 template <int NT>
-__global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, int nb, int fuse) {
+__global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, int nb, int fuse, int cols) {
   static_assert(NT % 32 == 0 && NT <= 1024, "block size");
   constexpr int NW = NT / 32;
   __shared__ long long wa[NW], wr[NW], wb[NW];
@@ -115,7 +115,7 @@ __global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, i
       fa = (long long)f * f + (long long)f * nb;
       fr = f;
       // (fronts of at most fuse rows are assembled by their front kernel)
-      fb = (f <= fuse && !P.sn_large[s]) ? 0 : (f + kAsmCols - 1) / kAsmCols;
+      fb = (f <= fuse && !P.sn_large[s]) ? 0 : (f + cols - 1) / cols;
     }
     // inclusive block scan of (fa, fr, fb): warp shuffles, then the warps'
     // totals scanned by warp 0
@@ -221,7 +221,7 @@ __global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int fuse) {
 }
 
 // Assembly of one level (process_front, multifrontal_serial.cpp:720-789):
-// each work item is a block of kAsmCols columns of one front. It zeroes the
+// each work item is a block of `cols` columns of one front. It zeroes the
 // lower part of its columns, adds the original entries of the pivot columns,
 // then extend-adds the children's Schur blocks in child order (the
 // reference's order of additions, so every entry is the reference's sum).
@@ -253,7 +253,7 @@ __device__ __forceinline__ int warp_lower_bound(const int *__restrict__ a, int l
 // not fit take the passes.
 constexpr int kAsmMap = 12288, kAsmKids = 16;
 
-__global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, int lo, int hi, int lvl) {
+__global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, int lo, int hi, int lvl, int cols) {
   unsigned long long *cnt = X.counters;
   if (cnt[kCFlags] & kFAbort) return;
   const int *pref = X.lvl_blk + lo + lvl;  // m + 1 prefix entries
@@ -273,8 +273,8 @@ __global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, 
     }
     const int s = P.lvl_sn[lo + a];
     const int f = X.sn_f[s], nd = X.sn_nd[s];
-    const int j0 = (w - pref[a]) * kAsmCols;
-    const int j1 = min(j0 + kAsmCols, f);
+    const int j0 = (w - pref[a]) * cols;
+    const int j1 = min(j0 + cols, f);
     double *F = X.arena + X.sn_off[s];
     const size_t sf = (size_t)f;
     const int t0 = P.child_ptr[s], nk = P.child_ptr[s + 1] - t0;
@@ -309,18 +309,22 @@ __global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, 
         double *Fj = F + jj * sf;
         for (int i0 = jj + lane; i0 < f; i0 += 4 * 32) {
           double v[4] = {0.0, 0.0, 0.0, 0.0};
-          for (int t = 0; t < nk; ++t) {
-            const int uj = inv[t * f + jj];
-            if (uj == 0xffff) continue;  // (the same for the whole warp)
-            const double *Fc = X.arena + ch_off[t] + (size_t)uj * ch_f[t];
-            double x[4];
+          for (int t = 0; t < nk; t += 2) {  // two children's loads in flight
+            double x[2][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int ui = i0 + 32 * u < f ? inv[t * f + i0 + 32 * u] : 0xffff;
-              x[u] = ui != 0xffff ? Fc[ui] : -0.0;  // (v + -0.0 is v)
+            for (int e = 0; e < 2; ++e) {
+              const int tt = min(t + e, nk - 1);
+              // (the same for the whole warp)
+              const int uj = t + e < nk ? inv[tt * f + jj] : 0xffff;
+              const double *Fc = X.arena + ch_off[tt] + (size_t)(uj == 0xffff ? 0 : uj) * ch_f[tt];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const int ui = (uj != 0xffff && i0 + 32 * u < f) ? inv[tt * f + i0 + 32 * u] : 0xffff;
+                x[e][u] = ui != 0xffff ? Fc[ui] : -0.0;  // (v + -0.0 is v)
+              }
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] += x[u];
+            for (int u = 0; u < 4; ++u) v[u] = (v[u] + x[0][u]) + x[1][u];
           }
 #pragma unroll
           for (int u = 0; u < 4; ++u)
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, 
     if (ca < cb) {
       const int k0 = P.pcp[cs + ca], k1 = P.pcp[cs + cb];
       for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        int c = ca;  // the column of slot k (at most kAsmCols candidates)
+        int c = ca;  // the column of slot k (at most cols candidates)
         while (c + 1 < cb && P.pcp[cs + c + 1] <= k) ++c;
         F[(nd + c) * sf + nd + P.amap[k]] += X.pv[k];
       }
@@ -762,13 +766,15 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
   }
   // The children's row maps, built in assembly order, now point at the
   // rows' final (pivot-order) positions: the solves read them that way.
-  for (int t = threadIdx.x; t < f; t += NT) inv[v.loc[t]] = t;
-  __syncthreads();
-  for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
-    const int c = P.child_idx[t];
-    const int pc = X.sn_p[c];
-    int *cmap = X.cbmap + X.sn_roff[c] + pc;
-    for (int u = threadIdx.x; u < X.sn_f[c] - pc; u += NT) cmap[u] = inv[cmap[u]];
+  if (!prm.posdef) {  // (SPD rows keep their order)
+    for (int t = threadIdx.x; t < f; t += NT) inv[v.loc[t]] = t;
+    __syncthreads();
+    for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
+      const int c = P.child_idx[t];
+      const int pc = X.sn_p[c];
+      int *cmap = X.cbmap + X.sn_roff[c] + pc;
+      for (int u = threadIdx.x; u < X.sn_f[c] - pc; u += NT) cmap[u] = inv[cmap[u]];
+    }
   }
   if (threadIdx.x == 0) {
     X.sn_p[s] = p;
@@ -841,7 +847,7 @@ __global__ void k_large_init(DevPlan P, DevFactor X, const int *__restrict__ lar
   const int f = X.sn_f[s];
   int *loc = X.ploc + X.sn_roff[s];
   int *inv = X.ploc + X.rows_cap + X.sn_roff[s];
-  for (int t = threadIdx.x; t < f; t += blockDim.x) {
+  for (int t = threadIdx.x; t < f && !posdef; t += blockDim.x) {
     loc[t] = t;
     inv[t] = t;
   }
@@ -1530,14 +1536,16 @@ __global__ void __launch_bounds__(NT) k_large_finish(DevPlan P, DevFactor X, con
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) set_flag(X.counters, kFNonfiniteD);
   }
-  int *inv = X.ploc + X.rows_cap + X.sn_roff[s];
-  for (int t = threadIdx.x; t < f; t += NT) inv[v.loc[t]] = t;
-  __syncthreads();
-  for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
-    const int c = P.child_idx[t];
-    const int pc = X.sn_p[c];
-    int *cmap = X.cbmap + X.sn_roff[c] + pc;
-    for (int u = threadIdx.x; u < X.sn_f[c] - pc; u += NT) cmap[u] = inv[cmap[u]];
+  if (!prm.posdef) {  // (SPD rows keep their order)
+    int *inv = X.ploc + X.rows_cap + X.sn_roff[s];
+    for (int t = threadIdx.x; t < f; t += NT) inv[v.loc[t]] = t;
+    __syncthreads();
+    for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
+      const int c = P.child_idx[t];
+      const int pc = X.sn_p[c];
+      int *cmap = X.cbmap + X.sn_roff[c] + pc;
+      for (int u = threadIdx.x; u < X.sn_f[c] - pc; u += NT) cmap[u] = inv[cmap[u]];
+    }
   }
   if (threadIdx.x == 0) {
     X.sn_p[s] = p;
@@ -1582,26 +1590,19 @@ __global__ void __launch_bounds__(256) k_large_store(DevPlan P, DevFactor X, con
       if (posdef) {
         if (threadIdx.x < c1 - c0) sdv[threadIdx.x] = sqrt(F[(size_t)(c0 + threadIdx.x) * sf + c0 + threadIdx.x]);
         __syncthreads();
-        // the item's columns as one run of (column, row) pairs (columns are
-        // contiguous, leading dimension f), eight entries a thread in flight
-        double *base = F + (size_t)c0 * sf;
-        const int64_t n = (int64_t)(c1 - c0) * f;
-        for (int64_t t0 = threadIdx.x; t0 < n; t0 += 8 * 256) {
-          double y[8];
-          int cc[8], ii[8];
+        // a warp per column, eight rows a lane in flight
+        const int lane = threadIdx.x & 31;
+        for (int c = c0 + (threadIdx.x >> 5); c < c1; c += 8) {
+          double *Lc = F + (size_t)c * sf;
+          const double sq = sdv[c - c0];
+          for (int i = lane; i < c; i += 32) Lc[i] = 0.0;
+          for (int i0 = c + 1 + lane; i0 < f; i0 += 8 * 32) {
+            double y[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int64_t t = t0 + 256 * u;
-            cc[u] = c0 + (int)(t / f);
-            ii[u] = (int)(t % f);
-            y[u] = (t < n && ii[u] > cc[u]) ? base[t] : 0.0;  // the strictly lower part is read
-          }
+            for (int u = 0; u < 8; ++u) y[u] = i0 + 32 * u < f ? Lc[i0 + 32 * u] : 0.0;
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int64_t t = t0 + 256 * u;
-            if (t >= n) continue;
-            if (ii[u] < cc[u]) base[t] = 0.0;
-            else if (ii[u] > cc[u]) base[t] = __dmul_rn(y[u], sdv[cc[u] - c0]);
+            for (int u = 0; u < 8; ++u)
+              if (i0 + 32 * u < f) Lc[i0 + 32 * u] = __dmul_rn(y[u], sq);
           }
         }
         __syncthreads();

@@ -183,15 +183,16 @@ def test_solve_trees(kind, nrhs):
 
 
 @pytest.mark.parametrize("n,ne", [(330, 130), (520, 260), (700, 77)])
-@pytest.mark.parametrize("zeros", [False, True])
-def test_schur_matrix_instructions(n, ne, zeros):
+@pytest.mark.parametrize("kind", ["wide", "zeros", "subnormal"])
+def test_schur_matrix_instructions(n, ne, kind):
     """The contribution block of a large front against chains of fused
     multiply-adds in pivot order (the oracle's): odd sizes, chunks with and
-    without zero multipliers, an infinity-free but wide range of magnitudes."""
+    without zero multipliers, a wide range of magnitudes, and entries down to
+    the subnormal numbers."""
     rng = np.random.default_rng(n)
     A = _spd(n, rng)
-    s = 10.0 ** rng.uniform(-6, 6, n)
-    if zeros:  # rows without entries in some of the pivots' columns
+    s = np.full(n, 1e-155) if kind == "subnormal" else 10.0 ** rng.uniform(-6, 6, n)
+    if kind == "zeros":  # rows without entries in some of the pivots' columns
         A[ne:, : ne // 2] *= rng.random((n - ne, 1)) < 0.6
         A[: ne // 2, ne:] = A[ne:, : ne // 2].T
         A[np.arange(n), np.arange(n)] += n
@@ -206,11 +207,35 @@ def test_schur_matrix_instructions(n, ne, zeros):
     arrays["front_row_ptr"] = np.int32([0, n, 2 * n - ne])
     arrays["front_row_idx"] = np.concatenate([np.arange(n), np.arange(ne, n)]).astype(np.int32)
     b = smfg.Analysis(n, arrays)
-    for posdef in (True, False):
+    for posdef in (True,) if kind == "subnormal" else (True, False):
         sv = smfg.Solver(b, device=0)
         info = sv.factor(v, posdef=posdef, aptp_min_rows=0)
         _compare(b, sv, info, v, posdef, aptp_min_rows=0)
         sv.close()
+
+
+@pytest.mark.parametrize("n,bad", [(300, 36), (300, 37), (300, 143), (96, 51), (97, 50)])
+def test_not_positive_definite_large(n, bad):
+    """A pivot that fails at an even or odd place of a pair, in the first or the
+    second panel of a step: the columns before it are those of the matrix that
+    differs from it in that diagonal entry alone, the run on the static layout
+    is given up and redone, and the next factorization of the plan is
+    unaffected."""
+    rng = np.random.default_rng(n + bad)
+    A = _spd(n, rng)
+    good = dense_lower(A)
+    A[bad, bad] = -5.0
+    _, cp, ri, v = dense_lower(A)
+    a = smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL)
+    sv = smfg.Solver(a, device=0)
+    for _ in range(2):
+        info = sv.factor(v, posdef=True)
+        assert info.factor_status == smfg.SMFG_FACTOR_NOT_POSDEF
+        stopped = sv.export().block(0)[:, :bad]
+        gi = sv.factor(good[3], posdef=True)
+        _compare(a, sv, gi, good[3], True)
+        assert np.array_equal(stopped, sv.export().block(0)[:, :bad])
+    sv.close()
 
 
 @pytest.mark.parametrize("m", [6, 12, 20])
