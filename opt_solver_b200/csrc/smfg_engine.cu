@@ -753,7 +753,7 @@ static bool aptp_sweep(Plan &pl, const smfg_control_t &c, const std::vector<int6
   if (gneed > 0) pl.aptp_gather = grow_buf(pl, pl.aptp_gather, pl.aptp_gather_cap, gneed);
   h.scratch = pl.aptp_gather;
   lc.n += aptp::sweep_finish(d_fr, d_st, nf, compact.data(), (int)compact.size(), h, st);
-  k_aptp_to_tpp<<<nf, 256, 0, st>>>(d_fr, d_st, pl.aptp_q, x.rows_cap, x.tpp, c.blocked_min_front);
+  k_aptp_to_tpp<<<nf, 256, 0, st>>>(d_fr, d_st, pl.aptp_q, x, c.blocked_min_front);
   lc.n += 1;
   // the host vectors above are read by copies already waited for
   return nf < nL || !compact.empty();

@@ -27,6 +27,17 @@ __device__ __forceinline__ void set_flag(unsigned long long *cnt, unsigned bit) 
   atomicOr(cnt + kCFlags, (unsigned long long)bit);
 }
 
+// Whether the factorization is given up, the same answer for every thread of
+// the block: one thread reads the flags. Kernels beside this one may set one at
+// any time (the size classes of a level run side by side, and blocks of one
+// launch too), and threads that read it for themselves could part: those that
+// go on would pass the block's barriers without the shared data of those that
+// left. Blocks may differ: the next kernel of the stream sees the flag in all.
+// Every thread of the block calls it, before any of them returns.
+__device__ __forceinline__ bool block_aborted(const DevFactor &X) {
+  return __syncthreads_or(threadIdx.x == 0 && (X.counters[kCFlags] & kFAbort) != 0) != 0;
+}
+
 // A pivot of an SPD front failed: on the static layout, which has no room for
 // delayed columns, the factorization stops there and is redone on the
 // level-by-level one.
@@ -190,7 +201,7 @@ __global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, i
 // into it. Fronts P.lvl_sn[lo + block].
 // (The static SPD layout: every front of the plan at once, fuse = 0.)
 __global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int fuse) {
-  if (fuse > 0 && (X.counters[kCFlags] & kFAbort)) return;
+  if (fuse > 0 && block_aborted(X)) return;
   const int s = P.lvl_sn[lo + blockIdx.x];
   const int64_t roff = X.sn_roff[s];
   const int nd = X.sn_nd[s], f = X.sn_f[s], fsym = P.sn_fsym[s];
@@ -255,7 +266,7 @@ constexpr int kAsmMap = 12288, kAsmKids = 16;
 
 __global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, int lo, int hi, int lvl, int cols) {
   unsigned long long *cnt = X.counters;
-  if (cnt[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const int *pref = X.lvl_blk + lo + lvl;  // m + 1 prefix entries
   const int m = hi - lo;
   const int total = pref[m];
@@ -793,7 +804,7 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
 template <int NT, bool SMEM>
 __global__ void __launch_bounds__(NT) k_factor(DevPlan P, DevFactor X, int i0, PivotParams prm, int fmin, int fmax) {
   extern __shared__ __align__(16) double smem[];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const int s = P.lvl_sn[i0 + blockIdx.x];
   const int f = X.sn_f[s];
   if (f < fmin || f > fmax || P.sn_large[s]) return;
@@ -833,7 +844,7 @@ __device__ __forceinline__ FrontRef large_view(DevPlan &P, DevFactor &X, int s) 
 
 __global__ void k_large_init(DevPlan P, DevFactor X, const int *__restrict__ large, int nlarge,
                              int posdef, int nbo) {
-  if (X.counters[kCFlags] & kFAbort) {
+  if (block_aborted(X)) {
     // the pivoting kernel takes its decisions from the state alone: done
     if (threadIdx.x == 0) {
       TppState S;
@@ -872,7 +883,7 @@ __global__ void k_large_init(DevPlan P, DevFactor X, const int *__restrict__ lar
 // would have passed the limit.
 __global__ void k_level_limits(DevPlan P, DevFactor X, int lo, int hi, long long neg_limit, long long work_cap) {
   __shared__ long long red[2][32];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   long long neg = 0, work = 0;
   for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
     const int s = P.lvl_sn[i];
@@ -920,16 +931,21 @@ __global__ void k_large_sizes(DevFactor X, const int *__restrict__ large, int nl
 // multifrontal_serial.cpp:810-814, ldlt_kernel.cpp:977), its Schur update
 // from those pivots on; the sweep's counts carried, and the position map
 // (inv, the inverse of loc, which the sweep permuted) rebuilt. One block per
-// front.
+// front. An aborted factorization's fronts are closed (a flag set after the
+// host looked, ahead of the sweep: k_large_init may have left loc unset).
 __global__ void k_aptp_to_tpp(const aptp::Front *__restrict__ fr, const aptp::State *__restrict__ st,
-                              const int *__restrict__ qpos, int64_t rows_cap, TppState *__restrict__ tpp, int bmf) {
+                              const int *__restrict__ qpos, DevFactor X, int bmf) {
   const int i = blockIdx.x;
+  if (block_aborted(X)) {
+    if (threadIdx.x == 0) X.tpp[qpos[i]].phase = 2;
+    return;
+  }
   const aptp::Front F = fr[i];
-  int *inv = F.loc + rows_cap;
+  int *inv = F.loc + X.rows_cap;
   for (int t = threadIdx.x; t < F.f; t += blockDim.x) inv[F.loc[t]] = t;
   if (threadIdx.x != 0) return;
   const aptp::State &A = st[i];
-  TppState &T = tpp[qpos[i]];
+  TppState &T = X.tpp[qpos[i]];
   T.k = A.num_elim;
   T.live = F.ne;
   T.k_paired = -1;
@@ -1229,17 +1245,15 @@ __device__ __forceinline__ int trap_tiles2(int rows, int cols) {
 }
 
 __device__ __forceinline__ void trap_tile2(int w, int rows, int cols, int &ti, int &tj) {
-  const int rt = (rows + kTM - 1) / kTM;
-  tj = 0;
-  while (true) {
+  const int rt = (rows + kTM - 1) / kTM, ct = (cols + kTN - 1) / kTN;
+  for (tj = 0;; ++tj) {
     const int first = (tj * kTN) / kTM;
     const int cnt = rt - first;
-    if (w < cnt) {
+    if (w < cnt || tj + 1 >= ct) {
       ti = first + w;
       return;
     }
     w -= cnt;
-    ++tj;
   }
 }
 
@@ -1249,7 +1263,7 @@ __global__ void __launch_bounds__(256) k_large_gemm(DevPlan P, DevFactor X, cons
   extern __shared__ __align__(16) double dsm_g[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(dsm_g);
   __shared__ int pref[kFrontChunk + 1];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
     const int cnt = min(kFrontChunk, nlarge - chunk);
     front_prefix<256>(cnt, pref, [&](int q) {
@@ -1302,14 +1316,14 @@ __device__ __forceinline__ int defer_tiles(int rows, int cols) {
 
 // Tile w of that order: the largest tj with S(tj) = tj rt - tj (tj - 1) / 2
 // <= w (a root of the quadratic, then corrected by exact integer steps).
-__device__ __forceinline__ void defer_tile(int w, int rows, int &ti, int &tj) {
-  const long long rt = (rows + kDT - 1) / kDT;
+__device__ __forceinline__ void defer_tile(int w, int rows, int cols, int &ti, int &tj) {
+  const long long rt = (rows + kDT - 1) / kDT, ct = (cols + kDT - 1) / kDT;
   auto S = [&](long long x) { return x * rt - x * (x - 1) / 2; };
   const double b = 2.0 * (double)rt + 1.0;
   long long t = (long long)((b - sqrt(fmax(b * b - 8.0 * (double)w, 0.0))) * 0.5);
   if (t < 0) t = 0;
   while (t > 0 && S(t) > w) --t;
-  while (S(t + 1) <= w) ++t;
+  while (t + 1 < ct && S(t + 1) <= w) ++t;
   tj = (int)t;
   ti = (int)(t + (w - S(t)));
 }
@@ -1327,7 +1341,7 @@ __global__ void __launch_bounds__(256, kDBlocksPerSM) k_large_defer(DevPlan P, D
   __shared__ long long m_off[kDFronts];
   __shared__ int m_wo[kDFronts];
   __shared__ int wsum[8];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = tid & 15, ty = tid >> 4;
   for (int chunk = 0; chunk < nlarge; chunk += kDFronts) {
@@ -1392,7 +1406,7 @@ __global__ void __launch_bounds__(256, kDBlocksPerSM) k_large_defer(DevPlan P, D
       }
       const int a = lo;
       int ti, tj;
-      defer_tile(w - pref[a], m_f[a] - m_c0[a], ti, tj);
+      defer_tile(w - pref[a], m_f[a] - m_c0[a], m_e[a] - m_c0[a], ti, tj);
       const int f = m_f[a], e = m_e[a], kk = m_kk[a], p0 = m_p0[a];
       const size_t sf = (size_t)f;
       double *F = X.arena + m_off[a];
@@ -1466,7 +1480,7 @@ __global__ void __launch_bounds__(256, 2) k_large_schur(DevPlan P, DevFactor X, 
   extern __shared__ __align__(16) double dsm_g[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(dsm_g);
   __shared__ int pref[kFrontChunk + 1];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
     const int cnt = min(kFrontChunk, nlarge - chunk);
     front_prefix<256>(cnt, pref, [&](int q) {
@@ -1505,7 +1519,7 @@ __global__ void __launch_bounds__(256, 2) k_large_schur(DevPlan P, DevFactor X, 
 template <int NT>
 __global__ void __launch_bounds__(NT) k_large_finish(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                      const TppState *__restrict__ tpp, PivotParams prm) {
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const int s = large[blockIdx.x];
   const TppState S = tpp[blockIdx.x];
   const FrontRef v = large_view(P, X, s);
@@ -1569,7 +1583,7 @@ __global__ void __launch_bounds__(256) k_large_store(DevPlan P, DevFactor X, con
                                                      int nlarge, int posdef) {
   __shared__ int pref[kFrontChunk + 1];
   __shared__ double sdv[32];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
     const int cnt = min(kFrontChunk, nlarge - chunk);
     front_prefix<256>(cnt, pref, [&](int q) { return (X.sn_pstore[large[chunk + q]] + 31) / 32; });
@@ -1654,7 +1668,7 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
   __shared__ int zero_sh;
   const int q = blockIdx.y;
   const TppState S = cur[q];
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const bool lead = blockIdx.x == 0;
   if (S.phase == 2) {
     if (lead && threadIdx.x == 0) {
@@ -2279,7 +2293,7 @@ constexpr int kInvSmem = kInvWarps * 32 * 33 * (int)sizeof(double);
 __global__ void __launch_bounds__(32 * kInvWarps) k_tri_invert(DevFactor X) {
   extern __shared__ __align__(16) unsigned char inv_smem[];
   double(*S)[33] = reinterpret_cast<double(*)[33]>(inv_smem) + (threadIdx.x >> 5) * 32;
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const int lane = threadIdx.x & 31;
   const int item = blockIdx.x * kInvWarps + (threadIdx.x >> 5);
   if (item >= X.inv_nitems) return;

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
   __shared__ long long ch_roff[KC], ch_off[KC];
   __shared__ int cnt_pos, cnt_neg, cnt_zero, cnt_two, bad_d;
   __shared__ unsigned long long flops_sh;
-  if (X.counters[kCFlags] & kFAbort) return;
+  if (block_aborted(X)) return;
   const int s = P.lvl_sn[i0 + blockIdx.x];
   const int f = X.sn_f[s];
   if (f < fmin || f > fmax || P.sn_large[s]) return;
