@@ -441,7 +441,7 @@ static void ensure_spd_layout(Plan &pl, int wcols, int fuse) {
   SMFG_CUDA(cudaMemcpyAsync(x.sn_ne, pl.d.sn_width, sizeof(int) * ns, cudaMemcpyDeviceToDevice, st));
   SMFG_CUDA(cudaMemsetAsync(x.sn_nd, 0, sizeof(int) * ns, st));
   SMFG_CUDA(cudaMemsetAsync(x.child_doff, 0, sizeof(int) * std::max<size_t>(1, pl.h_child_idx.size()), st));
-  if (ns > 0) k_level_rows<<<ns, 128, 0, st>>>(pl.d, x, 0, 0);
+  if (ns > 0) k_level_rows<true><<<ns, 128, 0, st>>>(pl.d, x, 0, 0);
   SMFG_CUDA(cudaGetLastError());
   SMFG_CUDA(cudaStreamSynchronize(st));  // the host arrays are read
   pl.spd_arena = a;
@@ -881,7 +881,7 @@ static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, in
   if (na > 0) {
     if (!x.spd_static) {
       // (a large front's thousands of rows: more threads a front)
-      k_level_rows<<<na, pl.lvl_maxf[l] >= 1024 ? 512 : 128, 0, st>>>(d, x, lo, fuse);
+      k_level_rows<false><<<na, pl.lvl_maxf[l] >= 1024 ? 512 : 128, 0, st>>>(d, x, lo, fuse);
       lc.n += 1;
     }
     k_level_assemble<<<8 * sm_count(pl.device), 256, 0, st>>>(d, x, lo, hi, l, pl.lvl_cols[l]);

@@ -199,9 +199,11 @@ __global__ void k_level_setup(DevPlan P, DevFactor X, int lo, int hi, int lvl, i
 // Rows of each front of more than fuse rows (children's delayed rows in child
 // order, then its symbolic rows) and each child's contribution-block row map
 // into it. Fronts P.lvl_sn[lo + block].
-// (The static SPD layout: every front of the plan at once, fuse = 0.)
+// STATIC: the SPD layout made ahead of any factorization (no delays, the
+// children's pivots are their widths).
+template <bool STATIC>
 __global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int fuse) {
-  if (fuse > 0 && block_aborted(X)) return;
+  if (!STATIC && block_aborted(X)) return;
   const int s = P.lvl_sn[lo + blockIdx.x];
   const int64_t roff = X.sn_roff[s];
   const int nd = X.sn_nd[s], f = X.sn_f[s], fsym = P.sn_fsym[s];
@@ -209,8 +211,8 @@ __global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int fuse) {
   int *rows = X.rows + roff;
   for (int t = P.child_ptr[s]; t < P.child_ptr[s + 1]; ++t) {
     const int c = P.child_idx[t];
-    const int dc = fuse > 0 ? X.sn_dout[c] : 0;
-    const int pc = fuse > 0 ? X.sn_p[c] : P.sn_width[c];
+    const int dc = STATIC ? 0 : X.sn_dout[c];
+    const int pc = STATIC ? P.sn_width[c] : X.sn_p[c];
     const int fc = X.sn_f[c];
     const int q = fc - pc;
     const int doff = X.child_doff[t];

@@ -118,6 +118,36 @@ def test_not_positive_definite():
     sv.close()
 
 
+def _factor(sv, v, posdef, rcs=(smfg.SMFG_OK, smfg.SMFG_ERR_SINGULAR), **fields):
+    """Factorization through the C entry with fields of the control set."""
+    c = smfg.default_control(posdef)
+    for k, x in fields.items():
+        setattr(c, k, x)
+    info = smfg.Info()
+    val = np.ascontiguousarray(v)
+    rc = smfg.lib().smfg_factor(sv._h, val.ctypes.data, C.byref(c), C.byref(info))
+    assert rc in rcs
+    sv.posdef, sv.info = posdef, info
+    return info
+
+
+@pytest.mark.parametrize("blocked", [1, 2, 33, 130])
+@pytest.mark.parametrize("kind", ["chain", "grid"])
+def test_blocked_min_front_tree(blocked, kind):
+    """The same on trees: from the first row on (no front is assembled by its
+    own block), with delayed columns and contribution blocks on both sides of
+    the edge."""
+    posdef = kind == "grid"
+    n, cp, ri, v = W.laplacian_2d(121, 97) if posdef else W.trajectory_kkt(200, np.random.default_rng(30))
+    a = smfg.analyse(n, cp, ri)
+    sv = smfg.Solver(a, device=0)
+    info = _factor(sv, v, posdef, blocked_min_front=blocked)
+    assert posdef or info.delayed_pivots > 0
+    assert info.max_front > 96
+    _compare(a, sv, info, v, posdef, blocked_min_front=blocked)
+    sv.close()
+
+
 @pytest.mark.parametrize("blocked", [20, 40, 96, 200])
 @pytest.mark.parametrize("posdef", [True, False])
 def test_blocked_min_front(blocked, posdef):
