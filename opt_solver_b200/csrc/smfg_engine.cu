@@ -399,13 +399,14 @@ static void ensure_arena(Plan &pl, int64_t arena_need, int64_t rows_need) {
 // Doubles of an SPD front of symbolic rows f in the static layout: the front
 // and its W (large fronts: wcols rows; those factored in global memory by one
 // block: nb; none in shared memory).
-static int64_t spd_front_doubles(const Plan &pl, int s, int wcols) {
+static int64_t spd_front_doubles(const Plan &pl, int s, const SpdLayout &y) {
   const int64_t f = pl.h_fsym[s];
-  return f * f + f * (pl.h_large[s] ? wcols : f > kMediumMax ? pl.nb : 0);
+  return f * f + f * (pl.h_large[s] ? y.wcols : f > kMediumMax ? y.nb : 0);
 }
-static int64_t spd_arena_doubles(const Plan &pl, int wcols) {
+static int64_t spd_arena_doubles(const Plan &pl, const SpdLayout &y) {
+  if (pl.spd_layout && pl.spd == y) return pl.spd_arena;
   int64_t t = 0;
-  for (int s = 0; s < pl.nsn; ++s) t += spd_front_doubles(pl, s, wcols);
+  for (int s = 0; s < pl.nsn; ++s) t += spd_front_doubles(pl, s, y);
   return t;
 }
 
@@ -413,8 +414,8 @@ static int64_t spd_arena_doubles(const Plan &pl, int wcols) {
 // assembly work items of every front, its rows and its children's row maps,
 // in place of two kernels a level on every factorization (k_level_setup is
 // one block: 119 us for the 33,000 leaves of the 64^3 operator).
-static void ensure_spd_layout(Plan &pl, int wcols, int fuse) {
-  if (pl.spd_layout && pl.spd_wcols == wcols && pl.spd_fuse == fuse) return;
+static void ensure_spd_layout(Plan &pl, const SpdLayout &y) {
+  if (pl.spd_layout && pl.spd == y) return;
   DevFactor &x = pl.x;
   const int ns = pl.nsn, nl = pl.nlevels;
   std::vector<int64_t> off(ns), roff(ns);
@@ -426,10 +427,10 @@ static void ensure_spd_layout(Plan &pl, int wcols, int fuse) {
       const int s = pl.h_lvl_sn[i], f = pl.h_fsym[s];
       off[s] = a;
       roff[s] = r;
-      a += spd_front_doubles(pl, s, wcols);
+      a += spd_front_doubles(pl, s, y);
       r += f;
       blk[i + l] = b;
-      b += (f <= fuse && !pl.h_large[s]) ? 0 : (f + pl.lvl_cols[l] - 1) / pl.lvl_cols[l];
+      b += (f <= y.fuse && !pl.h_large[s]) ? 0 : (f + pl.lvl_cols[l] - 1) / pl.lvl_cols[l];
     }
     blk[pl.lvl_ptr[l + 1] + l] = b;
   }
@@ -446,8 +447,7 @@ static void ensure_spd_layout(Plan &pl, int wcols, int fuse) {
   SMFG_CUDA(cudaStreamSynchronize(st));  // the host arrays are read
   pl.spd_arena = a;
   pl.spd_layout = true;
-  pl.spd_wcols = wcols;
-  pl.spd_fuse = fuse;
+  pl.spd = y;
 }
 
 // ---------------------------------------------------------------------------
@@ -1121,13 +1121,15 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
   set_kernel_attrs(pl.nb);
   set_large_mode(pl, c.posdef);
   if (!c.posdef) pl.spd_layout = false;
-  const int wcols = w_rows(pl, c, c.profile != 0), fuse = fuse_rows(c);
+  const int wcols = w_rows(pl, c, c.profile != 0);
+  const SpdLayout layout{wcols, pl.nb, fuse_rows(c)};
   bool use_static = c.posdef != 0;
   // arena: exact for SPD (no delays); head-room for delays, regrown on overflow
   // (look-ahead: a second W buffer, nb columns more per front)
   // (the symbolic sizes hold nb W rows per front; the SPD steps need more)
   const int64_t base_a = pl.sum_f2 + pl.sum_f * (int64_t)(wcols - c.nb), base_r = pl.sum_f;
-  int64_t need_a = c.posdef ? (pl.spd_layout && pl.spd_wcols == wcols ? pl.spd_arena : spd_arena_doubles(pl, wcols)) : base_a + base_a / 4 + (int64_t)pl.max_fsym * pl.max_fsym * 2 + 4096;
+  int64_t need_a = c.posdef ? spd_arena_doubles(pl, layout)
+                            : base_a + base_a / 4 + (int64_t)pl.max_fsym * pl.max_fsym * 2 + 4096;
   int64_t need_r = c.posdef ? base_r : base_r + base_r / 2 + 4096;
   // mixed fronts: large, at least min_front rows, allowed by the caller's mask
   const MixedCfg mc = mixed_cfg(c);
@@ -1183,7 +1185,7 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     put(&pl.x.tc_img, sizeof(pl.x.tc_img));
     put(&pl.x.tri_inv, sizeof(pl.x.tri_inv));
     if (pl.graph_exec && key == pl.graph_key) {
-      if (pl.graph_static) ensure_spd_layout(pl, wcols, fuse);
+      if (pl.graph_static) ensure_spd_layout(pl, layout);
       if (c.scale)
         SMFG_CUDA(cudaMemcpyAsync(pl.x.scale, c.scale, sizeof(double) * pl.n, cudaMemcpyHostToDevice, pl.stream));
       SMFG_CUDA(cudaEventRecord(pl.ev0, pl.stream));
@@ -1204,7 +1206,7 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     if (c.posdef && !use_static) need_a = std::max(need_a, base_a);
     ensure_arena(pl, std::max(need_a, pl.x.arena_cap), std::max(need_r, pl.x.rows_cap));
     pl.x.spd_static = use_static ? 1 : 0;
-    if (use_static) ensure_spd_layout(pl, wcols, fuse);
+    if (use_static) ensure_spd_layout(pl, layout);
     else pl.spd_layout = false;
     if (pl.x.tc_img_cap < tc_need) {
       dfree(pl, pl.x.tc_img);

@@ -85,6 +85,15 @@ struct DevFactor {
 
 constexpr int kSideStreams = 3;
 
+// What a static SPD layout depends on besides the analysis and the large
+// fronts: the W rows of the large fronts and of those one block factors in
+// global memory (the panel width), and the largest front that its own block
+// assembles.
+struct SpdLayout {
+  int wcols = 0, nb = 0, fuse = 0;
+  bool operator==(const SpdLayout &o) const { return wcols == o.wcols && nb == o.nb && fuse == o.fuse; }
+};
+
 struct Plan {
   int device = 0;
   int n = 0, nsn = 0, nlevels = 0;
@@ -102,10 +111,10 @@ struct Plan {
   std::vector<int8_t> h_grown;     // indefinite fronts that delays took to the APTP size
   int large_mode = -1;             // the lists' factorization kind: 1 SPD, 0 indefinite, -1 none yet
   // SPD fronts take no delays: their sizes, offsets, rows and row maps are
-  // the analysis', laid out once (spd_wcols: its W rows, spd_fuse: its
-  // fused class), until an indefinite factorization overwrites them
+  // the analysis', laid out once for the settings spd, until an indefinite
+  // factorization overwrites them
   bool spd_layout = false;
-  int spd_wcols = 0, spd_fuse = 0;
+  SpdLayout spd;
   int64_t spd_arena = 0;
   bool graph_static = false;       // the captured graph runs on the static layout
   std::vector<int> h_lvl_sn, h_width;  // supernodes by level; pivot columns

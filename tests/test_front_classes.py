@@ -289,3 +289,25 @@ def test_not_positive_definite_tree(m):
     gi = sv.factor(good, posdef=True)
     _compare(a, sv, gi, good, True)
     sv.close()
+
+
+def test_panel_width_changes():
+    """One SPD plan factored with panels of several widths, profiled or not: the
+    layout that is kept between factorizations has room for the panel of each
+    (width 16 profiled and width 32 give the large fronts as many rows of W).
+    Every factor is that of a plan of its own, bit for bit. The
+    fronts include some of 129..191 rows, which one block factors in global
+    memory, several on a level."""
+    n, cp, ri, v = W.varcoef_3d(14, seed=3)
+    a = smfg.analyse(n, cp, ri)
+    rows = np.diff(a.front_row_ptr)
+    assert np.sum((rows > 128) & (rows < 192)) >= 4 and rows.max() >= 192
+    sv = smfg.Solver(a, device=0)
+    for nb, profile in ((16, 0), (48, 0), (16, 0), (16, 1), (32, 0), (16, 1), (5, 0), (32, 0)):
+        _factor(sv, v, True, nb=nb, profile=profile)
+        own = smfg.Solver(a, device=0)
+        _factor(own, v, True, nb=nb, profile=profile)
+        gx, wx = sv.export(), own.export()
+        assert np.array_equal(gx.blocks, wx.blocks) and np.array_equal(gx.rows, wx.rows), (nb, profile)
+        own.close()
+    sv.close()
