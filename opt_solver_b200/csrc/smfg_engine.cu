@@ -81,7 +81,7 @@ int sm_count(int dev) {
 // rows, positions and tags.
 size_t front_smem_bytes(int fmax, int nb, int blocked_min_front = 0) {
   const size_t w = (fmax >= blocked_min_front) ? (size_t)fmax * nb * 8 : 0;
-  return (size_t)fmax * (fmax | 1) * 8 + w + (size_t)fmax * 12 + (size_t)fmax + 64;
+  return (size_t)fmax * smem_front_ld(fmax, nb) * 8 + w + (size_t)fmax * 12 + (size_t)fmax + 64;
 }
 
 }  // namespace

@@ -38,6 +38,11 @@ struct FrontStats {
 
 constexpr int kTeamMax = 16;  // CTAs of a team (a thread-block cluster)
 
+// Leading dimension of a front of f rows in shared memory: odd, so that a row
+// of the lower triangle is read without bank conflicts, but for panels so wide
+// that a front of 128 rows and its W would not fit with it (up to nb = 57 do).
+__host__ __device__ inline int smem_front_ld(int f, int nb) { return nb > 48 ? f : f | 1; }
+
 // Shared control block of a front kernel.
 struct FrontShared {
   double red[32];
@@ -53,11 +58,16 @@ struct FrontShared {
   int ckind[32], ca[32], cb[32];
   double pin[64], pout[64];
   int pr[64];
+  FrontStats st;
+};
+
+// The same of a team of CTAs (not in FrontShared: the one-block kernels need
+// the room for wide panels).
+struct TeamShared : FrontShared {
   int tr_seq;  // team reductions so far (alike in every CTA of a team)
   // the team's partial results, a row per CTA, written by each CTA into every
   // one of the team (two buffers alternate)
   double team[2][kTeamMax][6];
-  FrontStats st;
 };
 
 __device__ __forceinline__ double dmax_ref(double a, double b) {  // std::max(a, b)
@@ -638,7 +648,8 @@ static __device__ void team_bundle(const FrontRef &v, FrontShared &sh, Top2 &t, 
   if constexpr (C > 1) {
     // each CTA's partial into every CTA of the team; after the barrier a
     // warp's lanes merge the C rows
-    double(*slot)[6] = sh.team[sh.tr_seq & 1];
+    TeamShared &ts = static_cast<TeamShared &>(sh);
+    double(*slot)[6] = ts.team[ts.tr_seq & 1];
     const int rank = team_rank<C>();
     if ((int)threadIdx.x < C) {
       double *row = slot[rank];
@@ -661,7 +672,7 @@ static __device__ void team_bundle(const FrontRef &v, FrontShared &sh, Top2 &t, 
     t = warp_top2(o);
     x1 = warp_max(a);
     x2 = warp_max(b);
-    if (threadIdx.x == 0) sh.tr_seq += 1;
+    if (threadIdx.x == 0) ts.tr_seq += 1;
     __syncthreads();
   }
 }
@@ -974,7 +985,8 @@ static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, con
       const int cand = c0 + rank;
       int tk = 0, ta = -1, tb = -1;
       if (cand < limit) tk = cand_eval_team<NT, 1>(v, k, limit, cand, prm, sh, ta, tb);
-      double(*slot)[6] = sh.team[sh.tr_seq & 1];
+      TeamShared &ts = static_cast<TeamShared &>(sh);
+      double(*slot)[6] = ts.team[ts.tr_seq & 1];
       if ((int)threadIdx.x < C) {
         team_store(slot[rank] + 0, threadIdx.x, (double)tk);
         team_store(slot[rank] + 1, threadIdx.x, (double)ta);
@@ -992,7 +1004,7 @@ static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, con
         }
       }
       __syncthreads();
-      if (threadIdx.x == 0) sh.tr_seq += 1;
+      if (threadIdx.x == 0) ts.tr_seq += 1;
       __syncthreads();
     }
   } else if (f > 2048) {

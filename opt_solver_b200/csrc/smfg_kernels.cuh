@@ -663,7 +663,7 @@ __device__ void factor_one_front(DevPlan &P, DevFactor &X, int s, const PivotPar
   PivotParams prm = prm0;
   prm.eff_small = __longlong_as_double((long long)X.counters[kCEffSmall]);
   FrontRef v;
-  v.ld = SMEM ? f | 1 : f;  // (odd: rows of the front without bank conflicts)
+  v.ld = SMEM ? smem_front_ld(f, nb) : f;
   v.f = f;
   v.ne = ne;
   int *inv;
@@ -969,7 +969,7 @@ __global__ void k_aptp_to_tpp(const aptp::Front *__restrict__ fr, const aptp::St
 template <int NT, int C>
 __global__ void __launch_bounds__(NT) k_large_panel(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                     PivotParams prm, int iter) {
-  __shared__ FrontShared sh;
+  __shared__ TeamShared sh;
   __shared__ PairScratch s_pair;
   const int q = blockIdx.x / C;
   const bool lead = team_rank<C>() == 0 && threadIdx.x == 0;

@@ -311,3 +311,19 @@ def test_panel_width_changes():
         assert np.array_equal(gx.blocks, wx.blocks) and np.array_equal(gx.rows, wx.rows), (nb, profile)
         own.close()
     sv.close()
+
+
+@pytest.mark.parametrize("nb", [2, 48, 49, 54, 55, 57])
+@pytest.mark.parametrize("posdef", [True, False])
+def test_panel_widths(nb, posdef):
+    """Panels up to the widest that fits beside a front of 128 rows in shared
+    memory (57; from 49 on the front is not padded), bit for bit."""
+    rng = np.random.default_rng(nb)
+    for n in (97, 127, 128, 129):
+        A = _spd(n, rng) if posdef else _indefinite(n, rng)
+        n, cp, ri, v = dense_lower(A)
+        a = smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL)
+        sv = smfg.Solver(a, device=0)
+        info = _factor(sv, v, posdef, nb=nb)
+        _compare(a, sv, info, v, posdef, nb=nb)
+        sv.close()
