@@ -1185,7 +1185,9 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     put(&pl.x.tc_img, sizeof(pl.x.tc_img));
     put(&pl.x.tri_inv, sizeof(pl.x.tri_inv));
     if (pl.graph_exec && key == pl.graph_key) {
+      // (a graph of the level-by-level sequence lays its fronts out itself)
       if (pl.graph_static) ensure_spd_layout(pl, layout);
+      else pl.spd_layout = false;
       if (c.scale)
         SMFG_CUDA(cudaMemcpyAsync(pl.x.scale, c.scale, sizeof(double) * pl.n, cudaMemcpyHostToDevice, pl.stream));
       SMFG_CUDA(cudaEventRecord(pl.ev0, pl.stream));
@@ -1257,7 +1259,10 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     }
     break;
   }
-  if (use_graph && !replayed && !((unsigned)h_cnt[kCFlags] & (kFArena | kFRows | kFTcCap | kFAptpMiss))) {
+  // the redo of an SPD factorization that failed is not captured: the plan's
+  // graph stays that of the static layout
+  const bool redone = c.posdef && !use_static;
+  if (use_graph && !replayed && !redone && !((unsigned)h_cnt[kCFlags] & (kFArena | kFRows | kFTcCap | kFAptpMiss))) {
     // capture the sequence for the next call with this configuration
     key.clear();
     smfg_control_t kc = c;

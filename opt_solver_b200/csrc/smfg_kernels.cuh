@@ -1985,7 +1985,9 @@ __global__ void k_steps_check(unsigned long long *cnt, int steps) {
   if (threadIdx.x == 0 && cnt[kCActive] >= (unsigned long long)steps) set_flag(cnt, kFSteps);
 }
 
-// Totals over all fronts, in supernode order (deterministic).
+// Totals over all fronts, in supernode order (deterministic). On the static
+// layout every front has its symbolic rows; a front that has not was laid out
+// by something else meanwhile, and its class's kernel may have passed it by.
 struct FactorTotals {
   long long pos, neg, zero, two_by_two, delayed, entries;
   int max_front, pad;
@@ -2008,6 +2010,7 @@ __global__ void k_finish(DevPlan P, DevFactor X, FactorTotals *out) {
     a[4] += X.sn_dout[s];
     a[5] += (long long)X.sn_f[s] * X.sn_pstore[s];
     mx = max(mx, X.sn_f[s]);
+    if (X.spd_static && X.sn_f[s] != P.sn_fsym[s]) set_flag(X.counters, kFInternal);
     fsum += X.sn_flops[s];  // integer-valued: exact in any order
   }
   for (int o = 16; o > 0; o >>= 1) {

@@ -52,3 +52,55 @@ def test_graph_replay_bitwise(kind):
     x, _, om, _ = sv.refine(b, x, max_steps=20, omega_target=1e-13, method=smfg.REFINE_AUTO)
     assert om < 1e-12
     sv.close()
+
+
+def _two_supernodes(ne, n, rng):
+    """A dense SPD matrix whose first ne columns are one supernode and the rest
+    its parent: a pivot that fails in the first delays columns into the second."""
+    from opt_solver_b200 import smfg
+    from tests.cases import dense_lower
+    G = rng.standard_normal((n, n))
+    n, cp, ri, v = dense_lower(G @ G.T + n * np.eye(n))
+    a = smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL)
+    arrays = {k: getattr(a, k).copy() for k in smfg._ANALYSIS_FIELDS}
+    arrays["sn_start"], arrays["sn_end"] = np.int32([0, ne]), np.int32([ne, n])
+    arrays["sn_parent"], arrays["postorder"] = np.int32([1, -1]), np.int32([0, 1])
+    arrays["child_ptr"], arrays["child_idx"] = np.int32([0, 0, 1]), np.int32([0])
+    arrays["front_row_ptr"] = np.int32([0, n, 2 * n - ne])
+    arrays["front_row_idx"] = np.concatenate([np.arange(n), np.arange(ne, n)]).astype(np.int32)
+    return n, cp, v, smfg.Analysis(n, arrays)
+
+
+@pytest.mark.parametrize("ne,n", [(10, 38), (40, 130), (70, 230)])
+def test_graph_with_failed_pivots(ne, n):
+    """Matrices that are not positive definite, with a graph, between good ones
+    with and without it. The failed columns are delayed into a parent that
+    leaves its size class (28 rows to 34 and more); every good factorization
+    is that of a plan of its own, bit for bit, and the graph stays the one of
+    good factorizations."""
+    import torch
+    from opt_solver_b200 import smfg
+    n, cp, v, a = _two_supernodes(ne, n, np.random.default_rng(n))
+    bad = v.copy()
+    bad[cp[4]] = -1.0
+    sv, own = smfg.Solver(a, device=0), smfg.Solver(a, device=0)
+    own.factor(v, posdef=True)
+    want = own.export().blocks
+    d_v = torch.from_numpy(v.copy()).cuda()
+    reports, launches = [], []
+    for values, graph in ((bad, True), (v, False), (bad, True), (v, False), (v, True), (bad, True), (v, True),
+                          (bad, False), (v, True), (bad, True), (v, False)):
+        d_v.copy_(torch.from_numpy(values))
+        info = sv.factor(d_v, posdef=True, graph=graph)
+        if values is bad:
+            assert info.factor_status == smfg.SMFG_FACTOR_NOT_POSDEF
+            assert info.delayed_pivots == ne - 4
+            reports.append((info.inertia, info.delayed_pivots, info.flops, info.max_front))
+        else:
+            assert info.factor_status == smfg.SMFG_FACTOR_SUCCESS
+            assert np.array_equal(sv.export().blocks, want)
+            launches.append(info.kernel_launches)
+    assert all(r == reports[0] for r in reports)
+    assert len(set(launches)) == 1  # no good factorization takes the level-by-level kernels
+    sv.close()
+    own.close()
