@@ -421,8 +421,12 @@ static void ensure_spd_layout(Plan &pl, const SpdLayout &y) {
   std::vector<int64_t> off(ns), roff(ns);
   std::vector<int> blk((size_t)ns + nl + 1, 0);
   int64_t a = 0, r = 0;
+  pl.spd_lvl_a.resize(nl);
+  pl.spd_lvl_r.resize(nl);
   for (int l = 0; l < nl; ++l) {
     int b = 0;
+    pl.spd_lvl_a[l] = a;
+    pl.spd_lvl_r[l] = r;
     for (int i = pl.lvl_ptr[l]; i < pl.lvl_ptr[l + 1]; ++i) {
       const int s = pl.h_lvl_sn[i], f = pl.h_fsym[s];
       off[s] = a;
@@ -898,8 +902,8 @@ static unsigned launch_level_fronts(Plan &pl, const smfg_control_t &c, int l, in
   return used;
 }
 
-static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_t &c, LaunchCount &lc,
-                           GemmProfile &gp, bool fixed = false) {
+// The factorization's counters, per-front counts and values placed.
+static void enqueue_values(Plan &pl, const double *d_values, const smfg_control_t &c, LaunchCount &lc, bool fixed) {
   DevPlan &d = pl.d;
   DevFactor &x = pl.x;
   cudaStream_t st = pl.stream;
@@ -922,10 +926,28 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
   k_values<<<vgrid, 256, 0, st>>>(
       d_values, pl.nnz_in, d.vptr, d.vsrc, pcol, d.pri, d.perm, scale, pl.nnz, x.pv, x.pv_raw,
       x.counters);
-  const bool fixed_layout = x.spd_static != 0;  // SPD: sizes and offsets laid out before
-  k_eff_small<<<1, 1, 0, st>>>(x.counters, c.small_pivot, fixed_layout ? pl.spd_arena : 0,
-                               fixed_layout ? pl.sum_f : 0);
+  k_eff_small<<<1, 1, 0, st>>>(x.counters, c.small_pivot, x.spd_static ? pl.spd_arena : 0,
+                               x.spd_static ? pl.sum_f : 0);
   lc.n += 2;
+}
+
+// The launches of a factorization. from > 0: the levels from there on, level by
+// level, after a run on the static layout that failed in that level (the levels
+// below it took no delays and stand as that run left them; redoing them too
+// would cost a failing matrix nearly twice a good one's time).
+static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_t &c, LaunchCount &lc,
+                           GemmProfile &gp, bool fixed = false, int from = 0) {
+  DevPlan &d = pl.d;
+  DevFactor &x = pl.x;
+  cudaStream_t st = pl.stream;
+  const int sms = sm_count(pl.device);
+  const bool fixed_layout = x.spd_static != 0;  // SPD: sizes and offsets laid out before
+  if (from > 0) {
+    k_resume<<<1, 1, 0, st>>>(x.counters, pl.spd_lvl_a[from], pl.spd_lvl_r[from]);
+    lc.n += 1;
+  } else {
+    enqueue_values(pl, d_values, c, lc, fixed);
+  }
   const bool aptp_on = aptp_active(c);
   // early stops (indefinite): max_negative_pivots, the work limit
   const long long neg_limit = c.posdef ? -1 : (long long)c.max_negative_pivots;
@@ -938,7 +960,7 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
   const MixedCfg mc = mixed_cfg(c);
   const int wcols = w_rows(pl, c, gp.on);
   const int fuse = fuse_rows(c);
-  for (int l = 0; l < pl.nlevels; ++l) {
+  for (int l = from; l < pl.nlevels; ++l) {
     const int lo = pl.lvl_ptr[l], hi = pl.lvl_ptr[l + 1];
     if (!fixed_layout) {
       k_level_setup<1024><<<1, 1024, 0, st>>>(d, x, lo, hi, l, wcols, fuse, pl.lvl_cols[l]);
@@ -1171,6 +1193,7 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     key.insert(key.end(), b, b + n);
   };
   bool replayed = false;
+  int from = 0;  // the level that a redo starts from
   // the APTP sweeps read sizes back between levels: no capture then
   bool use_graph = c.graph != 0 && !gp.on && !(aptp_active(c) && pl.max_large > 0);
   if (use_graph) {
@@ -1199,13 +1222,18 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
       SMFG_CUDA(cudaEventElapsedTime(&ms, pl.ev0, pl.ev1));
       const unsigned fl = (unsigned)h_cnt[kCFlags];
       replayed = !(fl & (kFArena | kFRows | kFTcCap | kFSteps | kFAptpMiss | kFStatic));
-      if (fl & kFStatic) use_static = false;
+      if (fl & kFStatic) {
+        use_static = false;
+        from = (int)h_cnt[kCFailLevel];
+      }
       lc.n = pl.graph_launches;
     }
   }
   int attempt_extra = 0;
   for (int attempt = 0; attempt < 4 && !replayed; ++attempt) {
     if (c.posdef && !use_static) need_a = std::max(need_a, base_a);
+    // (arrays made anew lose the levels below)
+    if (need_a > pl.x.arena_cap || need_r > pl.x.rows_cap) from = 0;
     ensure_arena(pl, std::max(need_a, pl.x.arena_cap), std::max(need_r, pl.x.rows_cap));
     pl.x.spd_static = use_static ? 1 : 0;
     if (use_static) ensure_spd_layout(pl, layout);
@@ -1215,12 +1243,14 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
       pl.x.tc_img = dalloc<uint8_t>(pl, tc_need);
       pl.x.tc_img_cap = tc_need;
     }
-    lc = LaunchCount{};
     gp.used = 0;
     pl.aptp_failed = 0;
     pl.aptp_fronts = 0;
-    SMFG_CUDA(cudaEventRecord(pl.ev0, pl.stream));
-    enqueue_factor(pl, d_values, c, lc, gp);
+    if (from == 0) {
+      lc = LaunchCount{};
+      SMFG_CUDA(cudaEventRecord(pl.ev0, pl.stream));
+    }
+    enqueue_factor(pl, d_values, c, lc, gp, false, from);
     static_assert(sizeof(FactorTotals) <= 8 * sizeof(unsigned long long), "totals slot");
     k_finish<<<1, 1024, 0, pl.stream>>>(pl.d, pl.x, d_tot);
     lc.n += 1;
@@ -1231,12 +1261,15 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     SMFG_CUDA(cudaEventElapsedTime(&ms, pl.ev0, pl.ev1));
     const unsigned flags = (unsigned)h_cnt[kCFlags];
     if (flags & kFStatic) {
-      // not positive definite: redone with the failed columns delayed, as the
-      // reference reports it
+      // not positive definite: redone from the failing level with the failed
+      // columns delayed, for the report (under a profile the whole, so that
+      // the update kernels' figures hold no abandoned level)
       use_static = false;
+      from = gp.on ? 0 : (int)h_cnt[kCFailLevel];
       --attempt;
       continue;
     }
+    from = 0;
     if (flags & (kFArena | kFRows)) {
       need_a = std::max<int64_t>(need_a * 2, (int64_t)h_cnt[kCArena] * 2);
       need_r = std::max<int64_t>(need_r * 2, (int64_t)h_cnt[kCRows] * 2);

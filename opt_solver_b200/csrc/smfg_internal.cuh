@@ -115,6 +115,7 @@ struct Plan {
   // factorization overwrites them
   bool spd_layout = false;
   SpdLayout spd;
+  std::vector<int64_t> spd_lvl_a, spd_lvl_r;  // arena and rows in use below each level
   int64_t spd_arena = 0;
   bool graph_static = false;       // the captured graph runs on the static layout
   std::vector<int> h_lvl_sn, h_width;  // supernodes by level; pivot columns

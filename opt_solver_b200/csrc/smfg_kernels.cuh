@@ -11,7 +11,8 @@ namespace smfg {
 // counters[] slots
 enum : int { kCArena = 0, kCRows = 1, kCFlags = 2, kCMaxAbs = 3, kCAux = 4, kCEffSmall = 5,
              kCActive = 6, kCGemmFlops = 7, kCTcFlops = 8, kCDeferBytes = 9, kCDeferUpd = 10,
-             kCDeferSmall = 11, kCAptpMiss = 12, kCNegSoFar = 13, kCWorkSoFar = 14, kCCount = 15 };
+             kCDeferSmall = 11, kCAptpMiss = 12, kCNegSoFar = 13, kCWorkSoFar = 14, kCFailLevel = 15,
+             kCCount = 16 };
 // error flag bits (counters[kCFlags])
 enum : unsigned { kFArena = 1u, kFRows = 2u, kFNonfinite = 4u, kFNotPosdef = 8u, kFNonfiniteD = 16u,
                   kFMap = 32u, kFInternal = 64u, kFTcWait = 128u, kFTcCap = 256u, kFSteps = 512u,
@@ -38,10 +39,12 @@ __device__ __forceinline__ bool block_aborted(const DevFactor &X) {
   return __syncthreads_or(threadIdx.x == 0 && (X.counters[kCFlags] & kFAbort) != 0) != 0;
 }
 
-// A pivot of an SPD front failed: on the static layout, which has no room for
-// delayed columns, the factorization stops there and is redone on the
-// level-by-level one.
-__device__ __forceinline__ void flag_not_posdef(const DevFactor &X) {
+// A pivot of the SPD front s failed: on the static layout, which has no room
+// for delayed columns, the factorization stops there and goes on from the
+// front's level on the level-by-level one. (Every front that fails in a run on
+// the static layout is of one level: the next level's kernels see the flag.)
+__device__ __forceinline__ void flag_not_posdef(const DevPlan &P, const DevFactor &X, int s) {
+  if (X.spd_static) X.counters[kCFailLevel] = (unsigned long long)P.sn_level[s];
   set_flag(X.counters, kFNotPosdef | (X.spd_static ? kFStatic : 0u));
 }
 
@@ -88,6 +91,14 @@ __global__ void k_eff_small(unsigned long long *cnt, double small_pivot, long lo
   const double m = __longlong_as_double((long long)cnt[kCMaxAbs]);
   const double e = (m > 0.0 && m < small_pivot) ? small_pivot * m : small_pivot;
   cnt[kCEffSmall] = (unsigned long long)__double_as_longlong(e);
+}
+
+// A factorization that failed on the static layout goes on level by level: its
+// flags cleared, the arena and rows in use those of the levels below.
+__global__ void k_resume(unsigned long long *cnt, long long arena, long long rows) {
+  cnt[kCFlags] &= ~(unsigned long long)(kFStatic | kFNotPosdef);
+  cnt[kCArena] = (unsigned long long)arena;
+  cnt[kCRows] = (unsigned long long)rows;
 }
 
 // ---------------------------------------------------------------------------
@@ -732,7 +743,7 @@ __device__ void store_front(DevPlan &P, DevFactor &X, int s, const FrontRef &v, 
   }
   __syncthreads();
   if (prm.posdef) {
-    if (p < ne && threadIdx.x == 0) flag_not_posdef(X);
+    if (p < ne && threadIdx.x == 0) flag_not_posdef(P, X, s);
     // L = L_unit sqrt(D), upper part zero
     // (a warp per column: its square root taken once)
     for (int c = threadIdx.x >> 5; c < pstore; c += NT / 32) {
@@ -1540,7 +1551,7 @@ __global__ void __launch_bounds__(NT) k_large_finish(DevPlan P, DevFactor X, con
   }
   __syncthreads();
   if (prm.posdef) {
-    if (p < ne && threadIdx.x == 0) flag_not_posdef(X);
+    if (p < ne && threadIdx.x == 0) flag_not_posdef(P, X, s);
   } else {
     bool bad = false;
     for (int c = threadIdx.x; c < pstore; c += NT) {

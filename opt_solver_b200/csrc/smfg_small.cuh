@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
   // --- store: L and D (store_front's forms), counts, row maps
   const bool is_root = P.sn_parent[s] < 0;
   const int pstore = (is_root && p < ne) ? ne : p;
-  if (prm.posdef && p < ne && tid == 0) flag_not_posdef(X);
+  if (prm.posdef && p < ne && tid == 0) flag_not_posdef(P, X, s);
   small_sync<NT>();
   {
     int pos = 0, neg = 0, zero = 0, two = 0;

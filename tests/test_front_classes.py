@@ -327,3 +327,74 @@ def test_panel_widths(nb, posdef):
         info = _factor(sv, v, posdef, nb=nb)
         _compare(a, sv, info, v, posdef, nb=nb)
         sv.close()
+
+
+def _spd_report(a, v):
+    """What a factorization without pivoting finds when pivots may fail: the
+    columns from a front's first failed pivot on are delayed to its parent.
+    Per supernode (rows, pivots, delayed columns, flops); plain numpy."""
+    pv = O.permuted_values(a, v)
+    out, cb = np.zeros((a.nsn, 4)), {}
+    for s in a.postorder:
+        kids = a.child_idx[a.child_ptr[s]:a.child_ptr[s + 1]]
+        rows = [r for c in kids for r in cb[c][1]]
+        ne = len(rows) + a.sn_end[s] - a.sn_start[s]
+        rows += list(a.front_row_idx[a.front_row_ptr[s]:a.front_row_ptr[s + 1]])
+        pos = {r: i for i, r in enumerate(rows)}
+        f = len(rows)
+        F = np.zeros((f, f))
+        for j in range(a.sn_start[s], a.sn_end[s]):
+            for k in range(a.perm_col_ptr[j], a.perm_col_ptr[j + 1]):
+                F[pos[a.perm_row_idx[k]], pos[j]] += pv[k]
+        for c in kids:
+            m, _, r = cb.pop(c)
+            ix = np.array([pos[x] for x in r], dtype=np.int64)
+            F[np.ix_(ix, ix)] += m
+        p, fl = 0, 0.0
+        while p < ne and F[p, p] > 0.0:
+            F[p + 1:, p + 1:] -= np.outer(F[p + 1:, p], F[p + 1:, p] / F[p, p])
+            p += 1
+            fl += (f - p) + (f - p) * (f - p + 1.0)
+        root = a.sn_parent[s] < 0
+        out[s] = f, p, 0 if root else ne - p, fl
+        cb[s] = (np.tril(F[p:, p:]), [] if root else rows[p:ne], [] if root else rows[p:])
+    return out
+
+
+@pytest.mark.parametrize("m,bad", [(6, 1), (12, 1), (12, 3), (16, 2), (20, 1), (20, 4)])
+def test_not_positive_definite_report(m, bad):
+    """Counts, sizes and delays of a factorization that fails, whether it goes on
+    from the level that failed (from the second call on, and after a replay) or
+    is redone whole (the first, whose arena has no room; a profiled one)."""
+    import torch
+    n, cp, ri, good = W.varcoef_3d(m, seed=m)
+    v = good.copy()
+    v[W.diagonal_slots(n, cp, ri)[np.random.default_rng(m).choice(n, bad)]] *= -1
+    a = smfg.analyse(n, cp, ri)
+    want = _spd_report(a, v)
+    sv = smfg.Solver(a, device=0)
+    own = smfg.Solver(a, device=0)
+    own.factor(good, posdef=True)
+    blocks = own.export().blocks
+    d_v = torch.from_numpy(good.copy()).cuda()
+    rcs = (smfg.SMFG_ERR_SINGULAR,)
+    for how in ("plain", "plain", "profile", "plain", "graph", "plain"):
+        if how == "graph":
+            for values in (good, v):  # captured, then replayed
+                d_v.copy_(torch.from_numpy(values))
+                info = sv.factor(d_v, posdef=True, graph=True)
+        else:
+            info = _factor(sv, v, True, rcs=rcs, profile=int(how == "profile"))
+        assert info.factor_status == smfg.SMFG_FACTOR_NOT_POSDEF
+        gx, st = sv.export(), sv.front_stats()
+        assert np.array_equal(gx.f, want[:, 0]), how
+        assert np.array_equal(st[:, 0], want[:, 1]) and np.array_equal(st[:, 4], want[:, 2]), how
+        assert info.flops == want[:, 3].sum() and info.delayed_pivots == want[:, 2].sum()
+        assert info.max_front == want[:, 0].max()
+        assert info.inertia == (want[:, 1].sum(), 0, n - want[:, 1].sum())
+        # a front with delayed columns takes no pivot: the first is the failed one
+        assert not np.any(want[want[:, 0] > np.diff(a.front_row_ptr), 1])
+        sv.factor(good, posdef=True)
+        assert np.array_equal(sv.export().blocks, blocks)
+    sv.close()
+    own.close()
