@@ -129,12 +129,6 @@ static void large_state(Plan &pl) {
 
 // The lists of pl.h_large on the device, with the state they size.
 static void upload_large(Plan &pl) {
-  // a captured graph holds the old lists' and states' addresses
-  if (pl.graph_exec) {
-    cudaGraphExecDestroy(pl.graph_exec);
-    pl.graph_exec = nullptr;
-    pl.graph_key.clear();
-  }
   large_lists(pl);
   dfree(pl, pl.d.lvl_large);
   dfree(pl, pl.d.sn_large);
@@ -143,27 +137,51 @@ static void upload_large(Plan &pl) {
   large_state(pl);
   pl.spd_layout = false;
   SMFG_CUDA(cudaStreamSynchronize(pl.stream));
+  pl.large_made = true;
 }
 
 // Fronts that delays took to the APTP size outside the large-front path
 // join it (the caller redoes the factorization).
 static void add_large(Plan &pl, const std::vector<int> &sn) {
-  for (int s : sn) pl.h_large[s] = pl.h_grown[s] = 1;
+  // a captured graph may hold the old lists' and states' addresses
+  if (pl.graph_exec) {
+    cudaGraphExecDestroy(pl.graph_exec);
+    pl.graph_exec = nullptr;
+    pl.graph_key.clear();
+  }
+  for (int s : sn) pl.h_large[s] = 1;
   upload_large(pl);
 }
 
 // The large fronts of an SPD or an indefinite factorization: by symbolic
-// rows, and for the latter the fronts that delays took to the APTP size.
+// rows, and for the latter the fronts that delays took to the APTP size. Both
+// kinds' lists are kept, so that a caller who alternates between them on one
+// plan neither frees nor uploads anything, and keeps its graph.
 static void set_large_mode(Plan &pl, int posdef) {
-  if (pl.large_mode == (posdef ? 1 : 0)) return;
-  pl.large_mode = posdef ? 1 : 0;
+  const int mode = posdef ? 1 : 0;
+  if (pl.large_mode >= 0 && pl.large_mode != mode) {
+    LargeSet &o = pl.large_other;
+    std::swap(pl.lvl_large_ptr, o.lvl_large_ptr);
+    std::swap(pl.lvl_large_maxw, o.lvl_large_maxw);
+    std::swap(pl.lvl_large_maxf, o.lvl_large_maxf);
+    std::swap(pl.h_lvl_large, o.h_lvl_large);
+    std::swap(pl.h_large, o.h_large);
+    std::swap(pl.large_made, o.large_made);
+    std::swap(pl.max_large, o.max_large);
+    std::swap(pl.d.lvl_large, o.lvl_large);
+    std::swap(pl.d.sn_large, o.sn_large);
+    std::swap(pl.x.tpp, o.tpp);
+    std::swap(pl.x.tc_jobs, o.tc_jobs);
+    std::swap(pl.x.tc_ipref, o.tc_ipref);
+    std::swap(pl.x.tc_tpref, o.tc_tpref);
+    std::swap(pl.aptp_sizes, o.aptp_sizes);
+    std::swap(pl.aptp_q, o.aptp_q);
+  }
+  pl.large_mode = mode;
+  if (pl.large_made) return;
   const int lim = posdef ? kLargeMinSpd : kLargeMin;
-  for (int s = 0; s < pl.nsn; ++s) pl.h_large[s] = pl.h_fsym[s] >= lim || (!posdef && pl.h_grown[s]) ? 1 : 0;
-  for (void *p : {(void *)pl.x.tri_inv, (void *)pl.x.sn_ioff, (void *)pl.x.inv_items}) dfree(pl, p);
-  pl.x.tri_inv = nullptr;
-  pl.x.sn_ioff = nullptr;
-  pl.x.inv_items = nullptr;
-  pl.x.inv_nitems = 0;
+  pl.h_large.assign(pl.nsn, 0);
+  for (int s = 0; s < pl.nsn; ++s) pl.h_large[s] = pl.h_fsym[s] >= lim ? 1 : 0;
   upload_large(pl);
 }
 
@@ -202,9 +220,7 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   for (int l = 0; l < nl; ++l)
     std::stable_sort(lvl_sn.begin() + pl.lvl_ptr[l], lvl_sn.begin() + pl.lvl_ptr[l + 1],
                      [&](int x, int y) { return fsym[x] > fsym[y]; });
-  // the large fronts (multi-block path) are listed by the first factorization
-  pl.h_large.assign(ns, 0);
-  pl.h_grown.assign(ns, 0);
+  // (the large fronts are listed by the first factorization of each kind)
   pl.h_lvl_sn = lvl_sn;
   pl.h_width = width;
   pl.h_fsym = fsym;

@@ -94,6 +94,24 @@ struct SpdLayout {
   bool operator==(const SpdLayout &o) const { return wcols == o.wcols && nb == o.nb && fuse == o.fuse; }
 };
 
+// The large-front lists of one kind of factorization, with the device state
+// sized by them, while the plan holds the other kind's (its members of the
+// same names).
+struct LargeSet {
+  std::vector<int> lvl_large_ptr, lvl_large_maxw, lvl_large_maxf, h_lvl_large;
+  std::vector<int8_t> h_large;
+  bool large_made = false;
+  int max_large = 0;
+  int *lvl_large = nullptr;
+  int8_t *sn_large = nullptr;
+  TppState *tpp = nullptr;
+  void *tc_jobs = nullptr;
+  int64_t *tc_ipref = nullptr;
+  int *tc_tpref = nullptr;
+  int64_t *aptp_sizes = nullptr;
+  int *aptp_q = nullptr;
+};
+
 struct Plan {
   int device = 0;
   int n = 0, nsn = 0, nlevels = 0;
@@ -108,8 +126,11 @@ struct Plan {
   std::vector<int> lvl_large_pmax; // most stored pivots among them (last factorization)
   std::vector<int> h_lvl_large;    // host copy of the large-front lists
   std::vector<int8_t> h_large;     // per supernode: the large-front path (symbolic rows, or grown by delays)
-  std::vector<int8_t> h_grown;     // indefinite fronts that delays took to the APTP size
-  int large_mode = -1;             // the lists' factorization kind: 1 SPD, 0 indefinite, -1 none yet
+  // the lists' factorization kind (1 SPD, 0 indefinite, -1 none yet), whether
+  // they are on the device, and the other kind's
+  int large_mode = -1;
+  bool large_made = false;
+  LargeSet large_other;
   // SPD fronts take no delays: their sizes, offsets, rows and row maps are
   // the analysis', laid out once for the settings spd, until an indefinite
   // factorization overwrites them

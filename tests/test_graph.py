@@ -104,3 +104,29 @@ def test_graph_with_failed_pivots(ne, n):
     assert len(set(launches)) == 1  # no good factorization takes the level-by-level kernels
     sv.close()
     own.close()
+
+
+@pytest.mark.parametrize("m", [12, 20])
+def test_kinds_alternate_on_one_plan(m):
+    """SPD and indefinite factorizations of one plan in turn, plain and by graph:
+    each has its own large fronts, and every factor and solution is that of a
+    plan that only ever took its kind, bit for bit."""
+    import torch
+    from opt_solver_b200 import smfg
+    n, cp, ri, v = W.varcoef_3d(m, seed=m)
+    a = smfg.analyse(n, cp, ri)
+    b = W.rhs(n, 2, seed=3)
+    d_v = torch.from_numpy(v.copy()).cuda()
+    want = {}
+    for posdef in (True, False):
+        own = smfg.Solver(a, device=0)
+        own.factor(d_v, posdef=posdef)
+        want[posdef] = own.export().blocks, own.solve(b)
+        own.close()
+    sv = smfg.Solver(a, device=0)
+    for posdef, graph in ((True, True), (False, False), (True, True), (False, False), (True, False), (False, True),
+                          (True, False), (False, True), (True, True), (True, True), (False, False)):
+        sv.factor(d_v, posdef=posdef, graph=graph)
+        assert np.array_equal(sv.export().blocks, want[posdef][0])
+        assert np.array_equal(sv.solve(b), want[posdef][1])
+    sv.close()
