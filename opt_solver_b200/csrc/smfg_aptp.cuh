@@ -100,8 +100,13 @@ struct Group {
     if (WARP) __syncwarp();
     else __syncthreads();
   }
+  // (a barrier too: what the threads read before it may be written after it;
+  // a warp's vote alone orders no memory)
   static __device__ __forceinline__ bool any(bool b) {
-    return WARP ? __any_sync(0xffffffffu, b) != 0 : __syncthreads_or(b) != 0;
+    if (!WARP) return __syncthreads_or(b) != 0;
+    const bool r = __any_sync(0xffffffffu, b) != 0;
+    __syncwarp();
+    return r;
   }
 };
 
