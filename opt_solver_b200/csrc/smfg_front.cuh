@@ -122,13 +122,12 @@ __device__ __forceinline__ Top2 warp_top2(Top2 t) {
 
 template <int NT>
 struct Block {
-  static_assert(NT % 32 == 0 && NT <= 1024, "block size");
+  static_assert(NT % 32 == 0 && NT >= 256 && NT <= 1024, "block size");
   static constexpr int NW = NT / 32;
 
   // Max of non-negative values.
   static __device__ double max(double v, FrontShared &sh) {
     v = warp_max(v);
-    if (NW == 1) return v;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     __syncthreads();
     if (l == 0) sh.red[w] = v;
@@ -141,7 +140,6 @@ struct Block {
     t = warp_top2(t);
     a = warp_max(a);
     b = warp_max(b);
-    if (NW == 1) return;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     __syncthreads();
     if (l == 0) {
@@ -596,8 +594,6 @@ __device__ __forceinline__ bool two_by_two_ok_s(double d00, double d10, double d
   return true;
 }
 
-// select_pivot (ldlt_kernel.cpp:127-275). Result in sh.kind / sh.a / sh.b.
-
 // |col[i]| for i in [lo, hi), thread tid of nth: 16-byte loads of aligned
 // pairs, eight pairs in flight; each thread visits its indexes in increasing
 // order (the head element before its pairs, the tail after), so fn sees a
@@ -605,10 +601,6 @@ __device__ __forceinline__ bool two_by_two_ok_s(double d00, double d10, double d
 template <typename Fn>
 __device__ __forceinline__ void scanv(const double *__restrict__ col, int lo, int hi, int tid, int nth, Fn fn) {
   if (lo >= hi) return;
-  if (nth < 512) {  // small blocks (fronts in shared memory): one element at a time
-    for (int i = lo + tid; i < hi; i += nth) fn(fabs(col[i]), i);
-    return;
-  }
   int a = lo;
   if (reinterpret_cast<uintptr_t>(col + a) & 15) {
     if (tid == 0) fn(fabs(col[a]), a);
@@ -905,6 +897,7 @@ __device__ __forceinline__ int small_cand(const double *F, int ld, int f, int ne
   return 0;
 }
 
+// select_pivot (ldlt_kernel.cpp:127-275). Result in sh.kind / sh.a / sh.b.
 template <int NT, int C = 1>
 static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, const PivotParams &prm,
                                  FrontShared &sh) {
@@ -1025,15 +1018,6 @@ static __device__ void select_pivot_blk(const FrontRef &v, int k, int limit, con
     const int cand = c0 + warp;
     int wk = 0, wa = -1, wb = -1;
     if (cand < limit) wk = cand_eval_warp(v, k, limit, cand, prm, wa, wb);
-    if (NW == 1) {
-      if (wk) {
-        kind = wk;
-        pa = wa;
-        pb = wb;
-        done = true;
-      }
-      continue;
-    }
     if ((threadIdx.x & 31) == 0) {
       sh.ckind[warp] = wk;
       sh.ca[warp] = wa;
