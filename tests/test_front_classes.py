@@ -398,3 +398,31 @@ def test_not_positive_definite_report(m, bad):
         assert np.array_equal(sv.export().blocks, blocks)
     sv.close()
     own.close()
+
+
+def _leaves_under_root(k, m, posdef, rng):
+    """k leaves of one column, whose contribution blocks cover a dense root of m
+    columns (natural order)."""
+    n = k + m
+    A = np.zeros((n, n))
+    A[k:, k:] = _spd(m, rng) if posdef else _indefinite(m, rng)
+    A[k:, :k] = rng.standard_normal((m, k))
+    A[np.arange(k), np.arange(k)] = 4.0 * n if posdef else 1.0 + rng.random(k)
+    if posdef:
+        A[np.arange(k, n), np.arange(k, n)] += 4.0 * n
+    rows, cols = np.nonzero(np.tril(A))
+    order = np.lexsort((rows, cols))
+    cp = np.concatenate([[0], np.cumsum(np.bincount(cols, minlength=n))])
+    return n, cp.astype(np.int32), rows[order].astype(np.int32), A[rows, cols][order]
+
+
+@pytest.mark.parametrize("k,m", [(16, 110), (17, 110), (40, 100), (40, 250), (16, 768), (16, 769), (13, 946)])
+@pytest.mark.parametrize("posdef", [True, False])
+def test_assembly_maps(k, m, posdef):
+    """Assembly of a front past the fused sizes on both sides of the room for its
+    children's inverse row maps (16 children, children x rows 12,288): gathered,
+    or a pass per child."""
+    # (the last leaf is merged into the root)
+    a, _ = _run(*_leaves_under_root(k + 1, m - 1, posdef, np.random.default_rng(k + m)), posdef, nemin=1,
+                ordering=smfg.ORDER_NATURAL)
+    assert int(np.diff(a.child_ptr).max()) == k and int(np.diff(a.front_row_ptr).max()) == m
