@@ -128,7 +128,8 @@ typedef struct {
    * normally and captures the launch sequence; later calls with the same
    * configuration replay it (the refactor of an interior-point iteration).
    * A replay that finds a front needing more pivoting steps than captured,
-   * or an arena too small, falls back to the normal path. */
+   * an arena too small, or a failed pivot of an SPD matrix falls back to the
+   * normal path. */
   int graph;
   /* Dense kernel of the indefinite fronts: fronts of at least aptp_min_rows
    * realized rows take a posteriori threshold pivoting in 256-column tiles,
@@ -167,7 +168,9 @@ typedef struct {
   int reserved_i[7];      /* [0] profiled FP64 update launches, [1] tensor-core update passes,
                              [2] deferred front updates, [3] those of at most 2 pivots,
                              [4] columns the APTP sweeps failed (Info::aptp_failed_columns),
-                             [5] fronts swept by APTP */
+                             [5] fronts swept by APTP. ([2], [3] and the flops and bytes
+                             below count, of an unprofiled SPD factorization that failed,
+                             the updates of the level that was given up too) */
   double reserved_d[8];   /* [0] profiled FP64 update ms (deferred + Schur), [1] FP64 update
                              flops, [2] arena bytes, [3] tensor-core update flops (2 per
                              multiply-add), [4] profiled tensor-core update ms (split + product

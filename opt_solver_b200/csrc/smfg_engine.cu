@@ -228,9 +228,10 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   pl.lvl_maxkids.assign(nl, 0);
   pl.lvl_cols.assign(nl, kAsmCols);
   {
-    // (the 701 x 433 grid's upper levels of a few fronts: with this, two children
-    // in flight and the division-free store, its factorization 5.48 -> 5.15 ms;
-    // 64^3 operator 32.92 -> 32.79 ms, 23^3 3.85 -> 3.66 ms with its transfers)
+    // Factorization ms with 32 columns everywhere / 8 on levels of fewer items
+    // than SMs / than four times the SMs / 8 everywhere: 701 x 433 Laplacian 4.09 /
+    // 4.00 / 3.97 / 3.98, 64^3 operator 29.89 / 29.89 / 28.95 / 29.04, 23 x 19 x 21
+    // 2.71 / 2.59 / 2.59 / 2.58, KKT 12^3 14.65 / 14.55 / 14.56 / 14.55.
     std::vector<int64_t> items(nl, 0);
     for (int s = 0; s < ns; ++s)
       if (fsym[s] > kFuseMax) items[level[s]] += (fsym[s] + kAsmCols - 1) / kAsmCols;
@@ -545,7 +546,7 @@ static MixedCfg mixed_cfg(const smfg_control_t &c) {
 constexpr int kTcEvery = 16;
 
 // Deferred updates of a level's large fronts: the streamed kernel for
-// panels of up to 16 pivots, the general tiled one beyond.
+// panels of up to kDK pivots, the general tiled one beyond.
 static void launch_defer(Plan &pl, const int *lg, int nL, const TppState *states, int ggrid, int mode = 0,
                          cudaStream_t stream = nullptr) {
   cudaStream_t st = stream ? stream : pl.stream;

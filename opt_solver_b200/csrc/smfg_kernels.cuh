@@ -244,12 +244,6 @@ __global__ void k_level_rows(DevPlan P, DevFactor X, int lo, int fuse) {
   for (int u = threadIdx.x; u < f; u += blockDim.x) X.tags[roff + u] = 0;
 }
 
-// Assembly of one level (process_front, multifrontal_serial.cpp:720-789):
-// each work item is a block of `cols` columns of one front. It zeroes the
-// lower part of its columns, adds the original entries of the pivot columns,
-// then extend-adds the children's Schur blocks in child order (the
-// reference's order of additions, so every entry is the reference's sum).
-// A child's block is read in place from its own front.
 // First index in [lo, hi) of the increasing a[] whose value is >= key (hi
 // if none), by the 32 lanes of a warp: 32 probes a round (one load
 // latency), about three rounds for a few thousand entries.
@@ -267,14 +261,22 @@ __device__ __forceinline__ int warp_lower_bound(const int *__restrict__ a, int l
   return lo + __popc(__ballot_sync(0xffffffffu, pos < hi && a[pos] < key));
 }
 
-// Gather form (fronts whose children's inverse row maps fit in shared memory,
-// kAsmMap entries): every entry is formed in a register -- zero, then the
+// Assembly of one level's fronts past the fused sizes (process_front,
+// multifrontal_serial.cpp:720-789): each work item is a block of `cols` columns
+// of one front. An entry is zero, plus its original value (pivot columns), plus
+// the children's Schur blocks in child order (the reference's order of
+// additions, so every entry is the reference's sum); a child's block is read in
+// place from its own front.
+//
+// Gather form (at most kAsmKids children whose inverse row maps fit in shared
+// memory, kAsmMap entries): every entry is formed in a register -- zero, then the
 // children in order, each read at the row its inverse map gives -- and
 // written once; the few entries with an original value are formed again from
 // it. It replaces a zeroing pass and a read-modify-write pass a child, whose
 // dependent loads bound it (64^3 operator: 4.2 -> 3.4 ms a factorization, a
 // level of 1,500-row fronts 290 -> 200 us for 310 MB). Fronts whose maps do
-// not fit take the passes.
+// not fit take the passes: the lower part of the item's columns zeroed, the
+// original entries added, then each child's block.
 constexpr int kAsmMap = 12288, kAsmKids = 16;
 
 __global__ void __launch_bounds__(256) k_level_assemble(DevPlan P, DevFactor X, int lo, int hi, int lvl, int cols) {
@@ -1307,11 +1309,11 @@ __global__ void __launch_bounds__(256) k_large_gemm(DevPlan P, DevFactor X, cons
 }
 
 // ---------------------------------------------------------------------------
-// Deferred updates, streamed (nb <= 16): the same update as k_large_gemm,
+// Deferred updates, streamed (up to kDK pivots): the same update as k_large_gemm,
 // F[c0:f, c0:e] -= L[c0:f, p0:p1] W[:, c0:e] on the lower trapezoid, each
 // element by the same chain c = fma(-l_p, w_p, c) over p in order (w_p = 0
-// skipped), so the results are bitwise those of k_large_gemm. With at most
-// 16 pivots an element costs 2 K flops for 16 bytes of traffic: the update
+// skipped), so the results are bitwise those of k_large_gemm. With K = 16 or
+// 32 pivots an element costs 2 K flops for 16 bytes of traffic: the update
 // is bound by HBM, and the kernel is shaped for that: 64 x 64 tiles (every
 // front of the launch in one list), 16 elements a thread, at most 64
 // registers so that four blocks share an SM and their load, update and
@@ -2101,8 +2103,8 @@ __global__ void k_solve_scatter(double *__restrict__ b, int ldb, int nrhs, int n
 // Solves by level. Each front's work vector w (length f, at the front's row
 // offset) holds its pivot rows' values and, in the forward sweep, its update
 // vector for the parent (rows p..f); x (new numbering) holds the pivot
-// results. Large fronts (symbolic rows >= kLargeMin) take the multi-block
-// kernels below; the others' sweeps are in smfg_solve.cuh.
+// results. Large fronts (symbolic rows >= kLargeMin, SPD kLargeMinSpd) take the
+// multi-block kernels below; the others' sweeps are in smfg_solve.cuh.
 
 // The 32 x 32 lower block L[jb:jb+nb, jb:jb+nb) copied to shared memory
 // asynchronously (8-byte cp.async, zero fill

@@ -36,7 +36,7 @@ import numpy as np
 from . import smfg
 
 N_FEATURES = 10
-LARGE_MIN = 384  # the engine's large-front class (kLargeMin)
+LARGE_MIN = 384  # the smallest front the engine takes in mixed precision (kLargeMin)
 
 
 def _tree_height(parent):
