@@ -28,15 +28,17 @@ __device__ __forceinline__ void set_flag(unsigned long long *cnt, unsigned bit) 
   atomicOr(cnt + kCFlags, (unsigned long long)bit);
 }
 
-// Whether the factorization is given up, the same answer for every thread of
-// the block: one thread reads the flags. Kernels beside this one may set one at
+// Whether the factorization is given up. For one thread of a block.
+__device__ __forceinline__ bool abort_flagged(const DevFactor &X) { return (X.counters[kCFlags] & kFAbort) != 0; }
+
+// The same answer for every thread of the block: one thread reads the flags. Kernels beside this one may set one at
 // any time (the size classes of a level run side by side, and blocks of one
 // launch too), and threads that read it for themselves could part: those that
 // go on would pass the block's barriers without the shared data of those that
 // left. Blocks may differ: the next kernel of the stream sees the flag in all.
 // Every thread of the block calls it, before any of them returns.
 __device__ __forceinline__ bool block_aborted(const DevFactor &X) {
-  return __syncthreads_or(threadIdx.x == 0 && (X.counters[kCFlags] & kFAbort) != 0) != 0;
+  return __syncthreads_or(threadIdx.x == 0 && abort_flagged(X)) != 0;
 }
 
 // A pivot of the SPD front s failed: on the static layout, which has no room
@@ -857,10 +859,15 @@ __device__ __forceinline__ FrontRef large_view(DevPlan &P, DevFactor &X, int s) 
   return v;
 }
 
+// The state of each large front of a level before its first step. The kernels
+// of the steps and of the Schur update take every decision from it, without a
+// look at the abort flags: a team's CTAs and a launch's blocks agree, and
+// nothing is asked for of a front that is closed here because the factorization
+// is given up. (A flag set later, by a kernel beside them, costs the rest of
+// the level's work; the test in each of them cost 0.7% of a 64^3 factorization.)
 __global__ void k_large_init(DevPlan P, DevFactor X, const int *__restrict__ large, int nlarge,
                              int posdef, int nbo) {
   if (block_aborted(X)) {
-    // the pivoting kernel takes its decisions from the state alone: done
     if (threadIdx.x == 0) {
       TppState S;
       tpp_init(S, 0, posdef != 0);
@@ -976,9 +983,6 @@ __global__ void k_aptp_to_tpp(const aptp::Front *__restrict__ fr, const aptp::St
 // front is taken by a team of C CTAs launched as one thread-block cluster
 // (blockIdx.x / C = the front), the pivot decisions taken by every CTA of
 // the team alike and the swaps and panel eliminations split over it.
-// (No test of the abort flags here: a kernel beside this one may set one
-// while a team reads it, and the team's CTAs must agree; k_large_init closes
-// the fronts of an aborted factorization.)
 template <int NT, int C>
 __global__ void __launch_bounds__(NT) k_large_panel(DevPlan P, DevFactor X, const int *__restrict__ large,
                                                     PivotParams prm, int iter) {
@@ -1278,7 +1282,6 @@ __global__ void __launch_bounds__(256) k_large_gemm(DevPlan P, DevFactor X, cons
   extern __shared__ __align__(16) double dsm_g[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(dsm_g);
   __shared__ int pref[kFrontChunk + 1];
-  if (block_aborted(X)) return;
   for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
     const int cnt = min(kFrontChunk, nlarge - chunk);
     front_prefix<256>(cnt, pref, [&](int q) {
@@ -1356,7 +1359,6 @@ __global__ void __launch_bounds__(256, kDBlocksPerSM) k_large_defer(DevPlan P, D
   __shared__ long long m_off[kDFronts];
   __shared__ int m_wo[kDFronts];
   __shared__ int wsum[8];
-  if (block_aborted(X)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = tid & 15, ty = tid >> 4;
   for (int chunk = 0; chunk < nlarge; chunk += kDFronts) {
@@ -1495,7 +1497,6 @@ __global__ void __launch_bounds__(256, 2) k_large_schur(DevPlan P, DevFactor X, 
   extern __shared__ __align__(16) double dsm_g[];
   TileSmem &sm = *reinterpret_cast<TileSmem *>(dsm_g);
   __shared__ int pref[kFrontChunk + 1];
-  if (block_aborted(X)) return;
   for (int chunk = 0; chunk < nlarge; chunk += kFrontChunk) {
     const int cnt = min(kFrontChunk, nlarge - chunk);
     front_prefix<256>(cnt, pref, [&](int q) {
@@ -1683,7 +1684,6 @@ __global__ void __launch_bounds__(256) k_large_panel_spd2(DevPlan P, DevFactor X
   __shared__ int zero_sh;
   const int q = blockIdx.y;
   const TppState S = cur[q];
-  if (block_aborted(X)) return;
   const bool lead = blockIdx.x == 0;
   if (S.phase == 2) {
     if (lead && threadIdx.x == 0) {
@@ -1943,7 +1943,7 @@ __global__ void k_tc_jobs(DevPlan P, DevFactor X, const int *__restrict__ large,
   double flops = 0.0;
   X.tc_ipref[0] = 0;
   X.tc_tpref[0] = 0;
-  const bool dead = (X.counters[kCFlags] & kFAbort) != 0;
+  const bool dead = abort_flagged(X);
   for (int q = 0; q < nlarge && !dead; ++q) {
     TppState &S = tpp[q];
     if (!S.mixed) continue;

@@ -39,6 +39,18 @@ __device__ __forceinline__ void small_sync() {
   else __syncthreads();
 }
 
+// A barrier that tells every thread whether any gave true.
+template <int NT>
+__device__ __forceinline__ bool small_sync_or(bool b) {
+  if constexpr (NT == 32) {
+    const bool r = __any_sync(0xffffffffu, b) != 0;
+    __syncwarp();
+    return r;
+  } else {
+    return __syncthreads_or(b) != 0;
+  }
+}
+
 // Rows and columns p < q of the front exchanged (sym_swap_blk's pairs), then
 // a barrier.
 template <int NT>
@@ -91,7 +103,9 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
   __shared__ long long ch_roff[KC], ch_off[KC];
   __shared__ int cnt_pos, cnt_neg, cnt_zero, cnt_two, bad_d;
   __shared__ unsigned long long flops_sh;
-  if (block_aborted(X)) return;
+  // (one thread reads the flags, the first barrier tells the others: nothing is
+  // written to global memory before it)
+  const bool dead = threadIdx.x == 0 && abort_flagged(X);
   const int s = P.lvl_sn[i0 + blockIdx.x];
   const int f = X.sn_f[s];
   if (f < fmin || f > fmax || P.sn_large[s]) return;
@@ -132,7 +146,7 @@ __global__ void __launch_bounds__(NT) k_small_front(DevPlan P, DevFactor X, int 
     cnt_pos = cnt_neg = cnt_zero = cnt_two = bad_d = 0;
     flops_sh = 0;
   }
-  small_sync<NT>();
+  if (small_sync_or<NT>(dead)) return;
   {
     const int cs = P.sn_start[s], wdt = P.sn_width[s];
     const int k0 = P.pcp[cs], k1 = P.pcp[cs + wdt];

@@ -26,16 +26,19 @@ def _kernels():
 
 
 def test_abort_decided_per_block():
-    """No kernel of more than one working thread reads the abort flags but
-    through block_aborted, and none returns before calling it."""
+    """No kernel of more than one working thread reads the abort flags in more
+    than one thread of a block, and none that asks block_aborted returns before
+    it does."""
     seen = 0
     for name, body in _kernels():
+        assert "kFAbort" not in body, name
         if "block_aborted" in body:
             seen += 1
             assert "return" not in body[:body.index("block_aborted")], name
-        if "kFAbort" in body:
-            assert re.match(r"\s*if \(threadIdx\.x != 0", body), name
-    assert seen >= 12
+        if "abort_flagged" in body:
+            seen += 1
+            assert re.search(r"threadIdx\.x == 0 && abort_flagged|^\s*if \(threadIdx\.x != 0", body), name
+    assert seen >= 10
 
 
 def _forest(blocks):
