@@ -5,7 +5,7 @@
 // one another), so a front's L is brought into shared memory (up to 64 rows)
 // or requested into L2 (more) before the kernel waits for the one before it
 // (programmatic dependent launch), every right-hand side's chain runs beside
-// the others, and the reciprocals of an SPD diagonal are taken off the chain.
+// the others, and the reciprocals of an SPD diagonal are formed off the chain.
 // One grid: a block per front -- of up to 64 rows with L in shared memory and
 // a warp per right-hand side, of more in 32-column strips -- then blocks of
 // eight tiny fronts
@@ -52,6 +52,16 @@ struct LevelGrid {
 // The larger fronts' strip: its triangle and solved values, then vectors.
 constexpr int kStripDoubles = 32 * 33 + 32 * kSolveRhs;
 
+// w / d from d's rounded reciprocal r: the product corrected by its remainder
+// (Markstein), so that a pivot costs a multiply and two fused multiply-adds in
+// the chain in place of a division, and rounds as one. The product alone left
+// backward errors 5% larger on small 5- and 7-point operators; the correction
+// costs 0 to 0.6% of a solve (52 x 49 x 50: 2.35 -> 2.37 ms).
+__device__ __forceinline__ double quotient(double w, double d, double r) {
+  const double q = w * r, e = fma(-q, d, w), y = fma(e, r, q);
+  return e == e ? y : q;
+}
+
 // Four right-hand sides' (or one's) forward chain over a front in shared
 // memory (Ls: column j at j * ld, rows 0..f): rows lane (and lane + 32 when
 // two) of w.
@@ -60,10 +70,11 @@ __device__ __forceinline__ void small_fwd_chain(const double *Ls, int ld, int f,
                                                 double (&w0)[R], double (&w1)[R]) {
   const int lane = threadIdx.x & 31;
   for (int j0 = 0; j0 < p; j0 += 8) {
-    double l0[8], l1[8], r[8];
+    double l0[8], l1[8], r[8], d[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int j = j0 + u;
+      d[u] = (spd && j < p) ? Ls[j * ld + j] : 1.0;
       l0[u] = (j < p && lane > j && lane < f) ? Ls[j * ld + lane] : 0.0;
       l1[u] = (TWO && j < p && lane + 32 > j && lane + 32 < f) ? Ls[j * ld + lane + 32] : 0.0;
       r[u] = (spd && j < p) ? rd[j] : 1.0;
@@ -76,7 +87,7 @@ __device__ __forceinline__ void small_fwd_chain(const double *Ls, int ld, int f,
       for (int q = 0; q < R; ++q) {
         double wj = __shfl_sync(0xffffffffu, (TWO && j >= 32) ? w1[q] : w0[q], j & 31);
         if (spd) {
-          wj *= r[u];
+          wj = quotient(wj, d[u], r[u]);
           w0[q] = lane == j ? wj : w0[q];
           if (TWO) w1[q] = lane + 32 == j ? wj : w1[q];
         }
@@ -98,10 +109,11 @@ __device__ __forceinline__ void small_bwd_chain(const double *Ls, int ld, int p,
                                                 double (&v0)[R], double (&v1)[R]) {
   const int lane = threadIdx.x & 31;
   for (int j1 = p; j1 > 0; j1 -= 8) {
-    double l0[8], l1[8], r[8];
+    double l0[8], l1[8], r[8], d[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int j = j1 - 1 - u;  // row j of L11
+      d[u] = (spd && j >= 0) ? Ls[j * ld + j] : 1.0;
       l0[u] = (j >= 0 && lane < j) ? Ls[lane * ld + j] : 0.0;
       l1[u] = (TWO && j >= 0 && lane + 32 < j) ? Ls[(lane + 32) * ld + j] : 0.0;
       r[u] = (spd && j >= 0) ? rd[j] : 1.0;
@@ -114,7 +126,7 @@ __device__ __forceinline__ void small_bwd_chain(const double *Ls, int ld, int p,
       for (int q = 0; q < R; ++q) {
         double xj = __shfl_sync(0xffffffffu, (TWO && j >= 32) ? v1[q] : v0[q], j & 31);
         if (spd) {
-          xj *= r[u];
+          xj = quotient(xj, d[u], r[u]);
           v0[q] = lane == j ? xj : v0[q];
           if (TWO) v1[q] = lane + 32 == j ? xj : v1[q];
         }
@@ -258,10 +270,7 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
     stage_front(X.arena + X.sn_off[s], f, p, Ls, ld, lane, 32);
     const int my = lane < p ? rows[lane] : 0;
     __syncwarp();
-    double rdv = 1.0;
-    if (posdef && lane < p) rdv = 1.0 / Ls[lane * ld + lane];
-    __syncwarp();
-    if (posdef && lane < p) Ls[lane * ld + lane] = rdv;  // (the diagonal's reciprocals in its place)
+    const double dv = (posdef && lane < p) ? Ls[lane * ld + lane] : 1.0, rdv = 1.0 / dv;
     pdl_wait();
     pdl_trigger();
     auto one = [&](int r0, auto tag) {
@@ -279,12 +288,11 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
       }
       __syncwarp();
       for (int j0 = 0; j0 < p; j0 += 8) {
-        double l[8], rj[8];
+        double l[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int j = j0 + u;
           l[u] = (j < p && lane > j && lane < f) ? Ls[j * ld + lane] : 0.0;
-          rj[u] = (posdef && j < p) ? Ls[j * ld + j] : 1.0;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -292,11 +300,11 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_fwd_level(DevPlan P, DevFactor X,
           if (j >= p) break;
 #pragma unroll
           for (int q = 0; q < R; ++q) {
-            double wj = __shfl_sync(0xffffffffu, w0[q], j);
             if (posdef) {
-              wj *= rj[u];
-              w0[q] = lane == j ? wj : w0[q];
+              const double sc = quotient(w0[q], dv, rdv);
+              w0[q] = lane == j ? sc : w0[q];
             }
+            const double wj = __shfl_sync(0xffffffffu, w0[q], j);
             const double a = fma(-l[u], wj, w0[q]);
             w0[q] = l[u] != 0.0 ? a : w0[q];
           }
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_bwd_level(DevPlan P, DevFactor X,
     const int my = lane < f ? rows[lane] : 0;
     __syncwarp();
     const double *Lc = Ls + lane * ld;
-    const double rdv = (posdef && lane < p) ? 1.0 / Lc[lane] : 1.0;
+    const double dv = (posdef && lane < p) ? Lc[lane] : 1.0, rdv = 1.0 / dv;
     pdl_wait();
     pdl_trigger();
     auto one = [&](int r0, auto tag) {
@@ -543,7 +551,7 @@ __global__ void __launch_bounds__(kLvlNT, 2) k_bwd_level(DevPlan P, DevFactor X,
           const double l = lane < j ? Lc[j] : 0.0;
 #pragma unroll
           for (int q = 0; q < R; ++q) {
-            const double sc = v[q] * rdv;
+            const double sc = quotient(v[q], dv, rdv);
             v[q] = lane == j ? sc : v[q];
             const double xj = __shfl_sync(0xffffffffu, v[q], j);
             const double a = fma(-l, xj, v[q]);

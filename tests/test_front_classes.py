@@ -426,3 +426,22 @@ def test_assembly_maps(k, m, posdef):
     a, _ = _run(*_leaves_under_root(k + 1, m - 1, posdef, np.random.default_rng(k + m)), posdef, nemin=1,
                 ordering=smfg.ORDER_NATURAL)
     assert int(np.diff(a.child_ptr).max()) == k and int(np.diff(a.front_row_ptr).max()) == m
+
+
+@pytest.mark.parametrize("n", [1, 20, 32, 33, 64])
+@pytest.mark.parametrize("nrhs", [1, 5])
+def test_small_solves_divide(n, nrhs):
+    """SPD fronts of up to 64 rows divide by the diagonal of L (a rounded
+    reciprocal and its correction): a diagonal matrix in one dense front is
+    solved as plain divisions round it, infinities as divisions leave them."""
+    rng = np.random.default_rng(n)
+    d = 10.0 ** rng.uniform(-8, 8, n)
+    _, cp, ri, v = dense_lower(np.diag(d))
+    sv = smfg.Solver(smfg.analyse(n, cp, ri, ordering=smfg.ORDER_NATURAL), device=0)
+    sv.factor(v, posdef=True)
+    b = rng.standard_normal((nrhs, n)) * 10.0 ** rng.uniform(-100, 100, (nrhs, n))
+    b[0, 0] = np.inf
+    l = np.sqrt(d)
+    x = sv.solve(b if nrhs > 1 else b[0]).reshape(nrhs, n)
+    assert np.array_equal(x, (b / l) / l)
+    sv.close()
