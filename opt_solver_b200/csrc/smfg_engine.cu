@@ -46,11 +46,26 @@ T *dupload(Plan &pl, const std::vector<T> &v) {
   return p;
 }
 
-void dfree(Plan &pl, void *p) {
+// Frees p and forgets it, so that an allocation that fails next leaves no
+// address of freed memory behind.
+template <class T>
+void dfree(Plan &pl, T *&p) {
   if (!p) return;
-  auto it = std::find(pl.allocs.begin(), pl.allocs.end(), p);
+  auto it = std::find(pl.allocs.begin(), pl.allocs.end(), static_cast<void *>(p));
   if (it != pl.allocs.end()) pl.allocs.erase(it);
   cudaFree(p);
+  p = nullptr;
+}
+
+// p of at least `need` elements (capacity cap), its contents lost when it
+// grows; empty when that fails.
+template <class T>
+void dgrow(Plan &pl, T *&p, int64_t &cap, int64_t need) {
+  if (need <= cap) return;
+  dfree(pl, p);
+  cap = 0;
+  p = dalloc<T>(pl, (size_t)need);
+  cap = need;
 }
 
 thread_local std::string g_last_error;
@@ -115,9 +130,12 @@ static void large_lists(Plan &pl) {
 // Device state sized by the most large fronts of a level.
 static void large_state(Plan &pl) {
   DevFactor &x = pl.x;
-  for (void *p : {(void *)x.tpp, (void *)x.tc_jobs, (void *)x.tc_ipref,
-                  (void *)x.tc_tpref, (void *)pl.aptp_sizes, (void *)pl.aptp_q})
-    dfree(pl, p);
+  dfree(pl, x.tpp);
+  dfree(pl, x.tc_jobs);
+  dfree(pl, x.tc_ipref);
+  dfree(pl, x.tc_tpref);
+  dfree(pl, pl.aptp_sizes);
+  dfree(pl, pl.aptp_q);
   const size_t ml = (size_t)std::max(1, pl.max_large);
   x.tpp = dalloc<TppState>(pl, 2 * ml);  // two buffers (SPD panels)
   x.tc_jobs = dalloc<tc::Job>(pl, ml);
@@ -129,6 +147,7 @@ static void large_state(Plan &pl) {
 
 // The lists of pl.h_large on the device, with the state they size.
 static void upload_large(Plan &pl) {
+  pl.large_made = false;
   large_lists(pl);
   dfree(pl, pl.d.lvl_large);
   dfree(pl, pl.d.sn_large);
@@ -160,6 +179,7 @@ static void add_large(Plan &pl, const std::vector<int> &sn) {
 static void set_large_mode(Plan &pl, int posdef) {
   const int mode = posdef ? 1 : 0;
   if (pl.large_mode >= 0 && pl.large_mode != mode) {
+    pl.factored = false;  // (its lists go)
     LargeSet &o = pl.large_other;
     std::swap(pl.lvl_large_ptr, o.lvl_large_ptr);
     std::swap(pl.lvl_large_maxw, o.lvl_large_maxw);
@@ -392,14 +412,13 @@ static void build_plan(Plan &pl, const smfg_analysis_t &a) {
   x.rows_cap = 0;
 }
 
+// (The factor lives in these: it is lost where they grow.)
 static void ensure_arena(Plan &pl, int64_t arena_need, int64_t rows_need) {
   DevFactor &x = pl.x;
-  if (x.arena_cap < arena_need) {
-    dfree(pl, x.arena);
-    x.arena = dalloc<double>(pl, arena_need);
-    x.arena_cap = arena_need;
-  }
+  dgrow(pl, x.arena, x.arena_cap, arena_need);
   if (x.rows_cap < rows_need) {
+    pl.spd_layout = false;
+    x.rows_cap = 0;
     dfree(pl, x.rows);
     dfree(pl, x.tags);
     dfree(pl, x.cbmap);
@@ -409,7 +428,6 @@ static void ensure_arena(Plan &pl, int64_t arena_need, int64_t rows_need) {
     x.cbmap = dalloc<int>(pl, rows_need);
     x.ploc = dalloc<int>(pl, 2 * (size_t)rows_need);
     x.rows_cap = rows_need;
-    pl.spd_layout = false;
   }
 }
 
@@ -696,12 +714,10 @@ static void aptp_select(Plan &pl, const smfg_control_t &c, const int *lg, int nL
     if (asz[4 * q] >= c.aptp_min_rows) aq.push_back(q);
 }
 
+// As dgrow, by half as much again at least.
 template <class T>
-static T *grow_buf(Plan &pl, T *p, int64_t &cap, int64_t need) {
-  if (need <= cap && p) return p;
-  dfree(pl, p);
-  cap = std::max<int64_t>(need, cap + cap / 2);
-  return dalloc<T>(pl, (size_t)cap);
+static void grow_buf(Plan &pl, T *&p, int64_t &cap, int64_t need) {
+  if (need > cap) dgrow(pl, p, cap, std::max<int64_t>(need, cap + cap / 2));
 }
 
 // The APTP sweep of the level's fronts aq (positions in its large list;
@@ -721,13 +737,15 @@ static bool aptp_sweep(Plan &pl, const smfg_control_t &c, const std::vector<int6
     const int nb = std::min(aptp::kNb, std::max(1, ne));
     kmax = std::max(kmax, (ne + nb - 1) / nb);
   }
-  pl.aptp_buf = grow_buf(pl, pl.aptp_buf, pl.aptp_buf_cap, need);
+  grow_buf(pl, pl.aptp_buf, pl.aptp_buf_cap, need);
   if (nf > pl.aptp_cap) {
     dfree(pl, pl.aptp_fr);
     dfree(pl, pl.aptp_st);
-    pl.aptp_cap = std::max(nf, 2 * pl.aptp_cap);
-    pl.aptp_fr = dalloc<aptp::Front>(pl, pl.aptp_cap);
-    pl.aptp_st = dalloc<aptp::State>(pl, pl.aptp_cap);
+    const int cap = std::max(nf, 2 * pl.aptp_cap);
+    pl.aptp_cap = 0;
+    pl.aptp_fr = dalloc<aptp::Front>(pl, cap);
+    pl.aptp_st = dalloc<aptp::State>(pl, cap);
+    pl.aptp_cap = cap;
   }
   std::vector<aptp::Front> hf(nf);
   int64_t o = 0;
@@ -771,7 +789,7 @@ static bool aptp_sweep(Plan &pl, const smfg_control_t &c, const std::vector<int6
       pl.aptp_failed += hf[i].ne - hs[i].num_elim;
     }
   pl.aptp_fronts += nf;
-  if (gneed > 0) pl.aptp_gather = grow_buf(pl, pl.aptp_gather, pl.aptp_gather_cap, gneed);
+  if (gneed > 0) grow_buf(pl, pl.aptp_gather, pl.aptp_gather_cap, gneed);
   h.scratch = pl.aptp_gather;
   lc.n += aptp::sweep_finish(d_fr, d_st, nf, compact.data(), (int)compact.size(), h, st);
   k_aptp_to_tpp<<<nf, 256, 0, st>>>(d_fr, d_st, pl.aptp_q, x, c.blocked_min_front);
@@ -1225,6 +1243,7 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
     put(&pl.x.tc_img, sizeof(pl.x.tc_img));
     put(&pl.x.tri_inv, sizeof(pl.x.tri_inv));
     if (pl.graph_exec && key == pl.graph_key) {
+      pl.factored = false;
       // (a graph of the level-by-level sequence lays its fronts out itself)
       if (pl.graph_static) ensure_spd_layout(pl, layout);
       else pl.spd_layout = false;
@@ -1249,17 +1268,14 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
   int attempt_extra = 0;
   for (int attempt = 0; attempt < 4 && !replayed; ++attempt) {
     if (c.posdef && !use_static) need_a = std::max(need_a, base_a);
+    dgrow(pl, pl.x.tc_img, pl.x.tc_img_cap, tc_need);
+    pl.factored = false;  // overwritten from here on
     // (arrays made anew lose the levels below)
     if (need_a > pl.x.arena_cap || need_r > pl.x.rows_cap) from = 0;
     ensure_arena(pl, std::max(need_a, pl.x.arena_cap), std::max(need_r, pl.x.rows_cap));
     pl.x.spd_static = use_static ? 1 : 0;
     if (use_static) ensure_spd_layout(pl, layout);
     else pl.spd_layout = false;
-    if (pl.x.tc_img_cap < tc_need) {
-      dfree(pl, pl.x.tc_img);
-      pl.x.tc_img = dalloc<uint8_t>(pl, tc_need);
-      pl.x.tc_img_cap = tc_need;
-    }
     gp.used = 0;
     pl.aptp_failed = 0;
     pl.aptp_fronts = 0;
@@ -1437,11 +1453,7 @@ static int run_factor(Plan &pl, const double *d_values, const smfg_control_t &c,
 // Solve.
 
 static void ensure_work(Plan &pl, int64_t need) {
-  if (pl.x.work_cap < need) {
-    dfree(pl, pl.x.work);
-    pl.x.work = dalloc<double>(pl, need);
-    pl.x.work_cap = need;
-  }
+  if (pl.x.work_cap < need) dgrow(pl, pl.x.work, pl.x.work_cap, need);
 }
 
 // Upper bound of the stored pivots of level l's large fronts: their width

@@ -116,3 +116,24 @@ def test_refine_methods_plain(method):
     x, eta, om, it = sv.refine(b, x0, max_steps=10, omega_target=1e-15, method=method)
     assert om <= max(om0, 1e-15) and eta <= 1e-10
     sv.close()
+
+
+@pytest.mark.parametrize("posdef", [True, False])
+def test_arrays_that_cannot_grow(posdef):
+    """A factorization whose operand images do not fit on the device (an outer
+    block of 2^28 pivots) fails with an error; the factor before it can still
+    be solved with, and the next factorization is what it was."""
+    from opt_solver_b200 import smfg
+    n, cp, ri, v = W.varcoef_3d(20, seed=3)
+    sv = smfg.Solver(smfg.analyse(n, cp, ri), device=0)
+    b = W.rhs(n, 1, seed=4)
+    opt = dict(posdef=posdef, precision=smfg.PREC_MIXED, mixed_min_front=384, aptp_min_rows=0)
+    assert sv.factor(v, **opt).mixed_fronts > 0
+    blocks, x = sv.export().blocks, sv.solve(b)
+    for _ in range(2):
+        with pytest.raises(smfg.SmfgError):
+            sv.factor(v, mixed_block=1 << 28, **opt)
+        assert np.array_equal(sv.solve(b), x)
+    sv.factor(v, **opt)
+    assert np.array_equal(sv.export().blocks, blocks) and np.array_equal(sv.solve(b), x)
+    sv.close()
