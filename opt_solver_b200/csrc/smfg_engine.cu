@@ -1037,7 +1037,10 @@ static void enqueue_factor(Plan &pl, const double *d_values, const smfg_control_
       TppState *fin = x.tpp;  // where the final state of the level's fronts ends up
       if (c.posdef && c.nb == 16) {
         // no delays, no search: one multi-block step per panel, states
-        // double-buffered; the closing step leaves phase 2
+        // double-buffered; the closing step leaves phase 2. (In the redo of a
+        // factorization that failed, fronts with delayed columns outgrow
+        // these symbolic sizes, but they take no pivot: the first column is
+        // the failed one again, with the value it had.)
         const int rpb = (int64_t)nL * ((pl.lvl_large_maxf[l] + 127) / 128) <= 2 * sms ? 128 : 256;
         const dim3 pgrid((pl.lvl_large_maxf[l] + rpb - 1) / rpb, nL);
         // two panels (32 pivots) per step and one rank-32 deferred update.
